@@ -74,6 +74,25 @@ __device__ __forceinline__ u64 mulhi_chain(u64 a, u64 b) {
   return pack(h0, h1);
 }
 
+// floor(a b / 2^64) or one less, from three products: the low one, a0 b0, is
+// left out.
+__device__ __forceinline__ u64 mulhi_low1(u64 a, u64 b) {
+  u32 h0, h1;
+  asm("{\n\t"
+      ".reg .u32 t, m, c;\n\t"
+      "mul.lo.u32 t, %3, %4;\n\t"
+      "mul.hi.u32 m, %3, %4;\n\t"
+      "mad.lo.cc.u32 t, %2, %5, t;\n\t"
+      "madc.hi.cc.u32 m, %2, %5, m;\n\t"
+      "addc.u32 c, 0, 0;\n\t"
+      "mad.lo.cc.u32 %0, %3, %5, m;\n\t"
+      "madc.hi.u32 %1, %3, %5, c;\n\t"
+      "}"
+      : "=r"(h0), "=r"(h1)
+      : "r"(lo32(a)), "r"(hi32(a)), "r"(lo32(b)), "r"(hi32(b)));
+  return pack(h0, h1);
+}
+
 // a * b + c * d mod 2^64.
 __device__ __forceinline__ u64 mad2_lo(u64 a, u64 b, u64 c, u64 d) {
   u64 r;
@@ -92,6 +111,12 @@ __device__ __forceinline__ u64 shoup_lazy(u64 x, u64 w, u64 wp, u64 q) {
   return mad2_lo(x, w, mulhi_chain(x, wp), 0 - q);
 }
 
+// x * w mod q in [0, 3q) for any 64-bit x, with nq = -q: the quotient of
+// mulhi_low1 is at most two short of x w / q, and x (w 2^64 - wp q) / 2^64 < q.
+__device__ __forceinline__ u64 shoup_lazy3(u64 x, u64 w, u64 wp, u64 nq) {
+  return mad2_lo(x, w, mulhi_low1(x, wp), nq);
+}
+
 // Same, with one conditional subtraction: canonical for any 64-bit x.
 __device__ __forceinline__ u64 shoup(u64 x, u64 w, u64 wp, u64 q) {
   u64 r = shoup_lazy(x, w, wp, q);
@@ -99,6 +124,15 @@ __device__ __forceinline__ u64 shoup(u64 x, u64 w, u64 wp, u64 q) {
 }
 
 __device__ __forceinline__ u64 csub(u64 x, u64 m) { return x >= m ? x - m : x; }
+
+// The same for x, m with |x - m| < 2^63, by the sign of the difference: two
+// adds, a shift and two ands where a 64-bit compare takes the half-rate
+// predicate and select path (about 7 issue cycles a warp against 9).
+__device__ __forceinline__ u64 csub_sign(u64 x, u64 m) {
+  const u64 d = x - m;
+  const u32 s = (u32)((int)hi32(d) >> 31);
+  return d + pack(lo32(m) & s, hi32(m) & s);
+}
 
 // [0, 4q) -> [0, q)
 __device__ __forceinline__ u64 canon4(u64 x, u64 q, u64 q2) { return csub(csub(x, q2), q); }

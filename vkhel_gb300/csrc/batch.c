@@ -18,14 +18,18 @@
 
 #include "internal.h"
 
-#define MAX_CLASSES 64
+/* At most MAX_KINDS (kind, degree, q below 2^62 or not, epilogue, NTT(b)
+ * given) combinations; each with q < 2^62 is one class or two (VKCU_Q60 and
+ * VKCU_Q62). */
+#define MAX_KINDS 64
+#define MAX_CLASSES (2 * MAX_KINDS)
 
 struct job_rec {
 	uint32_t kind;         /* VKH_JOB_* */
 	uint32_t log_n;
 	uint32_t needs_scratch;
 	uint32_t lift;         /* index into the batch's lift table, 0 = none */
-	uint32_t wide;         /* modulus class: 2^62 <= q < 2^63 */
+	uint32_t qclass;       /* modulus class, VKCU_Q60 .. VKCU_Q63 */
 	uint32_t b_ntt;        /* b holds NTT(b) (VKCU_JOB_B_NTT) */
 	uint32_t order;        /* insertion order, keeps the sort stable */
 	vkcu_poly_job job;
@@ -160,7 +164,7 @@ static int add_jobs(struct vkhel_batch *b, struct vkhel_ntt_tables *const *table
 		r->log_n = log_n;
 		r->needs_scratch = kind == VKH_JOB_POLYMUL && !b_ntt && (!fused || overlap);
 		r->lift = lift_id;
-		r->wide = (uint32_t) vkcu_wide(tables[k]->q);
+		r->qclass = (uint32_t) vkcu_qclass(tables[k]->q);
 		r->b_ntt = (uint32_t) (b_ntt != 0);
 		r->order = b->njobs - 1;
 		r->job.a = ak;
@@ -269,8 +273,8 @@ static int cmp_rec(const void *x, const void *y) {
 		return (a->kind > b->kind) - (a->kind < b->kind);
 	if (a->log_n != b->log_n)
 		return (a->log_n > b->log_n) - (a->log_n < b->log_n);
-	if (a->wide != b->wide)
-		return (a->wide > b->wide) - (a->wide < b->wide);
+	if (a->qclass != b->qclass)
+		return (a->qclass > b->qclass) - (a->qclass < b->qclass);
 	if (a->lift != b->lift)
 		return (a->lift > b->lift) - (a->lift < b->lift);
 	if (a->b_ntt != b->b_ntt)
@@ -291,22 +295,22 @@ int vkh_issue_classes(void *stream, int sms, const vkcu_poly_job *dev_poly, cons
 		const vkcu_ntt_job *tj = dev_ntt + 3 * (size_t) cl->first;
 		int e;
 		if (cl->kind == VKH_JOB_FORWARD) {
-			e = vkcu_ntt_forward(stream, tj, (int) cl->count, NULL, cl->log_n, cl->wide, sms);
+			e = vkcu_ntt_forward(stream, tj, (int) cl->count, NULL, cl->log_n, cl->qclass, sms);
 		} else if (cl->kind == VKH_JOB_INVERSE) {
-			e = vkcu_ntt_inverse_lift(stream, tj, (int) cl->count, NULL, cl->log_n, cl->wide, sms, lift);
+			e = vkcu_ntt_inverse_lift(stream, tj, (int) cl->count, NULL, cl->log_n, cl->qclass, sms, lift);
 		} else if (cl->fused) {
-			e = vkcu_polymul_lift(stream, dev_poly + cl->first, (int) cl->count, NULL, cl->log_n, cl->wide, sms,
+			e = vkcu_polymul_lift(stream, dev_poly + cl->first, (int) cl->count, NULL, cl->log_n, cl->qclass, sms,
 					lift, (int) cl->b_ntt);
 		} else {
 			const vkcu_ntt_job *nj = dev_ntt + 3 * (size_t) cl->first;
-			e = cl->b_ntt ? 0 : vkcu_ntt_forward(stream, nj, (int) cl->count, NULL, cl->log_n, cl->wide, sms);
+			e = cl->b_ntt ? 0 : vkcu_ntt_forward(stream, nj, (int) cl->count, NULL, cl->log_n, cl->qclass, sms);
 			if (!e)
-				e = vkcu_ntt_forward(stream, nj + cl->count, (int) cl->count, NULL, cl->log_n, cl->wide, sms);
+				e = vkcu_ntt_forward(stream, nj + cl->count, (int) cl->count, NULL, cl->log_n, cl->qclass, sms);
 			if (!e)
-				e = vkcu_pointwise(stream, dev_poly + cl->first, (int) cl->count, cl->log_n, cl->wide, sms);
+				e = vkcu_pointwise(stream, dev_poly + cl->first, (int) cl->count, cl->log_n, cl->qclass, sms);
 			if (!e)
 				e = vkcu_ntt_inverse_lift(stream, nj + 2 * (size_t) cl->count, (int) cl->count, NULL, cl->log_n,
-						cl->wide, sms, lift);
+						cl->qclass, sms, lift);
 		}
 		if (e)
 			return e;
@@ -379,7 +383,7 @@ static int issue(struct vkhel_batch *b) {
 
 /* The single-launch form of a ragged batch (ntt_ragged.cu) when the tuning
  * table asks for it and every class is a fused product of degree 2^12 ..
- * 2^16 with q < 2^62 and no epilogue: items in decreasing size, 2^15 and
+ * 2^16 with q < 2^60 and no epilogue: items in decreasing size, 2^15 and
  * 2^12 products in pairs, an odd pair completed by a copy of its product
  * that writes a dummy buffer. */
 static int ragged_setup(struct vkhel_batch *b) {
@@ -394,7 +398,7 @@ static int ragged_setup(struct vkhel_batch *b) {
 	uint32_t first[17] = {0}, count[17] = {0};
 	for (uint32_t k = 0; k < b->nclasses; k++) {
 		const struct vkh_job_class *cl = &b->classes[k];
-		if (cl->kind != VKH_JOB_POLYMUL || !cl->fused || cl->wide || cl->lift || cl->b_ntt || cl->log_n < 12 ||
+		if (cl->kind != VKH_JOB_POLYMUL || !cl->fused || cl->qclass != VKCU_Q60 || cl->lift || cl->b_ntt || cl->log_n < 12 ||
 				cl->log_n > 16 || count[cl->log_n])
 			return VKHEL_OK;
 		first[cl->log_n] = cl->first;
@@ -488,18 +492,26 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 	 * the kernels of n >= 2^8 move 16 consecutive words with 32-byte vector
 	 * accesses, and slices of n = 1 or 2 words would shift the ones after them */
 	uint64_t scratch_words = 0;
+	uint32_t nkinds = 0;
 	b->nclasses = 0;
 	for (uint32_t i = 0; i < b->njobs; i++) {
 		struct job_rec *r = &b->recs[i];
 		if (b->nclasses == 0 || b->classes[b->nclasses - 1].kind != r->kind ||
-				b->classes[b->nclasses - 1].log_n != r->log_n || b->classes[b->nclasses - 1].wide != (int) r->wide ||
+				b->classes[b->nclasses - 1].log_n != r->log_n || b->classes[b->nclasses - 1].qclass != (int) r->qclass ||
 				b->classes[b->nclasses - 1].lift != r->lift || b->classes[b->nclasses - 1].b_ntt != r->b_ntt) {
-			if (b->nclasses == MAX_CLASSES)
+			int new_kind = 1;
+			for (uint32_t k = 0; r->qclass == VKCU_Q62 && k < b->nclasses; k++) {
+				const struct vkh_job_class *c = &b->classes[k];
+				if (c->kind == r->kind && c->log_n == r->log_n && c->qclass == VKCU_Q60 && c->lift == r->lift &&
+						c->b_ntt == r->b_ntt)
+					new_kind = 0;
+			}
+			if (new_kind && nkinds++ == MAX_KINDS)
 				return vkh_fail(ctx, VKHEL_ERR_UNSUPPORTED, "batch_commit: too many degree classes");
 			struct vkh_job_class *cl = &b->classes[b->nclasses++];
 			cl->kind = r->kind;
 			cl->log_n = r->log_n;
-			cl->wide = (int) r->wide;
+			cl->qclass = (int) r->qclass;
 			cl->lift = r->lift;
 			cl->b_ntt = r->b_ntt;
 			cl->first = i;

@@ -106,7 +106,7 @@ struct vkh_job_class {
 	uint32_t log_n;
 	uint32_t first, count;
 	int fused;
-	int wide;              /* modulus class of every job: 2^62 <= q < 2^63 */
+	int qclass;            /* modulus class of every job, VKCU_Q60 .. VKCU_Q63 */
 	uint32_t lift;         /* index into the lift table, 0 = none */
 	uint32_t b_ntt;        /* polymul jobs whose b holds NTT(b) (VKCU_JOB_B_NTT) */
 };

@@ -16,11 +16,17 @@ extern "C" {
 
 /* Device-resident constants of one (n, q, w) twiddle set.  `fwd` and `inv`
  * point to n interleaved (root, shoup(root)) pairs in the reference's
- * bit-reversed order (src/ntt_tables.c:25-43). */
+ * bit-reversed order (src/ntt_tables.c:25-43).  Each (factor, Shoup factor)
+ * pair lies on a 16-byte boundary: the kernels load it as one vector. */
 typedef struct vkcu_twset {
-	uint64_t q, q2, mu;          /* q, 2q, floor(2^(bits+62)/q) */
+	uint64_t q, q2;              /* q, 2q */
+	uint64_t mu, qinv;           /* floor(2^(bits+62)/q); q^-1 mod 2^64 (odd q) */
 	uint64_t ninv, ninv_s;       /* n^-1 mod q and its Shoup factor */
 	uint64_t w1ninv, w1ninv_s;   /* inv_roots[1] * n^-1 mod q and Shoup factor */
+	/* the same two times 2^64 mod q: the last inverse stage after products
+	 * left divided by 2^64 (a Montgomery product) */
+	uint64_t ninv_m, ninv_m_s;
+	uint64_t w1ninv_m, w1ninv_m_s;
 	uint32_t qbits, log_n;
 	const uint64_t *fwd;
 	const uint64_t *inv;
@@ -155,25 +161,31 @@ typedef struct vkcu_lift {
 /* ---- transforms (ntt.cu) ----
  * `jobs` is a device array of `njobs` jobs that all share log_n and the
  * modulus class, or NULL to launch the single job `one` passed by value.
- * `wide` selects the class: 0 for q < 2^62 (lazy [0, 4q) butterflies), 1 for
- * 2^62 <= q < 2^63 ([0, 2q) butterflies). */
-#define VKCU_WIDE_Q ((uint64_t) 1 << 62)
-static inline int vkcu_wide(uint64_t q) { return q >= VKCU_WIDE_Q; }
+ * `qclass` names the butterfly arithmetic (ntt_core.cuh): how far above q a
+ * lazy word may go in 64 bits. */
+enum {
+	VKCU_Q60 = 0,                /* odd q < 2^60: words below 12q */
+	VKCU_Q62 = 1,                /* other q < 2^62: words below 4q */
+	VKCU_Q63 = 2                 /* 2^62 <= q < 2^63: words below 2q */
+};
+static inline int vkcu_qclass(uint64_t q) {
+	return q < ((uint64_t) 1 << 60) && (q & 1) ? VKCU_Q60 : q < ((uint64_t) 1 << 62) ? VKCU_Q62 : VKCU_Q63;
+}
 int vkcu_ntt_forward(void *stream, const vkcu_ntt_job *jobs, int njobs,
-		const vkcu_ntt_job *one, uint32_t log_n, int wide, int sms);
+		const vkcu_ntt_job *one, uint32_t log_n, int qclass, int sms);
 int vkcu_ntt_inverse(void *stream, const vkcu_ntt_job *jobs, int njobs,
-		const vkcu_ntt_job *one, uint32_t log_n, int wide, int sms);
+		const vkcu_ntt_job *one, uint32_t log_n, int qclass, int sms);
 int vkcu_polymul(void *stream, const vkcu_poly_job *jobs, int njobs,
-		const vkcu_poly_job *one, uint32_t log_n, int wide, int sms);
+		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms);
 /* The same with an epilogue (`lift` NULL or count 0: none); fused into the
  * last pass for 2^8 <= n <= 2^17, a separate element-wise launch otherwise.
  * b_ntt: the jobs carry VKCU_JOB_B_NTT; only the epilogue instantiations of
  * the fused kernels read that flag, so such jobs run those (with no steps
  * when `lift` has none) and the plain kernels stay as lean as before. */
 int vkcu_ntt_inverse_lift(void *stream, const vkcu_ntt_job *jobs, int njobs,
-		const vkcu_ntt_job *one, uint32_t log_n, int wide, int sms, const vkcu_lift *lift);
+		const vkcu_ntt_job *one, uint32_t log_n, int qclass, int sms, const vkcu_lift *lift);
 int vkcu_polymul_lift(void *stream, const vkcu_poly_job *jobs, int njobs,
-		const vkcu_poly_job *one, uint32_t log_n, int wide, int sms, const vkcu_lift *lift, int b_ntt);
+		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms, const vkcu_lift *lift, int b_ntt);
 /* The epilogue alone, in place on `len` words at p (modulus q for TABLE_Q
  * steps), or on the n output words of every job. */
 int vkcu_lift_range(void *stream, uint64_t *p, uint64_t len, uint64_t q, int sms, const vkcu_lift *lift);
@@ -183,7 +195,7 @@ int vkcu_lift_jobs(void *stream, const vkcu_ntt_job *jobs, int njobs, const vkcu
  * outputs; the word the reference's elemmul stores): the pointwise step of a
  * polymul that is not fused. */
 int vkcu_pointwise(void *stream, const vkcu_poly_job *jobs, int njobs,
-		uint32_t log_n, int wide, int sms);
+		uint32_t log_n, int qclass, int sms);
 /* A ragged batch of fused limb products of degrees 2^12 .. 2^16 as one
  * persistent launch (ntt_ragged.cu): items in decreasing size, the first
  * n_cluster_items of kind 16 (one product of 2^16 on a cluster of four CTAs)

@@ -90,7 +90,7 @@ extern "C" VKHEL_EXPORT int vkhel_vector_polymul_noalloc(const struct vkhel_vect
   int e = scratch_address(ctx->device, &scratch);
   if (e) return vkh_cuda(ctx, e, "polymul_noalloc: scratch address");
   const vkcu_poly_job job = {a->dev, b->dev, result->dev, static_cast<uint64_t*>(scratch), d->dev_set};
-  e = vkcu_polymul(ctx->stream, nullptr, 1, &job, t->log_n, vkcu_wide(t->q), ctx->sms);
+  e = vkcu_polymul(ctx->stream, nullptr, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms);
   if (!e) e = vkcu_sync(ctx->stream);
   return vkh_cuda(ctx, e, "polymul_noalloc");
 }

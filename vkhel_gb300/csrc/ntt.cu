@@ -2,7 +2,7 @@
 // simple one-stage-per-barrier kernels (n < 256, unaligned operands), the
 // global-memory passes of n >= 2^18, and the pointwise step of a composed
 // polynomial multiply.  Every launcher takes the modulus class of its jobs
-// (`wide`: 2^62 <= q < 2^63).  The CTA-resident kernels are in
+// (`qclass`, VKCU_Q60 .. VKCU_Q63).  The CTA-resident kernels are in
 // ntt_core.cuh with one launcher per family (ntt_fwd.cu, ntt_inv.cu,
 // ntt_poly.cu).
 #include "elem_ops.cuh"
@@ -35,12 +35,13 @@ __global__ void k_ntt_fwd_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
         if (s == 0)
           ct_first<M>(sm[x], sm[x + half], wt.x, wt.y, t);
         else
-          M::ct(sm[x], sm[x + half], wt.x, wt.y, t);
+          M::template ct<true>(sm[x], sm[x + half], wt.x, wt.y, t);
       }
       __syncthreads();
     }
     u64* out = reinterpret_cast<u64*>(job.out);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = M::canon(sm[i], t);
+    const typename M::Out to(t);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = to.canon(sm[i]);
     __syncthreads();
   }
 }
@@ -65,14 +66,15 @@ __global__ void k_ntt_inv_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
         if (s == log_n - 1)
           gs_first_sd<M>(sm[x], sm[x + half], t, sum, dif);
         else
-          M::sd(sm[x], sm[x + half], t, sum, dif);
+          M::template sd<1>(sm[x], sm[x + half], t, sum, dif);
         if (s == 0) {
-          sm[x] = shoup(sum, t.ninv, t.ninv_s, t.q);
-          sm[x + half] = shoup(dif, t.w1ninv, t.w1ninv_s, t.q);
+          const ulonglong2 f0 = t.fold[0], f1 = t.fold[1];
+          sm[x] = shoup(sum, f0.x, f0.y, t.q);
+          sm[x + half] = shoup(dif, f1.x, f1.y, t.q);
         } else {
           const ulonglong2 wt = ld_tw(t.inv + (1 << s) + blk);
-          sm[x] = csub(sum, t.q2);
-          sm[x + half] = shoup_lazy(dif, wt.x, wt.y, t.q);
+          sm[x] = M::template settle<M::sum_bound(1)>(M::sum(sum, t), t);
+          sm[x + half] = M::mul(dif, wt.x, wt.y, t);
         }
       }
       __syncthreads();
@@ -124,8 +126,13 @@ __global__ void k_fwd_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, v
       ct_group<M, KK, 0, 0>(v, t.fwd, base, t);
     }
     u64* out = reinterpret_cast<u64*>(job.out);
+    if (handoff) {
+      const typename M::Out to(t);
 #pragma unroll
-    for (int j = 0; j < (1 << KK); j++) out[first + j * st] = handoff ? M::handoff(v[j], t) : v[j];
+      for (int j = 0; j < (1 << KK); j++) v[j] = to.handoff(v[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < (1 << KK); j++) out[first + j * st] = v[j];
   }
 }
 
@@ -249,46 +256,65 @@ static int split_small(int njobs, uint32_t log_n, int sms, bool single) {
   return (long)njobs * 8 <= (long)sms ? 3 : 0;
 }
 
-extern "C" int vkcu_ntt_forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
-                                uint32_t log_n, int wide, int sms) {
+// f(M{}) for the modulus class's M; the wide class has launchers of its own.
+template <class M>
+static constexpr bool kWide = std::is_same<M, Mod63>::value;
+
+template <class F>
+static int by_class(int qclass, F&& f) {
+  return qclass == VKCU_Q60 ? f(Mod60{}) : qclass == VKCU_Q62 ? f(Mod62{}) : f(Mod63{});
+}
+
+template <class M>
+static int forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one, uint32_t log_n,
+                   int sms) {
   cudaStream_t st = (cudaStream_t)stream;
   const vkcu_ntt_job o = one ? *one : vkcu_ntt_job{};
   if (log_n < 1 || log_n > (uint32_t)kMaxLogN || njobs < 1) return (int)cudaErrorInvalidValue;
   const bool aligned = jobs_aligned(jobs, one);
   if (log_n < 8 || (log_n <= (uint32_t)kMaxCta && !aligned))
-    return wide ? simple<Mod63>(st, false, jobs, njobs, o, (int)log_n, sms)
-                : simple<Mod62>(st, false, jobs, njobs, o, (int)log_n, sms);
+    return simple<M>(st, false, jobs, njobs, o, (int)log_n, sms);
   if (!aligned) return (int)cudaErrorMisalignedAddress;
-  if (wide) {
+  if constexpr (kWide<M>) {
     if (log_n <= (uint32_t)kMaxCta) return fwd_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms);
     if (log_n <= (uint32_t)kMaxCluster) return fwd_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta);
   } else {
     if (const int lc = split_small(njobs, log_n, sms, jobs == nullptr)) {
-      const int e = fwd_cluster(st, jobs, njobs, o, lc, (int)log_n - lc);
+      const int e = fwd_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc);
       // a GPU that cannot host 16-CTA clusters: the set-up refuses before any launch
-      return e == (int)cudaErrorInvalidConfiguration && lc == 4 ? fwd_cluster(st, jobs, njobs, o, 3, (int)log_n - 3)
-                                                                : e;
+      return e == (int)cudaErrorInvalidConfiguration && lc == 4
+                 ? fwd_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3)
+                 : e;
     }
-    if (log_n <= (uint32_t)kMaxCta) return fwd_cta(st, jobs, njobs, o, (int)log_n, 0, sms, vkh_variant_jobs(1, (int)log_n, njobs, sms));
-    if (log_n <= (uint32_t)kMaxCluster) return fwd_cluster(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta);
+    if (log_n <= (uint32_t)kMaxCta)
+      return fwd_cta<M>(st, jobs, njobs, o, (int)log_n, 0, sms, vkh_variant_jobs(1, (int)log_n, njobs, sms));
+    if (log_n <= (uint32_t)kMaxCluster) return fwd_cluster<M>(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta);
   }
   const int np = global_passes((int)log_n);
   for (int p = 0; p < np; p++) {
     int s0, kk;
     global_split((int)log_n, p, &s0, &kk);
-    const int e = wide ? global_pass<Mod63>(st, false, jobs, njobs, o, (int)log_n, s0, kk, p == np - 1, sms)
-                       : global_pass<Mod62>(st, false, jobs, njobs, o, (int)log_n, s0, kk, p == np - 1, sms);
+    const int e = global_pass<M>(st, false, jobs, njobs, o, (int)log_n, s0, kk, p == np - 1, sms);
     if (e) return e;
   }
   const int sub_log = (int)log_n - kMaxCta;
-  return wide ? fwd_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms)
-              : fwd_cta(st, jobs, njobs, o, kMaxCta, sub_log, sms, vkh_variant_jobs(1, kMaxCta, (long)njobs << sub_log, sms));
+  if constexpr (kWide<M>)
+    return fwd_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms);
+  else
+    return fwd_cta<M>(st, jobs, njobs, o, kMaxCta, sub_log, sms,
+                      vkh_variant_jobs(1, kMaxCta, (long)njobs << sub_log, sms));
+}
+
+extern "C" int vkcu_ntt_forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
+                                uint32_t log_n, int qclass, int sms) {
+  return by_class(qclass, [&](auto m) { return forward<decltype(m)>(stream, jobs, njobs, one, log_n, sms); });
 }
 
 static bool has_lift(const vkcu_lift* lift) { return lift && lift->count > 0; }
 
-extern "C" int vkcu_ntt_inverse_lift(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
-                                     uint32_t log_n, int wide, int sms, const vkcu_lift* lift) {
+template <class M>
+static int inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one, uint32_t log_n, int sms,
+                   const vkcu_lift* lift) {
   cudaStream_t st = (cudaStream_t)stream;
   const vkcu_ntt_job o = one ? *one : vkcu_ntt_job{};
   if (log_n < 1 || log_n > (uint32_t)kMaxLogN || njobs < 1) return (int)cudaErrorInvalidValue;
@@ -298,33 +324,36 @@ extern "C" int vkcu_ntt_inverse_lift(void* stream, const vkcu_ntt_job* jobs, int
   const vkcu_lift* lp = lifted ? lift : nullptr;
   int e;
   if (log_n < 8 || (log_n <= (uint32_t)kMaxCta && !aligned)) {
-    e = wide ? simple<Mod63>(st, true, jobs, njobs, o, (int)log_n, sms)
-             : simple<Mod62>(st, true, jobs, njobs, o, (int)log_n, sms);
+    e = simple<M>(st, true, jobs, njobs, o, (int)log_n, sms);
   } else if (!aligned) {
     return (int)cudaErrorMisalignedAddress;
-  } else if (wide && log_n <= (uint32_t)kMaxCta) {
-    return inv_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms, lp);
-  } else if (wide && log_n <= (uint32_t)kMaxCluster) {
-    return inv_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta, lp);
-  } else if (!wide && split_small(njobs, log_n, sms, jobs == nullptr)) {
-    const int lc = split_small(njobs, log_n, sms, jobs == nullptr);
-    const int e = inv_cluster(st, jobs, njobs, o, lc, (int)log_n - lc, lp);
-    return e == (int)cudaErrorInvalidConfiguration && lc == 4 ? inv_cluster(st, jobs, njobs, o, 3, (int)log_n - 3, lp)
-                                                              : e;
-  } else if (!wide && log_n <= (uint32_t)kMaxCta) {
-    if (lifted) return inv_cta_lift(st, jobs, njobs, o, (int)log_n, sms, *lift);
-    return inv_cta(st, jobs, njobs, o, (int)log_n, 0, sms, vkh_variant_jobs(2, (int)log_n, njobs, sms));
-  } else if (!wide && log_n <= (uint32_t)kMaxCluster) {
-    return inv_cluster(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta, lp);
   } else {
+    if constexpr (kWide<M>) {
+      if (log_n <= (uint32_t)kMaxCta) return inv_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms, lp);
+      if (log_n <= (uint32_t)kMaxCluster) return inv_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta, lp);
+    } else {
+      if (const int lc = split_small(njobs, log_n, sms, jobs == nullptr)) {
+        const int r = inv_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc, lp);
+        return r == (int)cudaErrorInvalidConfiguration && lc == 4
+                   ? inv_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3, lp)
+                   : r;
+      }
+      if (log_n <= (uint32_t)kMaxCta) {
+        if (lifted) return inv_cta_lift<M>(st, jobs, njobs, o, (int)log_n, sms, *lift);
+        return inv_cta<M>(st, jobs, njobs, o, (int)log_n, 0, sms, vkh_variant_jobs(2, (int)log_n, njobs, sms));
+      }
+      if (log_n <= (uint32_t)kMaxCluster) return inv_cluster<M>(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta, lp);
+    }
     const int sub_log = (int)log_n - kMaxCta;
-    e = wide ? inv_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms, nullptr)
-             : inv_cta(st, jobs, njobs, o, kMaxCta, sub_log, sms, vkh_variant_jobs(2, kMaxCta, (long)njobs << sub_log, sms));
+    if constexpr (kWide<M>)
+      e = inv_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms, nullptr);
+    else
+      e = inv_cta<M>(st, jobs, njobs, o, kMaxCta, sub_log, sms,
+                     vkh_variant_jobs(2, kMaxCta, (long)njobs << sub_log, sms));
     for (int p = global_passes((int)log_n) - 1; !e && p >= 0; p--) {
       int s0, kk;
       global_split((int)log_n, p, &s0, &kk);
-      e = wide ? global_pass<Mod63>(st, true, jobs, njobs, o, (int)log_n, s0, kk, 0, sms)
-               : global_pass<Mod62>(st, true, jobs, njobs, o, (int)log_n, s0, kk, 0, sms);
+      e = global_pass<M>(st, true, jobs, njobs, o, (int)log_n, s0, kk, 0, sms);
     }
   }
   // the multi-launch paths take the epilogue as one more element-wise launch
@@ -332,38 +361,53 @@ extern "C" int vkcu_ntt_inverse_lift(void* stream, const vkcu_ntt_job* jobs, int
   return e;
 }
 
-extern "C" int vkcu_ntt_inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
-                                uint32_t log_n, int wide, int sms) {
-  return vkcu_ntt_inverse_lift(stream, jobs, njobs, one, log_n, wide, sms, nullptr);
+extern "C" int vkcu_ntt_inverse_lift(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
+                                     uint32_t log_n, int qclass, int sms, const vkcu_lift* lift) {
+  return by_class(qclass, [&](auto m) { return inverse<decltype(m)>(stream, jobs, njobs, one, log_n, sms, lift); });
 }
 
-extern "C" int vkcu_polymul_lift(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one,
-                                 uint32_t log_n, int wide, int sms, const vkcu_lift* lift, int b_ntt) {
+extern "C" int vkcu_ntt_inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
+                                uint32_t log_n, int qclass, int sms) {
+  return vkcu_ntt_inverse_lift(stream, jobs, njobs, one, log_n, qclass, sms, nullptr);
+}
+
+template <class M>
+static int polymul(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one, uint32_t log_n,
+                   int sms, const vkcu_lift* lift, int b_ntt) {
   cudaStream_t st = (cudaStream_t)stream;
   const vkcu_poly_job o = one ? *one : vkcu_poly_job{};
   if (log_n < 8 || log_n > (uint32_t)kMaxCluster || njobs < 1) return (int)cudaErrorInvalidValue;
   if (has_lift(lift) && lift->count > VKCU_MAX_LIFT) return (int)cudaErrorInvalidValue;
   static const vkcu_lift kNoSteps{};  // the epilogue instantiations with nothing to apply
   const vkcu_lift* lp = has_lift(lift) ? lift : b_ntt ? &kNoSteps : nullptr;
-  if (wide) {
+  if constexpr (kWide<M>) {
     if (log_n <= (uint32_t)kMaxCta) return poly_cta_wide(st, jobs, njobs, o, (int)log_n, sms, lp);
     return poly_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta, lp);
+  } else {
+    if (const int lc = split_small(njobs, log_n, sms, jobs == nullptr)) {
+      const int e = poly_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc, lp);
+      return e == (int)cudaErrorInvalidConfiguration && lc == 4
+                 ? poly_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3, lp)
+                 : e;
+    }
+    if (log_n <= (uint32_t)kMaxCta) {
+      const int variant = vkh_variant_jobs(0, (int)log_n, njobs, sms);
+      if (lp) return poly_cta_lift<M>(st, jobs, njobs, o, (int)log_n, sms, variant, *lp);
+      return poly_cta<M>(st, jobs, njobs, o, (int)log_n, sms, variant);
+    }
+    return poly_cluster<M>(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta, lp);
   }
-  if (const int lc = split_small(njobs, log_n, sms, jobs == nullptr)) {
-    const int e = poly_cluster(st, jobs, njobs, o, lc, (int)log_n - lc, lp);
-    return e == (int)cudaErrorInvalidConfiguration && lc == 4 ? poly_cluster(st, jobs, njobs, o, 3, (int)log_n - 3, lp)
-                                                              : e;
-  }
-  if (log_n <= (uint32_t)kMaxCta) {
-    if (lp) return poly_cta_lift(st, jobs, njobs, o, (int)log_n, sms, vkh_variant_jobs(0, (int)log_n, njobs, sms), *lp);
-    return poly_cta(st, jobs, njobs, o, (int)log_n, sms, vkh_variant_jobs(0, (int)log_n, njobs, sms));
-  }
-  return poly_cluster(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta, lp);
+}
+
+extern "C" int vkcu_polymul_lift(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one,
+                                 uint32_t log_n, int qclass, int sms, const vkcu_lift* lift, int b_ntt) {
+  return by_class(qclass,
+                  [&](auto m) { return polymul<decltype(m)>(stream, jobs, njobs, one, log_n, sms, lift, b_ntt); });
 }
 
 extern "C" int vkcu_polymul(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one,
-                            uint32_t log_n, int wide, int sms) {
-  return vkcu_polymul_lift(stream, jobs, njobs, one, log_n, wide, sms, nullptr, 0);
+                            uint32_t log_n, int qclass, int sms) {
+  return vkcu_polymul_lift(stream, jobs, njobs, one, log_n, qclass, sms, nullptr, 0);
 }
 
 // The epilogue as its own element-wise pass: over `len` words at p, or over
@@ -568,7 +612,9 @@ __global__ void __launch_bounds__(256) k_pointwise(const vkcu_poly_job* __restri
     const long base = (ch & (cpj - 1)) << lw;
     u64* c = reinterpret_cast<u64*>(job.c) + base;
     const u64* y = reinterpret_cast<const u64*>(job.scratch) + base;
-    auto prod = [&](u64 x, u64 b) { return M::product_out(x, ref_reduce64_maybe(b, t.q, t.mu, t.qbits), t); };
+    const u64 mu = t.mu();
+    const u32 qbits = t.qbits();
+    auto prod = [&](u64 x, u64 b) { return M::product_out(x, ref_reduce64_maybe(b, t.q, mu, qbits), t, mu, qbits); };
     for (int p = (int)threadIdx.x; p < pairs; p += 2 * (int)blockDim.x) {
       const int p1 = p + (int)blockDim.x;
       const bool two = p1 < pairs;
@@ -584,15 +630,14 @@ __global__ void __launch_bounds__(256) k_pointwise(const vkcu_poly_job* __restri
   }
 }
 
-extern "C" int vkcu_pointwise(void* stream, const vkcu_poly_job* jobs, int njobs, uint32_t log_n, int wide, int sms) {
+extern "C" int vkcu_pointwise(void* stream, const vkcu_poly_job* jobs, int njobs, uint32_t log_n, int qclass, int sms) {
   if (njobs < 1 || !jobs || log_n < 1) return (int)cudaErrorInvalidValue;
   const long chunks = (long)njobs << (log_n > 11 ? log_n - 11 : 0);
   long blocks = chunks;
   if (blocks > (long)sms * 8) blocks = (long)sms * 8;
-  if (wide)
-    k_pointwise<Mod63><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(jobs, njobs, (int)log_n);
-  else
-    k_pointwise<Mod62><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(jobs, njobs, (int)log_n);
-  vkcu_count_launches(1);
-  return (int)cudaGetLastError();
+  return by_class(qclass, [&](auto m) {
+    k_pointwise<decltype(m)><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(jobs, njobs, (int)log_n);
+    vkcu_count_launches(1);
+    return (int)cudaGetLastError();
+  });
 }

@@ -37,8 +37,8 @@ namespace cg = cooperative_groups;
 
 namespace vk {
 
-using SubShape = Shape<14, 32>;  // the large-n sub-block
-using SubShape63 = Shape<14, 32, 1, Mod63>;  // the same for 2^62 <= q < 2^63
+template <class M>
+using SubShape = Shape<14, 32, 1, M>;  // the large-n sub-block
 
 template <int LOGC, class S>
 struct Cols {
@@ -151,8 +151,9 @@ __global__ void __launch_bounds__(S::T, 1)
     cl.sync();
     fwd_first_smem<S>(sm, t, tw_mult);
     fwd_passes<S>(sm, t, tw_mult, [&](int g, u64(&v)[16]) {
+      const typename S::M::Out to(t);
 #pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = S::M::canon(v[j], t);
+      for (int j = 0; j < 16; j++) v[j] = to.canon(v[j]);
       store16(v, out + 16 * g);
     });
   }
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(S::T, 1)
 #pragma unroll 1
   for (int w = cid; w < njobs; w += ncl) {
     const vkcu_poly_job job = fetch_job(jobs, one, w);
-    const Tw t = load_tw(job.tw);
+    const Tw t = load_tw_product<typename S::M>(job.tw);
     // b holds NTT(b): phase 0 is skipped (read by the epilogue instantiations only)
     const bool b_ntt = LIFT && (job.flags & VKCU_JOB_B_NTT);
     u64* scratch = (b_ntt ? const_cast<u64*>(reinterpret_cast<const u64*>(job.b)) : reinterpret_cast<u64*>(job.scratch)) +
@@ -223,15 +224,17 @@ __global__ void __launch_bounds__(S::T, 1)
       fwd_passes<S>(sm, t, tw_mult, [&](int g, u64(&v)[16]) {
         using M = typename S::M;
         if (ph == 0) {
+          const typename M::Out to(t);
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] = M::canon(v[j], t);
+          for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
           store16(v, scratch + 16 * g);
         } else {
           u64 bh[16];
           load16(bh, scratch + 16 * g);
           if (b_ntt) reduce_operand16(bh, t);
+          const typename M::Product product(t);
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] = M::product(v[j], bh[j], t);
+          for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
           // the sub-block's first inverse pass (stages HEAD + 3 .. HEAD) on the same words
           gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, t.inv, tw_mult * (u32)(S::N / 16) + (u32)g, t);
 #pragma unroll
@@ -301,37 +304,71 @@ static int launch_cluster(cudaStream_t st, int njobs, Args... args) {
 
 // Sub-blocks of 2^9 .. 2^13 words for n = 2^12 .. 2^16 on 8 CTAs (16 words
 // per thread; 32 at 2^13, so that 256 threads fit the register file).
-using Small9 = Shape<9, 16>;
-using Small10 = Shape<10, 16>;
-using Small11 = Shape<11, 16>;
-using Small12 = Shape<12, 16>;
-using Small13 = Shape<13, 32>;
+template <class M>
+using Small9 = Shape<9, 16, 1, M>;
+template <class M>
+using Small10 = Shape<10, 16, 1, M>;
+template <class M>
+using Small11 = Shape<11, 16, 1, M>;
+template <class M>
+using Small12 = Shape<12, 16, 1, M>;
+template <class M>
+using Small13 = Shape<13, 32, 1, M>;
 
 // logc: cluster size 2^logc; logs: sub-block size 2^logs (14, or 9 .. 13
 // with logc = 3, or 10 .. 12 with logc = 4: n = 2^14 .. 2^16 on 16 CTAs, a
 // cluster size the GPU allows on request).
 #define VK_CLUSTER_SHAPES(X)                                 \
   switch (logc * 32 + logs) {                                \
-    case 1 * 32 + 14: return X(1, SubShape);                 \
-    case 2 * 32 + 14: return X(2, SubShape);                 \
-    case 3 * 32 + 14: return X(3, SubShape);                 \
-    case 3 * 32 + 9: return X(3, Small9);                    \
-    case 3 * 32 + 10: return X(3, Small10);                  \
-    case 3 * 32 + 11: return X(3, Small11);                  \
-    case 3 * 32 + 12: return X(3, Small12);                  \
-    case 3 * 32 + 13: return X(3, Small13);                  \
-    case 4 * 32 + 10: return X(4, Small10);                  \
-    case 4 * 32 + 11: return X(4, Small11);                  \
-    case 4 * 32 + 12: return X(4, Small12);                  \
+    case 1 * 32 + 14: return X(1, SubShape<M>);                 \
+    case 2 * 32 + 14: return X(2, SubShape<M>);                 \
+    case 3 * 32 + 14: return X(3, SubShape<M>);                 \
+    case 3 * 32 + 9: return X(3, Small9<M>);                    \
+    case 3 * 32 + 10: return X(3, Small10<M>);                  \
+    case 3 * 32 + 11: return X(3, Small11<M>);                  \
+    case 3 * 32 + 12: return X(3, Small12<M>);                  \
+    case 3 * 32 + 13: return X(3, Small13<M>);                  \
+    case 4 * 32 + 10: return X(4, Small10<M>);                  \
+    case 4 * 32 + 11: return X(4, Small11<M>);                  \
+    case 4 * 32 + 12: return X(4, Small12<M>);                  \
     default: return (int)cudaErrorInvalidValue;              \
   }
 
-// The lifted inverse and polymul kernels are instantiated in their own
-// translation units (ntt_cluster_inv_lift.cu, ntt_cluster_poly_lift.cu) so
-// that the cluster kernels compile in parallel.
+// The launchers (ntt_core.cuh declares them) are instantiated per modulus
+// class, the lifted inverse and polymul kernels in their own translation
+// units, so that the cluster kernels compile in parallel.
+template <class M>
 int inv_cluster_lifted(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int logc,
                        int logs, const vkcu_lift& lift);
+template <class M>
 int poly_cluster_lifted(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int logc,
                         int logs, const vkcu_lift& lift);
+
+template <class M>
+int fwd_cluster(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int logc, int logs) {
+#define X(L, S) launch_cluster<L, S, k_ntt_fwd_cluster<L, S>>(st, njobs, jobs, njobs, one)
+  VK_CLUSTER_SHAPES(X)
+#undef X
+}
+
+template <class M>
+int inv_cluster(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int logc, int logs,
+                const vkcu_lift* lift) {
+  if (lift) return inv_cluster_lifted<M>(st, jobs, njobs, one, logc, logs, *lift);
+  const vkcu_lift l{};
+#define X(L, S) launch_cluster<L, S, k_ntt_inv_cluster<L, S, false>>(st, njobs, jobs, njobs, one, l)
+  VK_CLUSTER_SHAPES(X)
+#undef X
+}
+
+template <class M>
+int poly_cluster(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int logc, int logs,
+                 const vkcu_lift* lift) {
+  if (lift) return poly_cluster_lifted<M>(st, jobs, njobs, one, logc, logs, *lift);
+  const vkcu_lift l{};
+#define X(L, S) launch_cluster<L, S, k_polymul_cluster<L, S, false>>(st, njobs, jobs, njobs, one, l)
+  VK_CLUSTER_SHAPES(X)
+#undef X
+}
 
 }  // namespace vk

@@ -1,13 +1,8 @@
-// Fused polynomial multiply on a thread-block cluster with a fused lift epilogue.
-#include "ntt_cluster.cuh"
+// Fused polynomial multiply on a thread-block cluster with a fused lift epilogue: odd q < 2^60.
+#include "ntt_cluster_lift.cuh"
 
 namespace vk {
 
-int poly_cluster_lifted(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int logc,
-                        int logs, const vkcu_lift& l) {
-#define X(L, S) launch_cluster<L, S, k_polymul_cluster<L, S, true>>(st, njobs, jobs, njobs, one, l)
-  VK_CLUSTER_SHAPES(X)
-#undef X
-}
+template int poly_cluster_lifted<Mod60>(cudaStream_t, const vkcu_poly_job*, int, const vkcu_poly_job&, int, int, const vkcu_lift&);
 
 }  // namespace vk

@@ -25,11 +25,11 @@
 //     pass in the same registers;
 //   * the last inverse pass folds n^-1 into its final stage and writes global
 //     memory coalesced.
-// Butterflies are lazy (Harvey): values stay in [0, 4q) (forward) or [0, 2q)
-// (inverse) and are made canonical once at the end.  That needs 4q <= 2^64;
-// moduli 2^62 <= q < 2^63 (the top of the reference's range: its inverse-mod
-// works below 2^63, src/numbers.c:71-99) run the same kernels instantiated
-// with the Mod63 class below, whose values stay in [0, 2q) both ways.
+// Butterflies are lazy (Harvey): values stay in [0, kq) and are made canonical
+// once at the end, k as large as 64 bits allow: 12 for q < 2^60, 4 for q <
+// 2^62, 2 for q < 2^63 (the top of the reference's range: its inverse-mod
+// works below 2^63, src/numbers.c:71-99).  The kernels are templates over
+// these modulus classes (Mod60, Mod62, Mod63 below).
 //
 // Bit-exactness for unreduced inputs.  The reference's first stage computes
 // (X + WY) mod 2^64 mod q and (X - WY) mod q (forward), or (X + Y) mod 2^64
@@ -83,34 +83,65 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// Per-transform constants, loaded once per job into registers.
+// A constant that is needed late in a kernel, loaded where it is used (an L1
+// or L2 hit) instead of holding registers from the start: volatile, so that
+// the compiler does not hoist it.
+__device__ __forceinline__ u64 ld_late(const u64* p) {
+  u64 r;
+  asm volatile("ld.global.nc.u64 %0, [%1];" : "=l"(r) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ u32 ld_late32(const u32* p) {
+  u32 r;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(r) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ ulonglong2 ld_late2(const ulonglong2* p) {
+  ulonglong2 r;
+  asm volatile("ld.global.nc.v2.u64 {%0,%1}, [%2];" : "=l"(r.x), "=l"(r.y) : "l"(p));
+  return r;
+}
+
+// Per-transform constants: the modulus and the tables in registers, the rest
+// of the set loaded where it is used.
 struct Tw {
-  u64 q, q2, mu, ninv, ninv_s, w1ninv, w1ninv_s;
-  u32 qbits;
+  u64 q, q2;
   const ulonglong2* fwd;
   const ulonglong2* inv;
+  const ulonglong2* fold;  // (n^-1, shoup), (w1 n^-1, shoup) of the last inverse stage
+  const vkcu_twset* set;
+  __device__ __forceinline__ u64 mu() const { return ld_late(reinterpret_cast<const u64*>(&set->mu)); }
+  __device__ __forceinline__ u64 qinv() const { return ld_late(reinterpret_cast<const u64*>(&set->qinv)); }
+  __device__ __forceinline__ u32 qbits() const { return ld_late32(&set->qbits); }
 };
 
 __device__ __forceinline__ Tw load_tw(const vkcu_twset* p) {
   Tw t;
   t.q = __ldg(reinterpret_cast<const u64*>(&p->q));
   t.q2 = __ldg(reinterpret_cast<const u64*>(&p->q2));
-  t.mu = __ldg(reinterpret_cast<const u64*>(&p->mu));
-  t.ninv = __ldg(reinterpret_cast<const u64*>(&p->ninv));
-  t.ninv_s = __ldg(reinterpret_cast<const u64*>(&p->ninv_s));
-  t.w1ninv = __ldg(reinterpret_cast<const u64*>(&p->w1ninv));
-  t.w1ninv_s = __ldg(reinterpret_cast<const u64*>(&p->w1ninv_s));
-  t.qbits = __ldg(&p->qbits);
   t.fwd = reinterpret_cast<const ulonglong2*>(__ldg(reinterpret_cast<const u64*>(&p->fwd)));
   t.inv = reinterpret_cast<const ulonglong2*>(__ldg(reinterpret_cast<const u64*>(&p->inv)));
+  t.fold = reinterpret_cast<const ulonglong2*>(&p->ninv);
+  t.set = p;
+  return t;
+}
+
+// The same for a fused product, whose last stage takes what M::Product left
+// (divided by 2^64 by a Montgomery product).
+template <class M>
+__device__ __forceinline__ Tw load_tw_product(const vkcu_twset* p) {
+  Tw t = load_tw(p);
+  if (M::MONTGOMERY) t.fold = reinterpret_cast<const ulonglong2*>(&p->ninv_m);
   return t;
 }
 
 // A caller-supplied NTT(b) operand reduced as the reference's elemmul reduces
 // its operands (reduce64, elemmul.comp:36-47): canonical words pass through.
 __device__ __forceinline__ void reduce_operand16(u64 (&v)[16], const Tw& t) {
+  const u64 mu = t.mu();
+  const u32 qbits = t.qbits();
 #pragma unroll
-  for (int j = 0; j < 16; j++) v[j] = ref_reduce64_maybe(v[j], t.q, t.mu, t.qbits);
+  for (int j = 0; j < 16; j++) v[j] = ref_reduce64_maybe(v[j], t.q, mu, qbits);
 }
 
 // ---------------------------------------------------------------------------
@@ -120,10 +151,12 @@ struct U2 {
   u64 x, y;
 };
 
-// The reference's stage-0 butterfly for x >= 2q, exactly: X' = (X + WY) mod
+// The reference's stage-0 butterfly for x past the fast path's bound, exactly: X' = (X + WY) mod
 // 2^64 mod q, Y' = (X - WY) mod q.  Kept out of line: it is rarely taken.
 // reduce64 is an exact remainder for q < 2^62.
-static __device__ __noinline__ U2 ct_first_slow(u64 x, u64 y, u64 w, u64 wp, u64 q, u64 mu, u32 qbits) {
+static __device__ __noinline__ U2 ct_first_slow(u64 x, u64 y, u64 w, u64 wp, u64 q, const vkcu_twset* set) {
+  const u64 mu = set->mu;
+  const u32 qbits = set->qbits;
   const u64 wy = shoup(y, w, wp, q);
   const u64 xr = ref_reduce64(x, q, mu, qbits);
   return U2{ref_reduce64(x + wy, q, mu, qbits), xr >= wy ? xr - wy : xr + q - wy};
@@ -132,7 +165,9 @@ static __device__ __noinline__ U2 ct_first_slow(u64 x, u64 y, u64 w, u64 wp, u64
 // Inverse, stage m = n/2: the sum s and difference d before the twiddle
 // product, exactly as the reference's (X + Y) mod 2^64 mod q and the
 // residue of its `while (t < Y) t += q; t -= Y` loop.
-static __device__ __noinline__ U2 gs_first_slow(u64 x, u64 y, u64 q, u64 mu, u32 qbits) {
+static __device__ __noinline__ U2 gs_first_slow(u64 x, u64 y, u64 q, const vkcu_twset* set) {
+  const u64 mu = set->mu;
+  const u32 qbits = set->qbits;
   const u64 xr = ref_reduce64(x, q, mu, qbits);
   const u64 yr = ref_reduce64(y, q, mu, qbits);
   return U2{ref_reduce64(x + y, q, mu, qbits), xr >= yr ? xr - yr : xr + q - yr};
@@ -152,6 +187,31 @@ static __device__ __noinline__ U2 gs_first_slow63(u64 x, u64 y, u64 q) {
 
 // ---------------------------------------------------------------------------
 // Modulus classes: the butterfly arithmetic every kernel is instantiated with.
+// A class M gives
+//   ct<REDUCE>   a forward butterfly; REDUCE brings x down first, which the
+//                passes ask for in the sub-stages where reduce_at(u)
+//   sd<B>        sum and difference of two inverse words below B units before
+//                the twiddle product (a unit is the inverse passes' resting
+//                bound); the sum, after sum(), is below sum_bound(B) units
+//   mul          the twiddle product of a difference, below one unit
+//   settle<B>    a word below B units brought below one unit
+//   Out          forward words -> canonical, parked (NTT(b) held for the
+//                pointwise product) or handed to the next kernel's first stage
+//   Product      the pointwise product of a forward word and a parked or
+//                canonical one, below one unit (MONTGOMERY: times 2^-64)
+//   product_out  of two canonical words, the word the reference's elemmul stores
+//
+// Mod60 (odd q < 2^60): sixteen q fit in 64 bits.  The Shoup quotient leaves
+// out one of four 32-bit products and may be two short, so a twiddle product
+// is below 3q; forward words stay below 12q, x being brought below 6q in every
+// second stage only (12q -> 6q, then 9q, then 12q); inverse words rest below
+// 3q between passes and grow by sums inside a pass, at most to 12q, which the
+// compiler follows word by word (gs_bound below): 20 conditional subtractions
+// for the 32 butterflies of a radix-16 group instead of 32.  The pointwise
+// step is a Montgomery product, its 2^64 folded into the last stage's n^-1.
+// Against Mod62 on the same primes: 256 products of 2^14 words 168.0 -> 149.7
+// us, 3003 of 2^10 87.4 -> 75.1 us, 64 of 2^16 202.7 -> 182.5 us, 1000 forward
+// transforms of 2^14 208 -> 192 us, 150 inverse ones of 2^15 88.1 -> 82.0 us.
 //
 // Mod62 (q < 2^62): forward values in [0, 4q), inverse values in [0, 2q), one
 // conditional subtraction per butterfly (Harvey).  The pointwise product is
@@ -166,84 +226,187 @@ static __device__ __noinline__ U2 gs_first_slow63(u64 x, u64 y, u64 q) {
 // are not the true residues, and the polymul must reproduce them; the
 // inverse stage that follows then takes the exact first-stage rule, since
 // such a word need not be below q.
+struct Mod60 {
+  static constexpr bool EXACT_AFTER_PRODUCT = false, MONTGOMERY = true;
+  static constexpr bool reduce_at(int u) { return (u & 1) == 0; }
+  template <bool REDUCE>
+  __device__ __forceinline__ static void ct(u64& x, u64& y, u64 w, u64 wp, const Tw& t) {
+    const u64 q3 = t.q + t.q2;
+    const u64 xr = REDUCE ? csub_sign(x, 2 * q3) : x;
+    const u64 wy = shoup_lazy3(y, w, wp, 0 - t.q);
+    x = xr + wy;
+    y = xr - wy + q3;
+  }
+  // words below B units of 3q; 4 units come down to 2 first
+  template <int B>
+  __device__ __forceinline__ static void sd(u64 x, u64 y, const Tw& t, u64& s, u64& d) {
+    const u64 q3 = t.q + t.q2;
+    if (B == 4) {
+      x = csub_sign(x, 2 * q3);
+      y = csub_sign(y, 2 * q3);
+    }
+    s = x + y;
+    d = x - y + (B == 1 ? q3 : 2 * q3);
+  }
+  static constexpr int sum_bound(int b) { return b == 1 ? 2 : 4; }
+  __device__ __forceinline__ static u64 sum(u64 s, const Tw&) { return s; }
+  __device__ __forceinline__ static u64 mul(u64 d, u64 w, u64 wp, const Tw& t) {
+    return shoup_lazy3(d, w, wp, 0 - t.q);
+  }
+  template <int B>
+  __device__ __forceinline__ static u64 settle(u64 x, const Tw& t) {
+    const u64 q3 = t.q + t.q2;
+    if (B == 4) x = csub_sign(x, 2 * q3);
+    if (B >= 2) x = csub_sign(x, q3);
+    return x;
+  }
+  // A forward word (below 12q) below 2q: the quotient from its top 27 bits and
+  // floor(2^(qbits + 4) / q), at most 32, is short by less than 1 (its floor)
+  // + 0.75 (the 32's) + 2^-22 (the bits left out); all products fit 32 bits.
+  struct Out {
+    u64 q;
+    u32 m, sh, sh2;
+    __device__ __forceinline__ explicit Out(const Tw& t) : q(t.q) {
+      const u32 bits = t.qbits();
+      m = (u32)(t.mu() >> 58);
+      sh = bits > 23 ? bits - 23 : 0;
+      sh2 = bits + 4 - sh;
+    }
+    __device__ __forceinline__ u64 park(u64 x) const {
+      const u32 k = ((u32)(x >> sh) * m) >> sh2;
+      const u64 nq = 0 - q;
+      const u64 r = mad_wide(k, lo32(nq), x);
+      return pack(lo32(r), hi32(r) + k * hi32(nq));
+    }
+    __device__ __forceinline__ u64 canon(u64 x) const { return csub_sign(park(x), q); }
+    __device__ __forceinline__ u64 handoff(u64 x) const { return park(x); }
+  };
+  // x < 12q and y < 2q: (x y - ((x y) q^-1 mod 2^64) q) / 2^64 + q, below
+  // 24 q q / 2^64 + q < 2.5q
+  struct Product {
+    u64 q, qinv;
+    __device__ __forceinline__ explicit Product(const Tw& t) : q(t.q), qinv(t.qinv()) {}
+    __device__ __forceinline__ u64 operator()(u64 x, u64 y) const {
+      return mulhi_chain(x, y) - mulhi_chain(x * y * qinv, q) + q;
+    }
+  };
+  __device__ __forceinline__ static u64 product_out(u64 x, u64 y, const Tw& t, u64 mu, u32 qbits) {
+    return csub(barrett_mul_lazy(x, y, t.q, t.q2, mu, qbits), t.q);
+  }
+  // first-stage fast paths: the lazy butterfly is congruent to the reference's
+  __device__ __forceinline__ static bool fwd_fast(u64 x, const Tw& t) { return x < t.q + t.q2; }
+  __device__ __forceinline__ static bool inv_fast(u64 x, u64 y, const Tw& t) {
+    return x < t.q + t.q2 && y < t.q + t.q2;
+  }
+  __device__ __forceinline__ static U2 ct_slow(u64 x, u64 y, u64 w, u64 wp, const Tw& t) {
+    return ct_first_slow(x, y, w, wp, t.q, t.set);
+  }
+  __device__ __forceinline__ static U2 gs_slow(u64 x, u64 y, const Tw& t) { return gs_first_slow(x, y, t.q, t.set); }
+};
+
 struct Mod62 {
-  static constexpr bool EXACT_AFTER_PRODUCT = false;
+  static constexpr bool EXACT_AFTER_PRODUCT = false, MONTGOMERY = false;
+  static constexpr bool reduce_at(int) { return true; }
+  template <bool REDUCE>
   __device__ __forceinline__ static void ct(u64& x, u64& y, u64 w, u64 wp, const Tw& t) {
     ct_bfly(x, y, w, wp, t.q, t.q2);
   }
-  __device__ __forceinline__ static void gs(u64& x, u64& y, u64 w, u64 wp, const Tw& t) {
-    gs_bfly(x, y, w, wp, t.q, t.q2);
-  }
-  // sum and difference of two inverse-lazy words before the twiddle product
+  template <int B>
   __device__ __forceinline__ static void sd(u64 x, u64 y, const Tw& t, u64& s, u64& d) {
     s = x + y;
     d = x - y + t.q2;
   }
-  // forward-lazy word -> canonical
-  __device__ __forceinline__ static u64 canon(u64 x, const Tw& t) { return canon4(x, t.q, t.q2); }
-  // forward-lazy word -> below the next kernel's first-stage fast-path bound
-  __device__ __forceinline__ static u64 handoff(u64 x, const Tw& t) { return csub(x, t.q2); }
-  // first-stage fast paths: the lazy butterfly is congruent to the reference's
+  static constexpr int sum_bound(int) { return 1; }
+  __device__ __forceinline__ static u64 sum(u64 s, const Tw& t) { return csub(s, t.q2); }
+  __device__ __forceinline__ static u64 mul(u64 d, u64 w, u64 wp, const Tw& t) { return shoup_lazy(d, w, wp, t.q); }
+  template <int B>
+  __device__ __forceinline__ static u64 settle(u64 x, const Tw&) {
+    return x;
+  }
+  struct Out {
+    u64 q, q2;
+    __device__ __forceinline__ explicit Out(const Tw& t) : q(t.q), q2(t.q2) {}
+    __device__ __forceinline__ u64 canon(u64 x) const { return canon4(x, q, q2); }
+    __device__ __forceinline__ u64 park(u64 x) const { return canon(x); }
+    __device__ __forceinline__ u64 handoff(u64 x) const { return csub(x, q2); }
+  };
+  struct Product {
+    u64 q, q2, mu;
+    u32 qbits;
+    __device__ __forceinline__ explicit Product(const Tw& t) : q(t.q), q2(t.q2), mu(t.mu()), qbits(t.qbits()) {}
+    __device__ __forceinline__ u64 operator()(u64 x, u64 y) const {
+      return barrett_mul_lazy(canon4(x, q, q2), y, q, q2, mu, qbits);
+    }
+  };
+  __device__ __forceinline__ static u64 product_out(u64 x, u64 y, const Tw& t, u64 mu, u32 qbits) {
+    return csub(barrett_mul_lazy(x, y, t.q, t.q2, mu, qbits), t.q);
+  }
   __device__ __forceinline__ static bool fwd_fast(u64 x, const Tw& t) { return x < t.q2; }
   __device__ __forceinline__ static bool inv_fast(u64 x, u64 y, const Tw& t) { return x < t.q2 && y < t.q2; }
   __device__ __forceinline__ static U2 ct_slow(u64 x, u64 y, u64 w, u64 wp, const Tw& t) {
-    return ct_first_slow(x, y, w, wp, t.q, t.mu, t.qbits);
+    return ct_first_slow(x, y, w, wp, t.q, t.set);
   }
-  __device__ __forceinline__ static U2 gs_slow(u64 x, u64 y, const Tw& t) {
-    return gs_first_slow(x, y, t.q, t.mu, t.qbits);
-  }
-  // pointwise product of a forward-lazy word and a canonical one: an
-  // inverse-lazy word (fused kernels) ...
-  __device__ __forceinline__ static u64 product(u64 x, u64 y, const Tw& t) {
-    return barrett_mul_lazy(canon4(x, t.q, t.q2), y, t.q, t.q2, t.mu, t.qbits);
-  }
-  // ... or, from two canonical words, the word the reference's elemmul stores
-  __device__ __forceinline__ static u64 product_out(u64 x, u64 y, const Tw& t) {
-    return csub(barrett_mul_lazy(x, y, t.q, t.q2, t.mu, t.qbits), t.q);
-  }
+  __device__ __forceinline__ static U2 gs_slow(u64 x, u64 y, const Tw& t) { return gs_first_slow(x, y, t.q, t.set); }
 };
 
 struct Mod63 {
-  static constexpr bool EXACT_AFTER_PRODUCT = true;
+  static constexpr bool EXACT_AFTER_PRODUCT = true, MONTGOMERY = false;
+  static constexpr bool reduce_at(int) { return true; }
+  template <bool REDUCE>
   __device__ __forceinline__ static void ct(u64& x, u64& y, u64 w, u64 wp, const Tw& t) {
     const u64 xr = csub(x, t.q);
     const u64 wy = csub(shoup_lazy(y, w, wp, t.q), t.q);
     x = xr + wy;
     y = xr - wy + t.q;
   }
+  template <int B>
   __device__ __forceinline__ static void sd(u64 x, u64 y, const Tw& t, u64& s, u64& d) {
     const u64 xr = csub(x, t.q), yr = csub(y, t.q);
     s = xr + yr;
     d = xr - yr + t.q;
   }
-  __device__ __forceinline__ static void gs(u64& x, u64& y, u64 w, u64 wp, const Tw& t) {
-    u64 s, d;
-    sd(x, y, t, s, d);
-    x = s;
-    y = shoup_lazy(d, w, wp, t.q);
+  static constexpr int sum_bound(int) { return 1; }
+  __device__ __forceinline__ static u64 sum(u64 s, const Tw&) { return s; }
+  __device__ __forceinline__ static u64 mul(u64 d, u64 w, u64 wp, const Tw& t) { return shoup_lazy(d, w, wp, t.q); }
+  template <int B>
+  __device__ __forceinline__ static u64 settle(u64 x, const Tw&) {
+    return x;
   }
-  __device__ __forceinline__ static u64 canon(u64 x, const Tw& t) { return csub(x, t.q); }
-  __device__ __forceinline__ static u64 handoff(u64 x, const Tw& t) { return csub(x, t.q); }
+  struct Out {
+    u64 q;
+    __device__ __forceinline__ explicit Out(const Tw& t) : q(t.q) {}
+    __device__ __forceinline__ u64 canon(u64 x) const { return csub(x, q); }
+    __device__ __forceinline__ u64 park(u64 x) const { return csub(x, q); }
+    __device__ __forceinline__ u64 handoff(u64 x) const { return csub(x, q); }
+  };
+  // the reference's elemmul on canonical operands (its reduce64 returns them
+  // unchanged): the full 128-bit product through reduce128
+  struct Product {
+    u64 q, mu;
+    u32 qbits;
+    __device__ __forceinline__ explicit Product(const Tw& t) : q(t.q), mu(t.mu()), qbits(t.qbits()) {}
+    __device__ __forceinline__ u64 operator()(u64 x, u64 y) const {
+      const u64 xc = csub(x, q);
+      return ref_reduce128(mulhi(xc, y), xc * y, q, mu, qbits);
+    }
+  };
+  __device__ __forceinline__ static u64 product_out(u64 x, u64 y, const Tw& t, u64 mu, u32 qbits) {
+    return ref_reduce128(mulhi(x, y), x * y, t.q, mu, qbits);
+  }
   __device__ __forceinline__ static bool fwd_fast(u64 x, const Tw& t) { return x < t.q; }
   __device__ __forceinline__ static bool inv_fast(u64 x, u64 y, const Tw& t) { return x < t.q && y < t.q; }
   __device__ __forceinline__ static U2 ct_slow(u64 x, u64 y, u64 w, u64 wp, const Tw& t) {
     return ct_first_slow63(x, y, w, wp, t.q);
   }
   __device__ __forceinline__ static U2 gs_slow(u64 x, u64 y, const Tw& t) { return gs_first_slow63(x, y, t.q); }
-  // the reference's elemmul on canonical operands (its reduce64 returns them
-  // unchanged): the full 128-bit product through reduce128
-  __device__ __forceinline__ static u64 product_out(u64 x, u64 y, const Tw& t) {
-    return ref_reduce128(mulhi(x, y), x * y, t.q, t.mu, t.qbits);
-  }
-  __device__ __forceinline__ static u64 product(u64 x, u64 y, const Tw& t) { return product_out(csub(x, t.q), y, t); }
 };
 
 // Forward, stage m = 1, with the reference's exact rule for inputs outside
-// the fast path (x >= 2q for Mod62: then x + WY < 3q < 2^64 no longer holds).
+// the fast path (x + WY could wrap past 2^64 there).
 template <class M>
 __device__ __forceinline__ void ct_first(u64& x, u64& y, u64 w, u64 wp, const Tw& t) {
   if (M::fwd_fast(x, t)) {
-    M::ct(x, y, w, wp, t);
+    M::template ct<false>(x, y, w, wp, t);
   } else {
     const U2 r = M::ct_slow(x, y, w, wp, t);
     x = r.x;
@@ -255,7 +418,7 @@ __device__ __forceinline__ void ct_first(u64& x, u64& y, u64 w, u64 wp, const Tw
 template <class M>
 __device__ __forceinline__ void gs_first_sd(u64 x, u64 y, const Tw& t, u64& s, u64& d) {
   if (M::inv_fast(x, y, t)) {
-    M::sd(x, y, t, s, d);
+    M::template sd<1>(x, y, t, s, d);
   } else {
     const U2 r = M::gs_slow(x, y, t);
     s = r.x;
@@ -279,50 +442,61 @@ __device__ __forceinline__ void ct_group(u64 (&v)[NV], const ulonglong2* tw, u32
       const ulonglong2 w = ld_tw(tw + ((base << u) + r));
 #pragma unroll
       for (int jj = 0; jj < half; jj++)
-        M::ct(v[G0 + r * 2 * half + jj], v[G0 + r * 2 * half + jj + half], w.x, w.y, t);
+        M::template ct<M::reduce_at(u)>(v[G0 + r * 2 * half + jj], v[G0 + r * 2 * half + jj + half], w.x, w.y, t);
     });
   });
 }
 
-// Inverse group: sub-stages KK-1 .. 0.  EXACT_TOP applies the exact rule to
-// sub-stage KK-1 (global stage m = n/2); FOLD folds n^-1 into sub-stage 0
-// (global stage m = 1, root index 1) and leaves canonical outputs.
+// Bound, in units, of word j of an inverse group of 2^KK words when sub-stage
+// u begins: bit KK-1-s of j tells whether sub-stage s left it a sum or a
+// twiddle product (below one unit); all words begin below one unit.
+template <class M>
+constexpr int gs_bound(int KK, int u, int j) {
+  int b = 1;
+  for (int s = KK - 1; s > u; s--) b = ((j >> (KK - 1 - s)) & 1) ? 1 : M::sum_bound(b);
+  return b;
+}
+
+// Inverse group: sub-stages KK-1 .. 0, words below one unit before and after.
+// EXACT_TOP applies the exact rule to sub-stage KK-1 (global stage m = n/2);
+// FOLD folds n^-1 into sub-stage 0 (global stage m = 1, root index 1) and
+// leaves canonical outputs.
 template <class M, int KK, int G0, bool EXACT_TOP, bool FOLD, int NV>
 __device__ __forceinline__ void gs_group(u64 (&v)[NV], const ulonglong2* tw, u32 base, const Tw& t) {
   static_for<0, KK>([&](auto uc) {
     constexpr int u = KK - 1 - decltype(uc)::value;
     constexpr int half = 1 << (KK - 1 - u);
-    if constexpr (FOLD && u == 0) {
-#pragma unroll
-      for (int jj = 0; jj < half; jj++) {
-        u64& x = v[G0 + jj];
-        u64& y = v[G0 + jj + half];
-        u64 s, d;
-        if constexpr (EXACT_TOP && u == KK - 1) {
-          gs_first_sd<M>(x, y, t, s, d);
-        } else {
-          M::sd(x, y, t, s, d);
-        }
-        x = shoup(s, t.ninv, t.ninv_s, t.q);
-        y = shoup(d, t.w1ninv, t.w1ninv_s, t.q);
+    // (both words of a butterfly have the same bound: they differ in a later bit)
+    auto sums = [&](auto jc, u64& s, u64& d) {
+      constexpr int j = decltype(jc)::value;
+      if constexpr (EXACT_TOP && u == KK - 1) {
+        gs_first_sd<M>(v[G0 + j], v[G0 + j + half], t, s, d);
+      } else {
+        M::template sd<gs_bound<M>(KK, u, j)>(v[G0 + j], v[G0 + j + half], t, s, d);
       }
+    };
+    if constexpr (FOLD && u == 0) {
+      const ulonglong2 f0 = ld_late2(t.fold), f1 = ld_late2(t.fold + 1);
+      static_for<0, half>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        u64 s, d;
+        sums(jc, s, d);
+        v[G0 + j] = shoup(s, f0.x, f0.y, t.q);
+        v[G0 + j + half] = shoup(d, f1.x, f1.y, t.q);
+      });
     } else {
       static_for<0, (1 << u)>([&](auto rc) {
         constexpr int r = decltype(rc)::value;
         const ulonglong2 w = ld_tw(tw + ((base << u) + r));
-#pragma unroll
-        for (int jj = 0; jj < half; jj++) {
-          u64& x = v[G0 + r * 2 * half + jj];
-          u64& y = v[G0 + r * 2 * half + jj + half];
-          if constexpr (EXACT_TOP && u == KK - 1) {
-            u64 s, d;
-            gs_first_sd<M>(x, y, t, s, d);
-            x = csub(s, t.q2);
-            y = shoup_lazy(d, w.x, w.y, t.q);
-          } else {
-            M::gs(x, y, w.x, w.y, t);
-          }
-        }
+        static_for<r * 2 * half, r * 2 * half + half>([&](auto jc) {
+          constexpr int j = decltype(jc)::value;
+          u64 s, d;
+          sums(jc, s, d);
+          s = M::sum(s, t);
+          if constexpr (u == 0) s = M::template settle<M::sum_bound(gs_bound<M>(KK, 0, j))>(s, t);
+          v[G0 + j] = s;
+          v[G0 + j + half] = M::mul(d, w.x, w.y, t);
+        });
       });
     }
   });
@@ -339,7 +513,7 @@ __device__ __forceinline__ void gs_group(u64 (&v)[NV], const ulonglong2* tw, u32
 // a direction share one loop body (the stage offset is a runtime value), and
 // the fused polymul runs its two forward transforms through the same code.
 
-template <int LOGN_, int E_, int U_ = 1, class M_ = Mod62, bool DUAL_ = false>
+template <int LOGN_, int E_, int U_ = 1, class M_ = Mod60, bool DUAL_ = false>
 struct Shape {
   using M = M_;  // modulus class
   // DUAL: the CTA holds 2 T threads running two transforms of this shape in
@@ -380,7 +554,7 @@ constexpr int round_groups() {
 // in rounds of 16 (all of a round's loads in flight at once; 32 words at once
 // would spill), then FIRSTK stages per group, results to shared memory.
 // The first sub-stage uses the exact first-stage rule; after the global pass
-// of a large transform the inputs are < 2q and always take its fast path.
+// of a large transform the inputs always take its fast path.
 template <class S>
 __device__ __forceinline__ void fwd_first(u64* sm, const u64* __restrict__ in, const Tw& t, u32 tw_mult) {
   constexpr int KK = S::FIRSTK, G = S::E >> KK, TMIN = S::N >> KK;
@@ -642,7 +816,7 @@ __device__ __forceinline__ J fetch_job(const J* jobs, const J& one, int jid) {
 // (transforms of 2^(LOGN + sub_log) words after / before the global passes),
 // sub-block `sub` using twiddle multiplier 2^sub_log + sub.
 
-template <int LOGN, int E, int U, class M = Mod62>
+template <int LOGN, int E, int U, class M = Mod60>
 __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     k_ntt_fwd(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int sub_log) {
   using S = Shape<LOGN, E, U, M>;
@@ -658,15 +832,16 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     const u32 tw_mult = (1u << sub_log) + sub;
     fwd_first<S>(sm, in, t, tw_mult);
     fwd_passes<S>(sm, t, tw_mult, [&](int g, u64(&v)[16]) {
+      const typename M::Out to(t);
 #pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = M::canon(v[j], t);
+      for (int j = 0; j < 16; j++) v[j] = to.canon(v[j]);
       store16(v, out + 16 * g);
     });
   }
 }
 
 // LIFT: the epilogue `lift` follows the last stage (sub_log == 0 only).
-template <int LOGN, int E, int U, bool LIFT = false, class M = Mod62>
+template <int LOGN, int E, int U, bool LIFT = false, class M = Mod60>
 __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     k_ntt_inv(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int sub_log,
               const __grid_constant__ vkcu_lift lift) {
@@ -709,12 +884,12 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
 }
 
 // Fused c = INTT(NTT(a) . NTT(b)).  Phase 0 transforms b and parks NTT(b)
-// (canonical) in job.scratch; phase 1 transforms a with the same code, and its
+// in job.scratch; phase 1 transforms a with the same code, and its
 // last pass multiplies by NTT(b) (read back at the words this thread wrote)
 // and runs the first inverse pass on the products in the same registers; the
 // rest of the inverse transform then writes c.  a is prefetched
 // into L2 while b is transformed, the next job's b while a is.
-template <int LOGN, int E, int U, bool LIFT = false, class M = Mod62>
+template <int LOGN, int E, int U, bool LIFT = false, class M = Mod60>
 __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
     k_polymul(const vkcu_poly_job* __restrict__ jobs, int njobs, vkcu_poly_job one,
               const __grid_constant__ vkcu_lift lift) {
@@ -724,7 +899,7 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
 #pragma unroll 1
   for (int w = blockIdx.x; w < njobs; w += gridDim.x) {
     const vkcu_poly_job job = fetch_job(jobs, one, w);
-    const Tw t = load_tw(job.tw);
+    const Tw t = load_tw_product<M>(job.tw);
     // b holds NTT(b): phase 0 is skipped (read by the epilogue instantiations only)
     const bool b_ntt = LIFT && (job.flags & VKCU_JOB_B_NTT);
     u64* scratch = b_ntt ? const_cast<u64*>(reinterpret_cast<const u64*>(job.b)) : reinterpret_cast<u64*>(job.scratch);
@@ -738,15 +913,17 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
       }
       fwd_passes<S>(sm, t, 1u, [&](int g, u64(&v)[16]) {
         if (ph == 0) {
+          const typename M::Out to(t);
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] = M::canon(v[j], t);
+          for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
           store16(v, scratch + 16 * g);
         } else {
           u64 bh[16];
           load16(bh, scratch + 16 * g);
           if (b_ntt) reduce_operand16(bh, t);
+          const typename M::Product product(t);
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] = M::product(v[j], bh[j], t);
+          for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
           // the first inverse pass (stages HEAD + 3 .. HEAD) on the same 16 words
           gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, t.inv, (1u << S::HEAD) + (u32)g, t);
 #pragma unroll
@@ -763,25 +940,34 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
 // ---------------------------------------------------------------------------
 // Host side: per-family launchers (one translation unit each).
 
+// M: Mod60 or Mod62 (Mod63 has launchers of its own below).
 // variant: 0 = default shape, 1 = two radix-16 groups per thread in flight,
 // 2 = the other words-per-thread shape (2^10..2^13 only); others -> 0.
+template <class M>
 int fwd_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sub_log,
             int sms, int variant);
+template <class M>
 int inv_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sub_log,
             int sms, int variant);
+template <class M>
 int poly_cta(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int log_n, int sms,
              int variant);
 // With an epilogue, one CTA per transform: the inverse in the default shape
 // of each degree, the polymul in the variant given.
+template <class M>
 int inv_cta_lift(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sms,
                  const vkcu_lift& lift);
+template <class M>
 int poly_cta_lift(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int log_n, int sms,
                   int variant, const vkcu_lift& lift);
 // cluster of 2^logc CTAs with sub-blocks of 2^logs words, n = 2^(logc + logs):
 // logs = 14 for n = 2^15 .. 2^17; logc = 3 with logs = 10 / 11 for n = 2^13 / 2^14
+template <class M>
 int fwd_cluster(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int logc, int logs);
+template <class M>
 int inv_cluster(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int logc, int logs,
                 const vkcu_lift* lift = nullptr);
+template <class M>
 int poly_cluster(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int logc, int logs,
                  const vkcu_lift* lift = nullptr);
 

@@ -1,30 +1,9 @@
-// Launcher of the CTA-resident fused polynomial multiplies with a fused
-// epilogue (the reference's centred-lift element-wise ops after the inverse
-// transform) for 2^8 <= n <= 2^14, every shape variant of each degree.
-#include "ntt_core.cuh"
+// CTA-resident fused polynomial multiplies with a fused
+// epilogue, every shape variant of each degree: odd q < 2^60.
+#include "ntt_launch.cuh"
 
 namespace vk {
 
-template <int LOGN, int E, int U>
-static int launch_lift(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int sms,
-                       const vkcu_lift& lift) {
-  using S = Shape<LOGN, E, U>;
-  auto kern = k_polymul<LOGN, E, U, true>;
-  static KernelSetup setup;
-  int per_sm = 1;
-  if (const int e = setup_cta(kern, S::T, S::SMEM_BYTES, setup, &per_sm)) return e;
-  const int grid = grid_from(per_sm, (long)njobs, sms);
-  kern<<<grid, S::T, S::SMEM_BYTES, st>>>(jobs, njobs, one, lift);
-  vkcu_count_launches(1);
-  return (int)cudaGetLastError();
-}
-
-int poly_cta_lift(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int log_n, int sms,
-                  int variant, const vkcu_lift& lift) {
-retry:
-#define X(L, E, U) launch_lift<L, E, U>(st, jobs, njobs, one, sms, lift)
-  VK_FOR_LOGN(X)
-#undef X
-}
+template int poly_cta_lift<Mod60>(cudaStream_t, const vkcu_poly_job*, int, const vkcu_poly_job&, int, int, int, const vkcu_lift&);
 
 }  // namespace vk

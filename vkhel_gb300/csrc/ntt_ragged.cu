@@ -1,5 +1,5 @@
 // One persistent launch for a ragged batch of fused limb products of degrees
-// 2^12 .. 2^16 (q < 2^62, no epilogue): clusters of four CTAs of 512 threads,
+// 2^12 .. 2^16 (odd q < 2^60, no epilogue): clusters of four CTAs of 512 threads,
 // each CTA with the 2^14-word shared block of the other kernels.
 //
 // The work is a table of items in decreasing size, taken in order through
@@ -26,7 +26,7 @@ namespace vk {
 
 using R16 = Shape<14, 32>;                       // 2^16 / 2^15 sub-blocks and 2^14 products
 using R13 = Shape<13, 16>;                       // 2^13 products, 512 threads
-using R12 = Shape<12, 16, 1, Mod62, true>;       // two 2^12 products, 256 threads each
+using R12 = Shape<12, 16, 1, Mod60, true>;       // two 2^12 products, 256 threads each
 constexpr int kRaggedThreads = 512;
 static_assert(R16::T == kRaggedThreads && R13::T == kRaggedThreads && 2 * R12::T == kRaggedThreads, "CTA shapes");
 
@@ -34,21 +34,23 @@ static_assert(R16::T == kRaggedThreads && R13::T == kRaggedThreads && 2 * R12::T
 template <class S>
 __device__ __noinline__ void ragged_cta_product(u64* sm, const vkcu_poly_job& job) {
   using M = typename S::M;
-  const Tw t = load_tw(job.tw);
+  const Tw t = load_tw_product<M>(job.tw);
   u64* scratch = reinterpret_cast<u64*>(job.scratch);
 #pragma unroll 1
   for (int ph = 0; ph < 2; ph++) {
     fwd_first<S>(sm, reinterpret_cast<const u64*>(ph ? job.a : job.b), t, 1u);
     fwd_passes<S>(sm, t, 1u, [&](int g, u64(&v)[16]) {
       if (ph == 0) {
+        const typename M::Out to(t);
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = M::canon(v[j], t);
+        for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
         store16(v, scratch + 16 * g);
       } else {
         u64 bh[16];
         load16(bh, scratch + 16 * g);
+        const typename M::Product product(t);
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = M::product(v[j], bh[j], t);
+        for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
         gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, t.inv, (1u << S::HEAD) + (u32)g, t);
 #pragma unroll
         for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
@@ -69,7 +71,7 @@ __device__ __noinline__ void ragged_cluster_product(u64* sm, const cg::cluster_g
   using K = Cols<LOGC, S>;
   using M = typename S::M;
   const u32 tw_mult = (u32)(K::C + rank);
-  const Tw t = load_tw(job.tw);
+  const Tw t = load_tw_product<M>(job.tw);
   u64* scratch = reinterpret_cast<u64*>(job.scratch) + (size_t)rank * K::SUB;
 #pragma unroll 1
   for (int ph = 0; ph < 2; ph++) {
@@ -79,14 +81,16 @@ __device__ __noinline__ void ragged_cluster_product(u64* sm, const cg::cluster_g
     fwd_first_smem<S>(sm, t, tw_mult);
     fwd_passes<S>(sm, t, tw_mult, [&](int g, u64(&v)[16]) {
       if (ph == 0) {
+        const typename M::Out to(t);
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = M::canon(v[j], t);
+        for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
         store16(v, scratch + 16 * g);
       } else {
         u64 bh[16];
         load16(bh, scratch + 16 * g);
+        const typename M::Product product(t);
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = M::product(v[j], bh[j], t);
+        for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
         gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, t.inv, tw_mult * (u32)(S::N / 16) + (u32)g, t);
 #pragma unroll
         for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];

@@ -4,32 +4,37 @@
 // one mul.hi.u64 and two mul.lo.u64, each several IMADs), not by HBM, and the
 // device peaks recorded for this machine cover only copy bandwidth and dense
 // bf16.  These kernels measure, on the running GPU:
-//   * butterflies/s: independent lazy Cooley-Tukey butterflies (the exact
-//     instruction sequence of the transforms, ct_bfly) with all operands in
-//     registers, 16 independent chains per thread, grid = 4 CTAs x 256
-//     threads per SM;
+//   * butterflies/s: independent lazy Cooley-Tukey butterflies (those of the
+//     transforms for q < 2^60, Mod60::ct, with and without the subtraction in
+//     turn) with all operands in registers, 16 independent chains per thread,
+//     grid = 4 CTAs x 256 threads per SM;
 //   * IMAD/s: independent 32-bit multiply-adds (mad.lo.u32), same shape.
 // Each kernel folds its results into one store so nothing is dead code.
 #include <cuda_runtime.h>
 
-#include "arith.cuh"
 #include "kernels.h"
+#include "ntt_core.cuh"
 
 namespace vk {
 
 constexpr int kChains = 16;
 
-__global__ void __launch_bounds__(256) k_peak_bfly(const u64* __restrict__ seed, u64* __restrict__ sink, int iters) {
-  const u64 q = seed[0], q2 = 2 * q, w = seed[1], wp = seed[2];
+__global__ void __launch_bounds__(256, 2) k_peak_bfly(const u64* __restrict__ seed, u64* __restrict__ sink, int iters) {
+  const u64 q = seed[0], w = seed[1], wp = seed[2];
+  Tw t{};
+  t.q = q;
+  t.q2 = 2 * q;
   u64 x[kChains], y[kChains];
 #pragma unroll
   for (int c = 0; c < kChains; c++) {
     x[c] = (seed[3] + threadIdx.x * 131 + c * 7) % q;
     y[c] = (seed[4] + blockIdx.x * 17 + c * 3) % q;
   }
-  for (int it = 0; it < iters; it++) {
+  for (int it = 0; it < iters; it += 2) {
 #pragma unroll
-    for (int c = 0; c < kChains; c++) ct_bfly(x[c], y[c], w, wp, q, q2);
+    for (int c = 0; c < kChains; c++) Mod60::ct<true>(x[c], y[c], w, wp, t);
+#pragma unroll
+    for (int c = 0; c < kChains; c++) Mod60::ct<false>(x[c], y[c], w, wp, t);
   }
   u64 acc = 0;
 #pragma unroll

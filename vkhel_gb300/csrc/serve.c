@@ -41,9 +41,9 @@
 #include "internal.h"
 
 /* classes of one micro-batch: one per (degree, modulus class, resident
- * operand or not) present, at most 4 per degree 2^1 .. 2^26; the first
+ * operand or not) present, at most 6 per degree 2^1 .. 2^26; the first
  * SRV_AUX + 1 of them can run on concurrent streams */
-#define SRV_MAX_CLASSES 104
+#define SRV_MAX_CLASSES 156
 #define SRV_AUX 32
 /* At low load (the micro-batch took every queued request) a micro-batch of
  * at most SRV_CHUNKS requests and at least 2 SRV_CHUNK_MIN bytes of operands
@@ -203,17 +203,17 @@ static int issue_chunk(struct vkhel_server *s, struct srv_slot *sl, uint32_t c, 
 	qsort(keys + j0, j1 - j0, sizeof(uint64_t), cmp_job_log_n);
 	for (uint32_t i = j0; i < j1; i++) {
 		const uint32_t log_n = (uint32_t) (keys[i] >> 40);
-		const int wide = (int) ((keys[i] >> 39) & 1);
-		const uint32_t b_ntt = (uint32_t) ((keys[i] >> 38) & 1);
-		sl->host_poly[i] = tmp[keys[i] & 0x3fffffffffull];
-		if (nclasses == 0 || classes[nclasses - 1].log_n != log_n || classes[nclasses - 1].wide != wide ||
+		const int qclass = (int) ((keys[i] >> 38) & 3);
+		const uint32_t b_ntt = (uint32_t) ((keys[i] >> 37) & 1);
+		sl->host_poly[i] = tmp[keys[i] & 0x1fffffffffull];
+		if (nclasses == 0 || classes[nclasses - 1].log_n != log_n || classes[nclasses - 1].qclass != qclass ||
 				classes[nclasses - 1].b_ntt != b_ntt) {
 			if (nclasses == SRV_MAX_CLASSES)
 				return VKHEL_ERR_UNSUPPORTED;
 			struct vkh_job_class *cl = &classes[nclasses++];
 			cl->kind = VKH_JOB_POLYMUL;
 			cl->log_n = log_n;
-			cl->wide = wide;
+			cl->qclass = qclass;
 			cl->lift = 0;
 			cl->b_ntt = b_ntt;
 			cl->first = i;
@@ -295,8 +295,8 @@ static void launch_slot(struct vkhel_server *s, struct srv_slot *sl) {
 				j.scratch = fused ? j.c : base + 3 * words + (uint64_t) k * r->n;
 			}
 			j.tw = d->dev_set;
-			keys[njobs] = ((uint64_t) r->log_n << 40) | ((uint64_t) vkcu_wide(r->tables[k]->q) << 39) |
-					((uint64_t) (r->op != NULL) << 38) | njobs;
+			keys[njobs] = ((uint64_t) r->log_n << 40) | ((uint64_t) vkcu_qclass(r->tables[k]->q) << 38) |
+					((uint64_t) (r->op != NULL) << 37) | njobs;
 			tmp[njobs++] = j;
 			acc += up_per_word(r) * r->n;
 			const int last = i + 1 == sl->nreqs && k + 1 == r->limbs;
@@ -400,7 +400,7 @@ static int upload_operand(struct vkhel_server *s, struct srv_operand *op) {
 			break;
 		uint64_t *p = (uint64_t *) op->dev + (uint64_t) k * op->n;
 		const vkcu_ntt_job j = {p, p, d->dev_set};
-		e = vkcu_ntt_forward(s->s_in, NULL, 1, &j, op->log_n, vkcu_wide(op->tables[k]->q), ctx->sms);
+		e = vkcu_ntt_forward(s->s_in, NULL, 1, &j, op->log_n, vkcu_qclass(op->tables[k]->q), ctx->sms);
 	}
 	const int se = vkcu_sync(s->s_in);
 	if (!e)

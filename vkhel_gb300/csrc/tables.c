@@ -219,6 +219,15 @@ int vkh_devtab_get(struct vkhel_ctx *ctx, const struct vkhel_ntt_tables *t,
 	s.ninv_s = t->ninv_s;
 	s.w1ninv = t->w1ninv;
 	s.w1ninv_s = t->w1ninv_s;
+	if (t->q & 1) {
+		s.qinv = t->q; /* Newton: q q = 1 mod 8, then twice the bits each step */
+		for (int i = 0; i < 5; i++)
+			s.qinv *= 2 - t->q * s.qinv;
+		s.ninv_m = (uint64_t) (((u128) t->ninv << 64) % t->q);
+		s.ninv_m_s = vkh_shoup(s.ninv_m, t->q);
+		s.w1ninv_m = (uint64_t) (((u128) t->w1ninv << 64) % t->q);
+		s.w1ninv_m_s = vkh_shoup(s.w1ninv_m, t->q);
+	}
 	s.qbits = t->qbits;
 	s.log_n = t->log_n;
 	s.fwd = (const uint64_t *) ((char *) mem + head);
