@@ -14,10 +14,44 @@
 extern "C" {
 #endif
 
+#ifdef __CUDACC__
+#define VKCU_HD __host__ __device__
+#else
+#define VKCU_HD
+#endif
+
+/* Where root i of the reference's bit-reversed order (src/ntt_tables.c:25-43)
+ * lies in a device table of n = 2^log_n entries.  The last four stages act on
+ * groups of 16 consecutive words: sub-stage u of group G takes the roots
+ * ((n/16 + G) << u) + r, r < 2^u.  In that order neighbouring threads
+ * (groups) would read 2^u entries apart, a 128-byte line each in the last
+ * stage, so for n >= 2^8 those roots lie in rows of n/16 entries instead: row
+ * 2^u + r, column G.  Roots below n/16 (the stages before) keep their place
+ * (row 0).  vkcu_tw_root is the inverse map. */
+#define VKCU_TW_ROWS_LOG_N 8
+static inline VKCU_HD uint32_t vkcu_tw_slot(uint32_t log_n, uint32_t i) {
+	uint32_t u = 0;
+	if (log_n < VKCU_TW_ROWS_LOG_N || i >> (log_n - 4) == 0)
+		return i;
+	while (i >> (log_n - 4 + u + 1))
+		u++;
+	return ((((uint32_t) 1 << u) + (i & (((uint32_t) 1 << u) - 1))) << (log_n - 4)) + (i >> u) -
+			((uint32_t) 1 << (log_n - 4));
+}
+static inline VKCU_HD uint32_t vkcu_tw_root(uint32_t log_n, uint32_t slot) {
+	uint32_t u = 0;
+	const uint32_t row = log_n < VKCU_TW_ROWS_LOG_N ? 0 : slot >> (log_n - 4);
+	if (row == 0)
+		return slot;
+	while (row >> (u + 1))
+		u++;
+	return ((slot - (row << (log_n - 4)) + ((uint32_t) 1 << (log_n - 4))) << u) + row - ((uint32_t) 1 << u);
+}
+
 /* Device-resident constants of one (n, q, w) twiddle set.  `fwd` and `inv`
- * point to n interleaved (root, shoup(root)) pairs in the reference's
- * bit-reversed order (src/ntt_tables.c:25-43).  Each (factor, Shoup factor)
- * pair lies on a 16-byte boundary: the kernels load it as one vector. */
+ * point to n interleaved (root, shoup(root)) pairs, root i in slot
+ * vkcu_tw_slot(log_n, i).  Each (factor, Shoup factor) pair lies on a 16-byte
+ * boundary: the kernels load it as one vector. */
 typedef struct vkcu_twset {
 	uint64_t q, q2;              /* q, 2q */
 	uint64_t mu, qinv;           /* floor(2^(bits+62)/q); q^-1 mod 2^64 (odd q) */

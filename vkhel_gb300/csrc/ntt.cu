@@ -31,7 +31,7 @@ __global__ void k_ntt_fwd_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
       for (int p = threadIdx.x; p < n / 2; p += blockDim.x) {
         const int blk = p >> (log_n - 1 - s);
         const int x = blk * 2 * half + (p & (half - 1));
-        const ulonglong2 wt = ld_tw(t.fwd + (1 << s) + blk);
+        const ulonglong2 wt = ld_tw(t.fwd + vkcu_tw_slot(log_n, (1u << s) + blk));
         if (s == 0)
           ct_first<M>(sm[x], sm[x + half], wt.x, wt.y, t);
         else
@@ -72,7 +72,7 @@ __global__ void k_ntt_inv_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
           sm[x] = shoup(sum, f0.x, f0.y, t.q);
           sm[x + half] = shoup(dif, f1.x, f1.y, t.q);
         } else {
-          const ulonglong2 wt = ld_tw(t.inv + (1 << s) + blk);
+          const ulonglong2 wt = ld_tw(t.inv + vkcu_tw_slot(log_n, (1u << s) + blk));
           sm[x] = M::template settle<M::sum_bound(1)>(M::sum(sum, t), t);
           sm[x + half] = M::mul(dif, wt.x, wt.y, t);
         }
@@ -121,9 +121,9 @@ __global__ void k_fwd_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, v
       const ulonglong2 w0 = ld_tw(t.fwd + 1);
 #pragma unroll
       for (int jj = 0; jj < (1 << (KK - 1)); jj++) ct_first<M>(v[jj], v[jj + (1 << (KK - 1))], w0.x, w0.y, t);
-      ct_group<M, KK, 1, 0>(v, t.fwd, base, t);
+      ct_group<M, KK, 1, 0>(v, RowTw{t.fwd, base}, t);
     } else {
-      ct_group<M, KK, 0, 0>(v, t.fwd, base, t);
+      ct_group<M, KK, 0, 0>(v, RowTw{t.fwd, base}, t);
     }
     u64* out = reinterpret_cast<u64*>(job.out);
     if (handoff) {
@@ -157,9 +157,9 @@ __global__ void k_inv_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, v
     for (int j = 0; j < (1 << KK); j++) v[j] = out[first + j * st];
     const u32 base = (1u << s0) + (u32)blk;
     if (s0 == 0)
-      gs_group<M, KK, 0, false, true>(v, t.inv, base, t);
+      gs_group<M, KK, 0, false, true>(v, RowTw{t.inv, base}, t);
     else
-      gs_group<M, KK, 0, false, false>(v, t.inv, base, t);
+      gs_group<M, KK, 0, false, false>(v, RowTw{t.inv, base}, t);
 #pragma unroll
     for (int j = 0; j < (1 << KK); j++) out[first + j * st] = v[j];
   }

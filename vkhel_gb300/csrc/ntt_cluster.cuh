@@ -45,6 +45,7 @@ struct Cols {
   static constexpr int C = 1 << LOGC, SUB = S::N;
   static constexpr int COLS = SUB >> LOGC;  // columns per CTA
   static constexpr int PER = COLS / S::T;   // columns per thread
+  static constexpr int N16 = C * SUB / 16;  // groups of the last four stages
   static_assert(PER * C == S::E, "a column pass moves E words per thread");
   __device__ __forceinline__ static int col(int rank, int k) { return rank * COLS + (int)threadIdx.x + k * S::T; }
 };
@@ -84,7 +85,7 @@ __device__ __forceinline__ void col_fwd(const u64* __restrict__ in, u64* sm, con
 #pragma unroll
       for (int jj = 0; jj < K::C / 2; jj++)
         ct_first<typename S::M>(v[k * K::C + jj], v[k * K::C + jj + K::C / 2], w0.x, w0.y, t);
-      ct_group<typename S::M, LOGC, 1, k * K::C>(v, t.fwd, 1u, t);
+      ct_group<typename S::M, LOGC, 1, k * K::C>(v, RowTw{t.fwd, 1u}, t);
     });
     if (SPLIT && k0 == 0) cluster_wait();
 #pragma unroll
@@ -114,7 +115,7 @@ __device__ __forceinline__ void col_inv(u64* __restrict__ out, u64* sm, const cg
     }
     static_for<0, H>([&](auto kc) {
       constexpr int k = decltype(kc)::value;
-      gs_group<typename S::M, LOGC, k * K::C, false, true>(v, t.inv, 1u, t);
+      gs_group<typename S::M, LOGC, k * K::C, false, true>(v, RowTw{t.inv, 1u}, t);
     });
 #pragma unroll
     for (int k = 0; k < H; k++)
@@ -145,12 +146,13 @@ __global__ void __launch_bounds__(S::T, 1)
   for (int w = cid; w < njobs; w += ncl) {
     const vkcu_ntt_job job = fetch_job(jobs, one, w);
     const Tw t = load_tw(job.tw);
+    const LastTable<K::N16> last(t.fwd, rank * (S::N / 16), 0);
     u64* out = reinterpret_cast<u64*>(job.out) + (size_t)rank * K::SUB;
     cl.sync();
     col_fwd<LOGC, S, false>(reinterpret_cast<const u64*>(job.in), sm, cl, rank, t);
     cl.sync();
     fwd_first_smem<S>(sm, t, tw_mult);
-    fwd_passes<S>(sm, t, tw_mult, [&](int g, u64(&v)[16]) {
+    fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
       const typename S::M::Out to(t);
 #pragma unroll
       for (int j = 0; j < 16; j++) v[j] = to.canon(v[j]);
@@ -174,6 +176,7 @@ __global__ void __launch_bounds__(S::T, 1)
   for (int w = cid; w < njobs; w += ncl) {
     const vkcu_ntt_job job = fetch_job(jobs, one, w);
     const Tw t = load_tw(job.tw);
+    const LastTable<K::N16> last(t.inv, rank * (S::N / 16), 0);
     const u64* in = reinterpret_cast<const u64*>(job.in) + (size_t)rank * K::SUB;
     cl.sync();
 #pragma unroll 1
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__(S::T, 1)
       const int g = (int)threadIdx.x + i * S::T;
       u64 v[16];
       load16(v, in + 16 * g);
-      gs_group<typename S::M, 4, 0, true, false>(v, t.inv, tw_mult * (u32)(S::N / 16) + (u32)g, t);
+      gs_group<typename S::M, 4, 0, true, false>(v, last.at(g), t);
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
     }
@@ -211,8 +214,8 @@ __global__ void __launch_bounds__(S::T, 1)
     const Tw t = load_tw_product<typename S::M>(job.tw);
     // b holds NTT(b): phase 0 is skipped (read by the epilogue instantiations only)
     const bool b_ntt = LIFT && (job.flags & VKCU_JOB_B_NTT);
-    u64* scratch = (b_ntt ? const_cast<u64*>(reinterpret_cast<const u64*>(job.b)) : reinterpret_cast<u64*>(job.scratch)) +
-                   (size_t)rank * K::SUB;
+    u64* scratch = reinterpret_cast<u64*>(job.scratch) + (size_t)rank * K::SUB;
+    const LastTable<K::N16> last(t.fwd, rank * (S::N / 16), 0), last_inv(t.inv, rank * (S::N / 16), 0);
     if ((int)threadIdx.x < K::C)  // this CTA's column slices of a, for phase 1
       prefetch_l2(reinterpret_cast<const u64*>(job.a) + (size_t)threadIdx.x * K::SUB + rank * K::COLS, kSlice);
 #pragma unroll 1
@@ -221,22 +224,26 @@ __global__ void __launch_bounds__(S::T, 1)
       col_fwd<LOGC, S, true>(reinterpret_cast<const u64*>(ph ? job.a : job.b), sm, cl, rank, t);
       cl.sync();
       fwd_first_smem<S>(sm, t, tw_mult);
-      fwd_passes<S>(sm, t, tw_mult, [&](int g, u64(&v)[16]) {
+      fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
         using M = typename S::M;
         if (ph == 0) {
           const typename M::Out to(t);
 #pragma unroll
           for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
-          store16(v, scratch + 16 * g);
+          park16(v, scratch, g, S::N / 16);
         } else {
           u64 bh[16];
-          load16(bh, scratch + 16 * g);
-          if (b_ntt) reduce_operand16(bh, t);
+          if (b_ntt) {
+            load16(bh, reinterpret_cast<const u64*>(job.b) + (size_t)rank * K::SUB + 16 * g);
+            reduce_operand16(bh, t);
+          } else {
+            unpark16(bh, scratch, g, S::N / 16);
+          }
           const typename M::Product product(t);
 #pragma unroll
           for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
           // the sub-block's first inverse pass (stages HEAD + 3 .. HEAD) on the same words
-          gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, t.inv, tw_mult * (u32)(S::N / 16) + (u32)g, t);
+          gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.at(g), t);
 #pragma unroll
           for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
         }

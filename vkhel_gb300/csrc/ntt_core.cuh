@@ -429,17 +429,47 @@ __device__ __forceinline__ void gs_first_sd(u64 x, u64 y, const Tw& t, u64& s, u
 // ---------------------------------------------------------------------------
 // Register-resident radix-2^KK groups.  A group holds 2^KK words v[G0 + j]
 // at stride t_min of the transform, all inside one block of the first stage
-// of the pass; `base` = (tw_mult * m0 + block) so that the root of sub-stage u
-// and sub-block r is table[(base << u) + r].
+// of the pass; tw(u, r) is the root (and Shoup factor) of sub-stage u and
+// sub-block r.
 
-template <class M, int KK, int U0, int G0, int NV>
-__device__ __forceinline__ void ct_group(u64 (&v)[NV], const ulonglong2* tw, u32 base, const Tw& t) {
+// The roots of a pass before the last four stages: base = (tw_mult * m0 +
+// block), root (base << u) + r.
+struct RowTw {
+  const ulonglong2* p;
+  u32 base;
+  __device__ __forceinline__ ulonglong2 operator()(int u, int r) const { return ld_tw(p + ((base << u) + r)); }
+};
+
+// The roots of the last four stages, from the table's rows (vkcu_tw_slot): a
+// warp's 32 groups read 32 neighbouring entries, 4 wavefronts a load instead
+// of up to 32.  N16 = n/16 for the whole transform, 0 where it is known at run
+// time only.
+template <int N16>
+struct LastTw {
+  const ulonglong2* p;  // the group's column
+  u32 n16;
+  __device__ __forceinline__ ulonglong2 operator()(int u, int r) const {
+    return ld_tw(p + ((1u << u) + (u32)r) * (N16 ? (u32)N16 : n16));
+  }
+};
+// Those of a sub-block: at(g) for its group g.
+template <int N16>
+struct LastTable {
+  const ulonglong2* p;  // the sub-block's first column
+  u32 n16;
+  __device__ __forceinline__ LastTable(const ulonglong2* table, int first_group, u32 n16_)
+      : p(table + first_group), n16(n16_) {}
+  __device__ __forceinline__ LastTw<N16> at(int g) const { return LastTw<N16>{p + g, n16}; }
+};
+
+template <class M, int KK, int U0, int G0, int NV, class R>
+__device__ __forceinline__ void ct_group(u64 (&v)[NV], const R& tw, const Tw& t) {
   static_for<U0, KK>([&](auto uc) {
     constexpr int u = decltype(uc)::value;
     constexpr int half = 1 << (KK - 1 - u);
     static_for<0, (1 << u)>([&](auto rc) {
       constexpr int r = decltype(rc)::value;
-      const ulonglong2 w = ld_tw(tw + ((base << u) + r));
+      const ulonglong2 w = tw(u, r);
 #pragma unroll
       for (int jj = 0; jj < half; jj++)
         M::template ct<M::reduce_at(u)>(v[G0 + r * 2 * half + jj], v[G0 + r * 2 * half + jj + half], w.x, w.y, t);
@@ -461,8 +491,8 @@ constexpr int gs_bound(int KK, int u, int j) {
 // EXACT_TOP applies the exact rule to sub-stage KK-1 (global stage m = n/2);
 // FOLD folds n^-1 into sub-stage 0 (global stage m = 1, root index 1) and
 // leaves canonical outputs.
-template <class M, int KK, int G0, bool EXACT_TOP, bool FOLD, int NV>
-__device__ __forceinline__ void gs_group(u64 (&v)[NV], const ulonglong2* tw, u32 base, const Tw& t) {
+template <class M, int KK, int G0, bool EXACT_TOP, bool FOLD, int NV, class R>
+__device__ __forceinline__ void gs_group(u64 (&v)[NV], const R& tw, const Tw& t) {
   static_for<0, KK>([&](auto uc) {
     constexpr int u = KK - 1 - decltype(uc)::value;
     constexpr int half = 1 << (KK - 1 - u);
@@ -487,7 +517,7 @@ __device__ __forceinline__ void gs_group(u64 (&v)[NV], const ulonglong2* tw, u32
     } else {
       static_for<0, (1 << u)>([&](auto rc) {
         constexpr int r = decltype(rc)::value;
-        const ulonglong2 w = ld_tw(tw + ((base << u) + r));
+        const ulonglong2 w = tw(u, r);
         static_for<r * 2 * half, r * 2 * half + half>([&](auto jc) {
           constexpr int j = decltype(jc)::value;
           u64 s, d;
@@ -573,7 +603,7 @@ __device__ __forceinline__ void fwd_first(u64* sm, const u64* __restrict__ in, c
 #pragma unroll
       for (int jj = 0; jj < (1 << (KK - 1)); jj++)
         ct_first<typename S::M>(v[i * (1 << KK) + jj], v[i * (1 << KK) + jj + (1 << (KK - 1))], w0.x, w0.y, t);
-      ct_group<typename S::M, KK, 1, i * (1 << KK)>(v, t.fwd, tw_mult, t);
+      ct_group<typename S::M, KK, 1, i * (1 << KK)>(v, RowTw{t.fwd, tw_mult}, t);
       const int g = S::tid() + (i0 + i) * S::T;
 #pragma unroll
       for (int j = 0; j < (1 << KK); j++) sm[pad(g + j * TMIN)] = v[i * (1 << KK) + j];
@@ -596,7 +626,7 @@ __device__ __forceinline__ void fwd_first_smem(u64* sm, const Tw& t, u32 tw_mult
 #pragma unroll
       for (int j = 0; j < (1 << KK); j++) v[i * (1 << KK) + j] = sm[pad(g0 + i * S::T + j * TMIN)];
     static_for<0, GR>(
-        [&](auto ic) { ct_group<typename S::M, KK, 0, decltype(ic)::value * (1 << KK)>(v, t.fwd, tw_mult, t); });
+        [&](auto ic) { ct_group<typename S::M, KK, 0, decltype(ic)::value * (1 << KK)>(v, RowTw{t.fwd, tw_mult}, t); });
 #pragma unroll
     for (int i = 0; i < GR; i++)
 #pragma unroll
@@ -608,10 +638,10 @@ __device__ __forceinline__ void fwd_first_smem(u64* sm, const Tw& t, u32 tw_mult
 // Radix-16 forward passes s0 = FIRSTK, FIRSTK + 4, ..., HEAD on shared
 // memory.  The last pass hands each group (words 16g .. 16g+15) to epi(g, v)
 // instead of storing it back.  Ends with a barrier.
-template <class S, class Epi>
-__device__ __forceinline__ void fwd_passes(u64* sm, const Tw& t, u32 tw_mult, Epi&& epi) {
+template <class S, class L, class Epi>
+__device__ __forceinline__ void fwd_passes(u64* sm, const Tw& t, u32 tw_mult, const L& last, Epi&& epi) {
 #pragma unroll 1
-  for (int s0 = S::FIRSTK; s0 <= S::HEAD; s0 += 4) {
+  for (int s0 = S::FIRSTK; s0 < S::HEAD; s0 += 4) {
     const Pass16 ps(S::LOGN, s0, tw_mult);
     const int st = 1 << ps.lt;
 #pragma unroll(S::U)
@@ -621,16 +651,22 @@ __device__ __forceinline__ void fwd_passes(u64* sm, const Tw& t, u32 tw_mult, Ep
       u64 v[16];
 #pragma unroll
       for (int j = 0; j < 16; j++) v[j] = sm[pad(a0 + j * st)];
-      ct_group<typename S::M, 4, 0, 0>(v, t.fwd, ps.base(g), t);
-      if (s0 < S::HEAD) {
+      ct_group<typename S::M, 4, 0, 0>(v, RowTw{t.fwd, ps.base(g)}, t);
 #pragma unroll
-        for (int j = 0; j < 16; j++) sm[pad(a0 + j * st)] = v[j];
-      } else {
-        epi(g, v);
-      }
+      for (int j = 0; j < 16; j++) sm[pad(a0 + j * st)] = v[j];
     }
     __syncthreads();
   }
+#pragma unroll(S::U)
+  for (int i = 0; i < S::E / 16; i++) {
+    const int g = S::tid() + i * S::T;
+    u64 v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = sm[17 * g + j];  // pad(16 g + j)
+    ct_group<typename S::M, 4, 0, 0>(v, last.at(g), t);
+    epi(g, v);
+  }
+  __syncthreads();
 }
 
 // Radix-16 inverse passes s0 = s_top, s_top - 4, ..., FIRSTK on shared
@@ -648,7 +684,7 @@ __device__ __forceinline__ void inv_passes(u64* sm, const Tw& t, u32 tw_mult, in
       u64 v[16];
 #pragma unroll
       for (int j = 0; j < 16; j++) v[j] = sm[pad(a0 + j * st)];
-      gs_group<typename S::M, 4, 0, false, false>(v, t.inv, ps.base(g), t);
+      gs_group<typename S::M, 4, 0, false, false>(v, RowTw{t.inv, ps.base(g)}, t);
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(a0 + j * st)] = v[j];
     }
@@ -670,7 +706,7 @@ __device__ __forceinline__ void inv_last_smem(u64* sm, const Tw& t, u32 tw_mult)
 #pragma unroll
       for (int j = 0; j < (1 << KK); j++) v[i * (1 << KK) + j] = sm[pad(g0 + i * S::T + j * TMIN)];
     static_for<0, GR>(
-        [&](auto ic) { gs_group<typename S::M, KK, decltype(ic)::value * (1 << KK), false, false>(v, t.inv, tw_mult, t); });
+        [&](auto ic) { gs_group<typename S::M, KK, decltype(ic)::value * (1 << KK), false, false>(v, RowTw{t.inv, tw_mult}, t); });
 #pragma unroll
     for (int i = 0; i < GR; i++)
 #pragma unroll
@@ -760,9 +796,9 @@ __device__ __forceinline__ void inv_last_epi(u64* sm, const Tw& t, u32 tw_mult, 
 #pragma unroll
     for (int j = 0; j < (1 << KK); j++) v[j] = sm[pad(g + j * TMIN)];
     if (fold)
-      gs_group<typename S::M, KK, 0, false, true>(v, t.inv, tw_mult, t);
+      gs_group<typename S::M, KK, 0, false, true>(v, RowTw{t.inv, tw_mult}, t);
     else
-      gs_group<typename S::M, KK, 0, false, false>(v, t.inv, tw_mult, t);
+      gs_group<typename S::M, KK, 0, false, false>(v, RowTw{t.inv, tw_mult}, t);
 #pragma unroll
     for (int j = 0; j < (1 << KK); j++) out[g + j * TMIN] = epi(v[j]);
   }
@@ -788,6 +824,24 @@ __device__ __forceinline__ void load16(u64 (&v)[16], const u64* p) {
 __device__ __forceinline__ void store16(const u64 (&v)[16], u64* p) {
 #pragma unroll
   for (int h = 0; h < 4; h++) st4(p + 4 * h, v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+}
+
+// NTT(b) parked between the phases of a fused product: 16-byte pairs, pair jj
+// of group g (of G) at jj G + g, so that a warp moves whole lines (each thread
+// reads back what it wrote).
+__device__ __forceinline__ void park16(const u64 (&v)[16], u64* p, int g, int G) {
+#pragma unroll
+  for (int jj = 0; jj < 8; jj++)
+    asm volatile("st.global.v2.u64 [%0], {%1,%2};" ::"l"(p + 2 * (jj * G + g)), "l"(v[2 * jj]), "l"(v[2 * jj + 1])
+                 : "memory");
+}
+
+__device__ __forceinline__ void unpark16(u64 (&v)[16], const u64* p, int g, int G) {
+#pragma unroll
+  for (int jj = 0; jj < 8; jj++)
+    asm volatile("ld.global.v2.u64 {%0,%1}, [%2];"
+                 : "=l"(v[2 * jj]), "=l"(v[2 * jj + 1])
+                 : "l"(p + 2 * (jj * G + g)));
 }
 
 // Resident CTAs per SM the register budget is sized for: 512 threads per SM
@@ -816,22 +870,26 @@ __device__ __forceinline__ J fetch_job(const J* jobs, const J& one, int jid) {
 // (transforms of 2^(LOGN + sub_log) words after / before the global passes),
 // sub-block `sub` using twiddle multiplier 2^sub_log + sub.
 
-template <int LOGN, int E, int U, class M = Mod60>
+// SUB: sub_log may be above 0 (a template flag so that the others know their
+// table's row length at compile time).
+template <int LOGN, int E, int U, class M = Mod60, bool SUB = false>
 __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     k_ntt_fwd(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int sub_log) {
   using S = Shape<LOGN, E, U, M>;
   extern __shared__ u64 sm[];
+  if (!SUB) sub_log = 0;
   const int total = njobs << sub_log;
 #pragma unroll 1
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
     const vkcu_ntt_job job = fetch_job(jobs, one, w >> sub_log);
     const int sub = w & ((1 << sub_log) - 1);
     const Tw t = load_tw(job.tw);
+    const LastTable<SUB ? 0 : S::N / 16> last(t.fwd, sub * (S::N / 16), (S::N / 16) << sub_log);
     u64* out = reinterpret_cast<u64*>(job.out) + ((size_t)sub << LOGN);
     const u64* in = sub_log ? out : reinterpret_cast<const u64*>(job.in);
     const u32 tw_mult = (1u << sub_log) + sub;
     fwd_first<S>(sm, in, t, tw_mult);
-    fwd_passes<S>(sm, t, tw_mult, [&](int g, u64(&v)[16]) {
+    fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
       const typename M::Out to(t);
 #pragma unroll
       for (int j = 0; j < 16; j++) v[j] = to.canon(v[j]);
@@ -841,18 +899,20 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
 }
 
 // LIFT: the epilogue `lift` follows the last stage (sub_log == 0 only).
-template <int LOGN, int E, int U, bool LIFT = false, class M = Mod60>
+template <int LOGN, int E, int U, bool LIFT = false, class M = Mod60, bool SUB = false>
 __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     k_ntt_inv(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int sub_log,
               const __grid_constant__ vkcu_lift lift) {
   using S = Shape<LOGN, E, U, M>;
   extern __shared__ u64 sm[];
+  if (!SUB) sub_log = 0;
   const int total = njobs << sub_log;
 #pragma unroll 1
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
     const vkcu_ntt_job job = fetch_job(jobs, one, w >> sub_log);
     const int sub = w & ((1 << sub_log) - 1);
     const Tw t = load_tw(job.tw);
+    const LastTable<SUB ? 0 : S::N / 16> last(t.inv, sub * (S::N / 16), (S::N / 16) << sub_log);
     const u64* in = reinterpret_cast<const u64*>(job.in) + ((size_t)sub << LOGN);
     u64* out = reinterpret_cast<u64*>(job.out) + ((size_t)sub << LOGN);
     // the next work item's words into L2 while this one runs (2.6-3.4 % on
@@ -872,7 +932,7 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
       const int g = (int)threadIdx.x + i * S::T;
       u64 v[16];
       load16(v, in + 16 * g);
-      gs_group<M, 4, 0, true, false>(v, t.inv, tw_mult * (u32)(S::N / 16) + (u32)g, t);
+      gs_group<M, 4, 0, true, false>(v, last.at(g), t);
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
     }
@@ -902,7 +962,8 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
     const Tw t = load_tw_product<M>(job.tw);
     // b holds NTT(b): phase 0 is skipped (read by the epilogue instantiations only)
     const bool b_ntt = LIFT && (job.flags & VKCU_JOB_B_NTT);
-    u64* scratch = b_ntt ? const_cast<u64*>(reinterpret_cast<const u64*>(job.b)) : reinterpret_cast<u64*>(job.scratch);
+    u64* scratch = reinterpret_cast<u64*>(job.scratch);
+    const LastTable<S::N / 16> last(t.fwd, 0, 0), last_inv(t.inv, 0, 0);
     if (threadIdx.x < 4) prefetch_l2(reinterpret_cast<const char*>(job.a) + threadIdx.x * kChunk, kChunk);
 #pragma unroll 1
     for (int ph = b_ntt ? 1 : 0; ph < 2; ph++) {
@@ -911,21 +972,25 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
         const vkcu_poly_job nx = fetch_job(jobs, one, w + (int)gridDim.x);
         prefetch_l2(reinterpret_cast<const char*>(nx.b) + threadIdx.x * kChunk, kChunk);
       }
-      fwd_passes<S>(sm, t, 1u, [&](int g, u64(&v)[16]) {
+      fwd_passes<S>(sm, t, 1u, last, [&](int g, u64(&v)[16]) {
         if (ph == 0) {
           const typename M::Out to(t);
 #pragma unroll
           for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
-          store16(v, scratch + 16 * g);
+          park16(v, scratch, g, S::N / 16);
         } else {
           u64 bh[16];
-          load16(bh, scratch + 16 * g);
-          if (b_ntt) reduce_operand16(bh, t);
+          if (b_ntt) {
+            load16(bh, reinterpret_cast<const u64*>(job.b) + 16 * g);
+            reduce_operand16(bh, t);
+          } else {
+            unpark16(bh, scratch, g, S::N / 16);
+          }
           const typename M::Product product(t);
 #pragma unroll
           for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
           // the first inverse pass (stages HEAD + 3 .. HEAD) on the same 16 words
-          gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, t.inv, (1u << S::HEAD) + (u32)g, t);
+          gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.at(g), t);
 #pragma unroll
           for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
         }

@@ -36,22 +36,23 @@ __device__ __noinline__ void ragged_cta_product(u64* sm, const vkcu_poly_job& jo
   using M = typename S::M;
   const Tw t = load_tw_product<M>(job.tw);
   u64* scratch = reinterpret_cast<u64*>(job.scratch);
+  const LastTable<S::N / 16> last(t.fwd, 0, 0), last_inv(t.inv, 0, 0);
 #pragma unroll 1
   for (int ph = 0; ph < 2; ph++) {
     fwd_first<S>(sm, reinterpret_cast<const u64*>(ph ? job.a : job.b), t, 1u);
-    fwd_passes<S>(sm, t, 1u, [&](int g, u64(&v)[16]) {
+    fwd_passes<S>(sm, t, 1u, last, [&](int g, u64(&v)[16]) {
       if (ph == 0) {
         const typename M::Out to(t);
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
-        store16(v, scratch + 16 * g);
+        park16(v, scratch, g, S::N / 16);
       } else {
         u64 bh[16];
-        load16(bh, scratch + 16 * g);
+        unpark16(bh, scratch, g, S::N / 16);
         const typename M::Product product(t);
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
-        gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, t.inv, (1u << S::HEAD) + (u32)g, t);
+        gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.at(g), t);
 #pragma unroll
         for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
       }
@@ -73,25 +74,26 @@ __device__ __noinline__ void ragged_cluster_product(u64* sm, const cg::cluster_g
   const u32 tw_mult = (u32)(K::C + rank);
   const Tw t = load_tw_product<M>(job.tw);
   u64* scratch = reinterpret_cast<u64*>(job.scratch) + (size_t)rank * K::SUB;
+  const LastTable<K::N16> last(t.fwd, rank * (S::N / 16), 0), last_inv(t.inv, rank * (S::N / 16), 0);
 #pragma unroll 1
   for (int ph = 0; ph < 2; ph++) {
     cluster_arrive();  // done with every shared memory the column pass writes (col_fwd waits)
     col_fwd<LOGC, S, true>(reinterpret_cast<const u64*>(ph ? job.a : job.b), sm, cl, rank, t, rbase);
     cl.sync();
     fwd_first_smem<S>(sm, t, tw_mult);
-    fwd_passes<S>(sm, t, tw_mult, [&](int g, u64(&v)[16]) {
+    fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
       if (ph == 0) {
         const typename M::Out to(t);
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
-        store16(v, scratch + 16 * g);
+        park16(v, scratch, g, S::N / 16);
       } else {
         u64 bh[16];
-        load16(bh, scratch + 16 * g);
+        unpark16(bh, scratch, g, S::N / 16);
         const typename M::Product product(t);
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
-        gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, t.inv, tw_mult * (u32)(S::N / 16) + (u32)g, t);
+        gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.at(g), t);
 #pragma unroll
         for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
       }

@@ -9,8 +9,11 @@ namespace vk {
 
 int fwd_cta_wide(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n,
                  int sub_log, int sms) {
+  if (sub_log)
+    return launch_cta<Shape<14, 32, 1, Mod63>, k_ntt_fwd<14, 32, 1, Mod63, true>>(st, (long)njobs << sub_log, sms, jobs,
+                                                                                   njobs, one, sub_log);
 #define X(L, E, U) \
-  launch_cta<Shape<L, E, U, Mod63>, k_ntt_fwd<L, E, U, Mod63>>(st, (long)njobs << sub_log, sms, jobs, njobs, one, sub_log)
+  launch_cta<Shape<L, E, U, Mod63>, k_ntt_fwd<L, E, U, Mod63>>(st, (long)njobs, sms, jobs, njobs, one, 0)
   VK_FOR_LOGN_DEFAULT(X)
 #undef X
 }

@@ -15,9 +15,11 @@ int inv_cta_wide(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkc
 #undef X
   }
   const vkcu_lift none{};
-#define X(L, E, U)                                                                                                \
-  launch_cta<Shape<L, E, U, Mod63>, k_ntt_inv<L, E, U, false, Mod63>>(st, (long)njobs << sub_log, sms, jobs, njobs, \
-                                                                       one, sub_log, none)
+  if (sub_log)
+    return launch_cta<Shape<14, 32, 1, Mod63>, k_ntt_inv<14, 32, 1, false, Mod63, true>>(
+        st, (long)njobs << sub_log, sms, jobs, njobs, one, sub_log, none);
+#define X(L, E, U) \
+  launch_cta<Shape<L, E, U, Mod63>, k_ntt_inv<L, E, U, false, Mod63>>(st, (long)njobs, sms, jobs, njobs, one, 0, none)
   VK_FOR_LOGN_DEFAULT(X)
 #undef X
 }

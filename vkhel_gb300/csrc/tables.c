@@ -253,10 +253,11 @@ int vkh_devtab_get(struct vkhel_ctx *ctx, const struct vkhel_ntt_tables *t,
 	} else {
 		uint64_t *fwd = host + head / 8, *inv = fwd + 2 * n;
 		for (uint64_t i = 0; i < n; i++) {
-			fwd[2 * i] = t->roots[i];
-			fwd[2 * i + 1] = t->roots_shoup[i];
-			inv[2 * i] = t->inv_roots[i];
-			inv[2 * i + 1] = t->inv_roots_shoup[i];
+			const uint64_t at = vkcu_tw_slot(t->log_n, (uint32_t) i);
+			fwd[2 * at] = t->roots[i];
+			fwd[2 * at + 1] = t->roots_shoup[i];
+			inv[2 * at] = t->inv_roots[i];
+			inv[2 * at + 1] = t->inv_roots_shoup[i];
 		}
 		st = vkcu_h2d(ctx->stream, mem, host, bytes);
 	}
@@ -298,14 +299,15 @@ int vkhel_ntt_tables_device_copy(struct vkhel_ctx *ctx, const struct vkhel_ntt_t
 		e = vkcu_sync(ctx->stream);
 	if (!e) {
 		for (uint64_t i = 0; i < n; i++) {
+			const uint64_t at = vkcu_tw_slot(t->log_n, (uint32_t) i);
 			if (roots)
-				roots[i] = h[2 * i];
+				roots[i] = h[2 * at];
 			if (roots_shoup)
-				roots_shoup[i] = h[2 * i + 1];
+				roots_shoup[i] = h[2 * at + 1];
 			if (inv_roots)
-				inv_roots[i] = h[2 * n + 2 * i];
+				inv_roots[i] = h[2 * n + 2 * at];
 			if (inv_roots_shoup)
-				inv_roots_shoup[i] = h[2 * n + 2 * i + 1];
+				inv_roots_shoup[i] = h[2 * n + 2 * at + 1];
 		}
 	}
 	free(h);
