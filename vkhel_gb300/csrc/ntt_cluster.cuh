@@ -181,14 +181,13 @@ __global__ void __launch_bounds__(S::T, 1)
     cl.sync();
 #pragma unroll 1
     for (int i = 0; i < S::E / 16; i++) {
-      const int g = (int)threadIdx.x + i * S::T;
+      const int g = S::group(i);
       u64 v[16];
       load16(v, in + 16 * g);
       gs_group<typename S::M, 4, 0, true, false>(v, last.at(g), t);
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
     }
-    __syncthreads();
     inv_passes<S>(sm, t, tw_mult, S::HEAD - 4);
     inv_last_smem<S>(sm, t, tw_mult);
     cl.sync();

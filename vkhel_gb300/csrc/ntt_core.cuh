@@ -558,6 +558,32 @@ struct Shape {
   static_assert(E >= 16 && (E % 16) == 0 && HEAD >= 1 && T >= 1, "unsupported shape");
   // this thread's index within its transform
   __device__ __forceinline__ static int tid() { return DUAL ? (int)(threadIdx.x & (T - 1)) : (int)threadIdx.x; }
+  // its i-th group in the radix-16 passes: a warp's groups are consecutive, so
+  // that a block of 2^k consecutive words belongs to 2^k / E consecutive
+  // threads in every such pass
+  __device__ __forceinline__ static int group(int i) {
+    const int t = tid();
+    return (t >> 5) * (2 * E) + (t & 31) + 32 * i;
+  }
+  // Barrier of the threads that share this thread's block of 2^lb words.  A
+  // pass mixes words inside its blocks only, so a CTA-wide barrier is needed
+  // around the first pass alone; from the 2^8-word blocks of the pass before
+  // the last on it is one warp's, and for 2^13 and 2^14 words the pass between
+  // synchronizes 2 or 4 parts of the CTA on their own.  Besides the barriers
+  // saved, the warps of an SM drift apart, so that one's loads fall into
+  // another's arithmetic (256 products of 2^14 words 137.3 -> 132.3 us, 1000
+  // forward transforms 175.8 -> 165.9 us).
+  __device__ __forceinline__ static void sync_block(int lb) {
+    if ((1 << lb) <= 32 * E) {
+      __syncwarp(T < 32 ? (1u << (T & 31)) - 1u : 0xffffffffu);
+    } else if ((1 << lb) == N) {
+      __syncthreads();
+    } else {
+      static_assert(!DUAL || N <= 32 * E * 16, "a part of half a CTA");
+      const int threads = (1 << lb) / E;
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + tid() / threads), "r"(threads) : "memory");
+    }
+  }
 };
 
 // A radix-16 pass starting at stage s0 of an n = 2^logn transform: group g
@@ -584,7 +610,8 @@ constexpr int round_groups() {
 // in rounds of 16 (all of a round's loads in flight at once; 32 words at once
 // would spill), then FIRSTK stages per group, results to shared memory.
 // The first sub-stage uses the exact first-stage rule; after the global pass
-// of a large transform the inputs always take its fast path.
+// of a large transform the inputs always take its fast path.  The barrier that
+// frees the shared words comes after the first round's loads and butterflies.
 template <class S>
 __device__ __forceinline__ void fwd_first(u64* sm, const u64* __restrict__ in, const Tw& t, u32 tw_mult) {
   constexpr int KK = S::FIRSTK, G = S::E >> KK, TMIN = S::N >> KK;
@@ -604,10 +631,12 @@ __device__ __forceinline__ void fwd_first(u64* sm, const u64* __restrict__ in, c
       for (int jj = 0; jj < (1 << (KK - 1)); jj++)
         ct_first<typename S::M>(v[i * (1 << KK) + jj], v[i * (1 << KK) + jj + (1 << (KK - 1))], w0.x, w0.y, t);
       ct_group<typename S::M, KK, 1, i * (1 << KK)>(v, RowTw{t.fwd, tw_mult}, t);
-      const int g = S::tid() + (i0 + i) * S::T;
-#pragma unroll
-      for (int j = 0; j < (1 << KK); j++) sm[pad(g + j * TMIN)] = v[i * (1 << KK) + j];
     });
+    if (i0 == 0) __syncthreads();  // everyone is done with what the shared words held
+#pragma unroll
+    for (int i = 0; i < GR; i++)
+#pragma unroll
+      for (int j = 0; j < (1 << KK); j++) sm[pad(S::tid() + (i0 + i) * S::T + j * TMIN)] = v[i * (1 << KK) + j];
   }
   __syncthreads();
 }
@@ -637,7 +666,7 @@ __device__ __forceinline__ void fwd_first_smem(u64* sm, const Tw& t, u32 tw_mult
 
 // Radix-16 forward passes s0 = FIRSTK, FIRSTK + 4, ..., HEAD on shared
 // memory.  The last pass hands each group (words 16g .. 16g+15) to epi(g, v)
-// instead of storing it back.  Ends with a barrier.
+// instead of storing it back.  No barrier at the end.
 template <class S, class L, class Epi>
 __device__ __forceinline__ void fwd_passes(u64* sm, const Tw& t, u32 tw_mult, const L& last, Epi&& epi) {
 #pragma unroll 1
@@ -646,7 +675,7 @@ __device__ __forceinline__ void fwd_passes(u64* sm, const Tw& t, u32 tw_mult, co
     const int st = 1 << ps.lt;
 #pragma unroll(S::U)
     for (int i = 0; i < S::E / 16; i++) {
-      const int g = S::tid() + i * S::T;
+      const int g = S::group(i);
       const int a0 = ps.first(g);
       u64 v[16];
 #pragma unroll
@@ -655,31 +684,31 @@ __device__ __forceinline__ void fwd_passes(u64* sm, const Tw& t, u32 tw_mult, co
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(a0 + j * st)] = v[j];
     }
-    __syncthreads();
+    S::sync_block(ps.lb);
   }
 #pragma unroll(S::U)
   for (int i = 0; i < S::E / 16; i++) {
-    const int g = S::tid() + i * S::T;
+    const int g = S::group(i);
     u64 v[16];
 #pragma unroll
     for (int j = 0; j < 16; j++) v[j] = sm[17 * g + j];  // pad(16 g + j)
     ct_group<typename S::M, 4, 0, 0>(v, last.at(g), t);
     epi(g, v);
   }
-  __syncthreads();
 }
 
 // Radix-16 inverse passes s0 = s_top, s_top - 4, ..., FIRSTK on shared
-// memory, each followed by a barrier.
+// memory, each preceded by a barrier of its blocks; a CTA barrier at the end.
 template <class S>
 __device__ __forceinline__ void inv_passes(u64* sm, const Tw& t, u32 tw_mult, int s_top) {
 #pragma unroll 1
   for (int s0 = s_top; s0 >= S::FIRSTK; s0 -= 4) {
     const Pass16 ps(S::LOGN, s0, tw_mult);
     const int st = 1 << ps.lt;
+    S::sync_block(ps.lb);
 #pragma unroll(S::U)
     for (int i = 0; i < S::E / 16; i++) {
-      const int g = S::tid() + i * S::T;
+      const int g = S::group(i);
       const int a0 = ps.first(g);
       u64 v[16];
 #pragma unroll
@@ -688,8 +717,8 @@ __device__ __forceinline__ void inv_passes(u64* sm, const Tw& t, u32 tw_mult, in
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(a0 + j * st)] = v[j];
     }
-    __syncthreads();
   }
+  __syncthreads();
 }
 
 // Last inverse pass of a cluster sub-block: stages FIRSTK-1 .. 0 in place in
@@ -929,17 +958,16 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     // U groups in flight, as in the other passes
 #pragma unroll(S::U)
     for (int i = 0; i < S::E / 16; i++) {
-      const int g = (int)threadIdx.x + i * S::T;
+      const int g = S::group(i);
       u64 v[16];
       load16(v, in + 16 * g);
       gs_group<M, 4, 0, true, false>(v, last.at(g), t);
+      if (i == 0) __syncthreads();  // the last job's words are read
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
     }
-    __syncthreads();
     inv_passes<S>(sm, t, tw_mult, S::HEAD - 4);
     inv_last<S, LIFT>(sm, t, tw_mult, out, sub_log == 0, &lift);
-    __syncthreads();
   }
 }
 
@@ -998,7 +1026,6 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
     }
     inv_passes<S>(sm, t, 1u, S::HEAD - 4);
     inv_last<S, LIFT>(sm, t, 1u, reinterpret_cast<u64*>(job.c), true, &lift);
-    __syncthreads();
   }
 }
 
