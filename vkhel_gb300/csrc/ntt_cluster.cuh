@@ -40,14 +40,30 @@ namespace vk {
 template <class M>
 using SubShape = Shape<14, 32, 1, M>;  // the large-n sub-block
 
+// The column pass: the first LOGC stages, which mix the sub-blocks, and with
+// them the sub-block's own first pass (FIRSTK stages) where both fit one
+// radix-16 group -- 2^15 and 2^16 on 2^14-word sub-blocks, 2^12 and 2^16 on 8
+// CTAs -- which saves that pass over shared memory and its barrier (64 products of
+// 2^16 words 161.9 -> 153.7 us, 150 inverse transforms of 2^15 with a lift
+// 75.9 -> 71.8 us, the ragged batch of 512 instances 3.22 -> 3.06 ms).
+// A group is W = 2^KK words TM apart; word j belongs to CTA j >> LJ.
 template <int LOGC, class S>
 struct Cols {
   static constexpr int C = 1 << LOGC, SUB = S::N;
-  static constexpr int COLS = SUB >> LOGC;  // columns per CTA
-  static constexpr int PER = COLS / S::T;   // columns per thread
+  static constexpr bool MERGED = LOGC + S::FIRSTK <= 4;
+  static constexpr int LJ = MERGED ? S::FIRSTK : 0;
+  static constexpr int KK = LOGC + LJ, W = 1 << KK;
+  static constexpr int TM = SUB >> LJ;
+  static constexpr int COLS = TM >> LOGC;   // groups per CTA
+  static constexpr int PER = COLS / S::T;   // groups per thread
+  static constexpr int H = PER >= 2 ? PER / 2 : 1;  // of them in flight at once
   static constexpr int N16 = C * SUB / 16;  // groups of the last four stages
-  static_assert(PER * C == S::E, "a column pass moves E words per thread");
+  static_assert(PER * W == S::E, "a column pass moves E words per thread");
+  static_assert(W <= S::T, "a thread per slice prefetches");
   __device__ __forceinline__ static int col(int rank, int k) { return rank * COLS + (int)threadIdx.x + k * S::T; }
+  // word j of column c: its CTA (static) and its place there
+  static constexpr int cta(int j) { return j >> LJ; }
+  __device__ __forceinline__ static int local(int c, int j) { return pad(c + (j & ((1 << LJ) - 1)) * TM); }
 };
 
 // The cluster barrier split in two: arrive (release: this thread's accesses
@@ -57,7 +73,7 @@ struct Cols {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// Forward column pass: global stages 0 .. LOGC-1 (exact first-stage rule),
+// Forward column pass: global stages 0 .. KK-1 (exact first-stage rule),
 // outputs scattered to the owning CTAs' shared memory, forward-lazy.  A
 // thread's PER columns go in two rounds of H = PER / 2 (16 words in flight:
 // all 32 at once would spill).  SPLIT: the caller has arrived on the cluster
@@ -71,64 +87,82 @@ template <int LOGC, class S, bool SPLIT>
 __device__ __forceinline__ void col_fwd(const u64* __restrict__ in, u64* sm, const cg::cluster_group& cl, int rank,
                                         const Tw& t, int rbase = 0) {
   using K = Cols<LOGC, S>;
-  constexpr int H = K::PER >= 2 ? K::PER / 2 : 1;
   const ulonglong2 w0 = ld_tw(t.fwd + 1);
 #pragma unroll 1
-  for (int k0 = 0; k0 < K::PER; k0 += H) {
-    u64 v[H * K::C];
+  for (int k0 = 0; k0 < K::PER; k0 += K::H) {
+    u64 v[K::H * K::W];
 #pragma unroll
-    for (int k = 0; k < H; k++)
+    for (int k = 0; k < K::H; k++)
 #pragma unroll
-      for (int j = 0; j < K::C; j++) v[k * K::C + j] = ld_stream(in + K::col(rank, k0 + k) + (size_t)j * K::SUB);
-    static_for<0, H>([&](auto kc) {
+      for (int j = 0; j < K::W; j++) v[k * K::W + j] = ld_stream(in + K::col(rank, k0 + k) + (size_t)j * K::TM);
+    static_for<0, K::H>([&](auto kc) {
       constexpr int k = decltype(kc)::value;
 #pragma unroll
-      for (int jj = 0; jj < K::C / 2; jj++)
-        ct_first<typename S::M>(v[k * K::C + jj], v[k * K::C + jj + K::C / 2], w0.x, w0.y, t);
-      ct_group<typename S::M, LOGC, 1, k * K::C>(v, RowTw{t.fwd, 1u}, t);
+      for (int jj = 0; jj < K::W / 2; jj++)
+        ct_first<typename S::M>(v[k * K::W + jj], v[k * K::W + jj + K::W / 2], w0.x, w0.y, t);
+      ct_group<typename S::M, K::KK, 1, k * K::W>(v, RowTw{t.fwd, 1u}, t);
     });
     if (SPLIT && k0 == 0) cluster_wait();
 #pragma unroll
-    for (int j = 0; j < K::C; j++) {
-      u64* rem = cl.map_shared_rank(sm, rbase + j);
+    for (int j = 0; j < K::W; j++) {
+      u64* rem = cl.map_shared_rank(sm, rbase + K::cta(j));
 #pragma unroll
-      for (int k = 0; k < H; k++) rem[pad(K::col(rank, k0 + k))] = v[k * K::C + j];
+      for (int k = 0; k < K::H; k++) rem[K::local(K::col(rank, k0 + k), j)] = v[k * K::W + j];
     }
   }
 }
 
-// Inverse column pass: gather, global stages LOGC-1 .. 0 with n^-1 folded in,
+// Inverse column pass: gather, global stages KK-1 .. 0 with n^-1 folded in,
 // canonical words to global memory; two rounds of H columns as above.
 template <int LOGC, class S, class Epi>
 __device__ __forceinline__ void col_inv(u64* __restrict__ out, u64* sm, const cg::cluster_group& cl, int rank,
                                         const Tw& t, const Epi& epi, int rbase = 0) {
   using K = Cols<LOGC, S>;
-  constexpr int H = K::PER >= 2 ? K::PER / 2 : 1;
 #pragma unroll 1
-  for (int k0 = 0; k0 < K::PER; k0 += H) {
-    u64 v[H * K::C];
+  for (int k0 = 0; k0 < K::PER; k0 += K::H) {
+    u64 v[K::H * K::W];
 #pragma unroll
-    for (int j = 0; j < K::C; j++) {
-      const u64* rem = cl.map_shared_rank(sm, rbase + j);
+    for (int j = 0; j < K::W; j++) {
+      const u64* rem = cl.map_shared_rank(sm, rbase + K::cta(j));
 #pragma unroll
-      for (int k = 0; k < H; k++) v[k * K::C + j] = rem[pad(K::col(rank, k0 + k))];
+      for (int k = 0; k < K::H; k++) v[k * K::W + j] = rem[K::local(K::col(rank, k0 + k), j)];
     }
-    static_for<0, H>([&](auto kc) {
+    static_for<0, K::H>([&](auto kc) {
       constexpr int k = decltype(kc)::value;
-      gs_group<typename S::M, LOGC, k * K::C, false, true>(v, RowTw{t.inv, 1u}, t);
+      gs_group<typename S::M, K::KK, k * K::W, false, true>(v, RowTw{t.inv, 1u}, t);
     });
+    epi.apply(v);
 #pragma unroll
-    for (int k = 0; k < H; k++)
+    for (int k = 0; k < K::H; k++)
 #pragma unroll
-      for (int j = 0; j < K::C; j++) out[K::col(rank, k0 + k) + (size_t)j * K::SUB] = epi(v[k * K::C + j]);
+      for (int j = 0; j < K::W; j++) out[K::col(rank, k0 + k) + (size_t)j * K::TM] = v[k * K::W + j];
   }
+}
+
+// The passes of a sub-block between the column pass and the last radix-16
+// pass, with the cluster barriers: forward after col_fwd, inverse before
+// col_inv.
+template <int LOGC, class S>
+__device__ __forceinline__ void sub_fwd(u64* sm, const cg::cluster_group& cl, const Tw& t, u32 tw_mult) {
+  cl.sync();
+  if constexpr (!Cols<LOGC, S>::MERGED) fwd_first_smem<S>(sm, t, tw_mult);
+}
+
+template <int LOGC, class S>
+__device__ __forceinline__ void sub_inv(u64* sm, const cg::cluster_group& cl, const Tw& t, u32 tw_mult) {
+  inv_passes<S>(sm, t, tw_mult, S::HEAD - 4);
+  if constexpr (!Cols<LOGC, S>::MERGED) {
+    __syncthreads();
+    inv_last_smem<S>(sm, t, tw_mult);
+  }
+  cl.sync();
 }
 
 template <int LOGC, class S, bool LIFT>
 __device__ __forceinline__ void col_inv_out(u64* __restrict__ out, u64* sm, const cg::cluster_group& cl, int rank,
                                             const Tw& t, const vkcu_lift* lift, int rbase = 0) {
   if constexpr (LIFT)
-    col_inv<LOGC, S>(out, sm, cl, rank, t, LiftRun(lift, t.q), rbase);
+    col_inv<LOGC, S>(out, sm, cl, rank, t, LiftFold(lift, t.q), rbase);
   else
     col_inv<LOGC, S>(out, sm, cl, rank, t, NoLift{}, rbase);
 }
@@ -150,8 +184,7 @@ __global__ void __launch_bounds__(S::T, 1)
     u64* out = reinterpret_cast<u64*>(job.out) + (size_t)rank * K::SUB;
     cl.sync();
     col_fwd<LOGC, S, false>(reinterpret_cast<const u64*>(job.in), sm, cl, rank, t);
-    cl.sync();
-    fwd_first_smem<S>(sm, t, tw_mult);
+    sub_fwd<LOGC, S>(sm, cl, t, tw_mult);
     fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
       const typename S::M::Out to(t);
 #pragma unroll
@@ -188,9 +221,7 @@ __global__ void __launch_bounds__(S::T, 1)
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
     }
-    inv_passes<S>(sm, t, tw_mult, S::HEAD - 4);
-    inv_last_smem<S>(sm, t, tw_mult);
-    cl.sync();
+    sub_inv<LOGC, S>(sm, cl, t, tw_mult);
     col_inv_out<LOGC, S, LIFT>(reinterpret_cast<u64*>(job.out), sm, cl, rank, t, &lift);
   }
   cl.sync();
@@ -215,14 +246,13 @@ __global__ void __launch_bounds__(S::T, 1)
     const bool b_ntt = LIFT && (job.flags & VKCU_JOB_B_NTT);
     u64* scratch = reinterpret_cast<u64*>(job.scratch) + (size_t)rank * K::SUB;
     const LastTable<K::N16> last(t.fwd, rank * (S::N / 16), 0), last_inv(t.inv, rank * (S::N / 16), 0);
-    if ((int)threadIdx.x < K::C)  // this CTA's column slices of a, for phase 1
-      prefetch_l2(reinterpret_cast<const u64*>(job.a) + (size_t)threadIdx.x * K::SUB + rank * K::COLS, kSlice);
+    if ((int)threadIdx.x < K::W)  // this CTA's column slices of a, for phase 1
+      prefetch_l2(reinterpret_cast<const u64*>(job.a) + (size_t)threadIdx.x * K::TM + rank * K::COLS, kSlice);
 #pragma unroll 1
     for (int ph = b_ntt ? 1 : 0; ph < 2; ph++) {
       cluster_arrive();  // done with every shared memory the column pass writes (col_fwd waits)
       col_fwd<LOGC, S, true>(reinterpret_cast<const u64*>(ph ? job.a : job.b), sm, cl, rank, t);
-      cl.sync();
-      fwd_first_smem<S>(sm, t, tw_mult);
+      sub_fwd<LOGC, S>(sm, cl, t, tw_mult);
       fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
         using M = typename S::M;
         if (ph == 0) {
@@ -248,16 +278,14 @@ __global__ void __launch_bounds__(S::T, 1)
         }
       });
     }
-    if (w + ncl < njobs && (int)threadIdx.x < K::C) {
+    if (w + ncl < njobs && (int)threadIdx.x < K::W) {
       // the next job's b: its column slices, or (NTT(b) given) this CTA's sub-block
       const vkcu_poly_job nx = fetch_job(jobs, one, w + ncl);
       const size_t off = (LIFT && (nx.flags & VKCU_JOB_B_NTT)) ? (size_t)rank * K::SUB + (size_t)threadIdx.x * K::COLS
-                                                     : (size_t)threadIdx.x * K::SUB + rank * K::COLS;
+                                                     : (size_t)threadIdx.x * K::TM + rank * K::COLS;
       prefetch_l2(reinterpret_cast<const u64*>(nx.b) + off, kSlice);
     }
-    inv_passes<S>(sm, t, tw_mult, S::HEAD - 4);
-    inv_last_smem<S>(sm, t, tw_mult);
-    cl.sync();
+    sub_inv<LOGC, S>(sm, cl, t, tw_mult);
     col_inv_out<LOGC, S, LIFT>(reinterpret_cast<u64*>(job.c), sm, cl, rank, t, &lift);
   }
   cl.sync();

@@ -59,6 +59,7 @@ __device__ __noinline__ void ragged_cta_product(u64* sm, const vkcu_poly_job& jo
     });
   }
   inv_passes<S>(sm, t, 1u, S::HEAD - 4);
+  __syncthreads();
   inv_last<S>(sm, t, 1u, reinterpret_cast<u64*>(job.c), true);
   __syncthreads();
 }
@@ -79,8 +80,7 @@ __device__ __noinline__ void ragged_cluster_product(u64* sm, const cg::cluster_g
   for (int ph = 0; ph < 2; ph++) {
     cluster_arrive();  // done with every shared memory the column pass writes (col_fwd waits)
     col_fwd<LOGC, S, true>(reinterpret_cast<const u64*>(ph ? job.a : job.b), sm, cl, rank, t, rbase);
-    cl.sync();
-    fwd_first_smem<S>(sm, t, tw_mult);
+    sub_fwd<LOGC, S>(sm, cl, t, tw_mult);
     fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
       if (ph == 0) {
         const typename M::Out to(t);
@@ -99,9 +99,7 @@ __device__ __noinline__ void ragged_cluster_product(u64* sm, const cg::cluster_g
       }
     });
   }
-  inv_passes<S>(sm, t, tw_mult, S::HEAD - 4);
-  inv_last_smem<S>(sm, t, tw_mult);
-  cl.sync();
+  sub_inv<LOGC, S>(sm, cl, t, tw_mult);
   col_inv_out<LOGC, S, false>(reinterpret_cast<u64*>(job.c), sm, cl, rank, t, nullptr, rbase);
 }
 
