@@ -690,16 +690,9 @@ static int polymul_impl(const struct vkhel_vector *a, const struct vkhel_vector 
 		const vkcu_poly_job job = {a->dev, b->dev, res->dev, scratch, d->dev_set, b_ntt ? VKCU_JOB_B_NTT : 0};
 		e = vkcu_polymul_lift(ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms, lp, b_ntt);
 	} else {
-		const vkcu_ntt_job jb = {b->dev, scratch, d->dev_set};
-		const vkcu_ntt_job ja = {a->dev, res->dev, d->dev_set};
-		const vkcu_ntt_job jc = {res->dev, res->dev, d->dev_set};
-		e = b_ntt ? 0 : vkcu_ntt_forward(ctx->stream, NULL, 1, &jb, t->log_n, vkcu_qclass(t->q), ctx->sms);
-		if (!e)
-			e = vkcu_ntt_forward(ctx->stream, NULL, 1, &ja, t->log_n, vkcu_qclass(t->q), ctx->sms);
-		if (!e)
-			e = vkcu_elemmul(ctx->stream, res->dev, res->dev, scratch, t->n, t->q, t->mu, t->qbits);
-		if (!e)
-			e = vkcu_ntt_inverse_lift(ctx->stream, NULL, 1, &jc, t->log_n, vkcu_qclass(t->q), ctx->sms, lp);
+		const vkcu_poly_job job = {a->dev, b->dev, res->dev, scratch, d->dev_set, b_ntt ? VKCU_JOB_B_NTT : 0};
+		e = vkcu_polymul_composed(ctx->stream, NULL, NULL, NULL, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms,
+				lp, b_ntt);
 	}
 	st = finish(ctx, e, "polymul");
 	if (tmp)

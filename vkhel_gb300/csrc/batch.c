@@ -283,9 +283,9 @@ static int cmp_rec(const void *x, const void *y) {
 }
 
 /* Launch the kernels of `nclasses` degree classes on `stream`: one fused
- * polymul launch per class with 2^8 <= n <= 2^17, otherwise forward(b ->
- * scratch), forward(a -> c), pointwise, inverse(c) over the class's slice of
- * the ntt-job array (laid out at 3 * first: b jobs, a jobs, c jobs).  A
+ * polymul launch per class with 2^8 <= n <= 2^17, otherwise the composed
+ * product (b -> scratch, a -> c, product, inverse of c) over the class's slice
+ * of the ntt-job array (laid out at 3 * first: b jobs, a jobs, c jobs).  A
  * class's epilogue rides on its last launch. */
 int vkh_issue_classes(void *stream, int sms, const vkcu_poly_job *dev_poly, const vkcu_ntt_job *dev_ntt,
 		const struct vkh_job_class *classes, uint32_t nclasses, const vkcu_lift *lifts) {
@@ -302,15 +302,8 @@ int vkh_issue_classes(void *stream, int sms, const vkcu_poly_job *dev_poly, cons
 			e = vkcu_polymul_lift(stream, dev_poly + cl->first, (int) cl->count, NULL, cl->log_n, cl->qclass, sms,
 					lift, (int) cl->b_ntt);
 		} else {
-			const vkcu_ntt_job *nj = dev_ntt + 3 * (size_t) cl->first;
-			e = cl->b_ntt ? 0 : vkcu_ntt_forward(stream, nj, (int) cl->count, NULL, cl->log_n, cl->qclass, sms);
-			if (!e)
-				e = vkcu_ntt_forward(stream, nj + cl->count, (int) cl->count, NULL, cl->log_n, cl->qclass, sms);
-			if (!e)
-				e = vkcu_pointwise(stream, dev_poly + cl->first, (int) cl->count, cl->log_n, cl->qclass, sms);
-			if (!e)
-				e = vkcu_ntt_inverse_lift(stream, nj + 2 * (size_t) cl->count, (int) cl->count, NULL, cl->log_n,
-						cl->qclass, sms, lift);
+			e = vkcu_polymul_composed(stream, dev_poly + cl->first, tj, tj + cl->count, tj + 2 * (size_t) cl->count,
+					(int) cl->count, NULL, cl->log_n, cl->qclass, sms, lift, (int) cl->b_ntt);
 		}
 		if (e)
 			return e;

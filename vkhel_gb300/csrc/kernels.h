@@ -212,7 +212,7 @@ int vkcu_ntt_inverse(void *stream, const vkcu_ntt_job *jobs, int njobs,
 int vkcu_polymul(void *stream, const vkcu_poly_job *jobs, int njobs,
 		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms);
 /* The same with an epilogue (`lift` NULL or count 0: none); fused into the
- * last pass for 2^8 <= n <= 2^17, a separate element-wise launch otherwise.
+ * last pass for n >= 2^8, a separate element-wise launch otherwise.
  * b_ntt: the jobs carry VKCU_JOB_B_NTT; only the epilogue instantiations of
  * the fused kernels read that flag, so such jobs run those (with no steps
  * when `lift` has none) and the plain kernels stay as lean as before. */
@@ -229,7 +229,13 @@ int vkcu_lift_jobs(void *stream, const vkcu_ntt_job *jobs, int njobs, const vkcu
  * outputs; the word the reference's elemmul stores): the pointwise step of a
  * polymul that is not fused. */
 int vkcu_pointwise(void *stream, const vkcu_poly_job *jobs, int njobs,
-		uint32_t log_n, int qclass, int sms);
+		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms);
+/* Products outside the single-launch degrees.  b, a and c are the jobs'
+ * transforms b -> scratch, a -> c and c -> c (device arrays, or NULL with a
+ * single job `one`). */
+int vkcu_polymul_composed(void *stream, const vkcu_poly_job *jobs, const vkcu_ntt_job *b,
+		const vkcu_ntt_job *a, const vkcu_ntt_job *c, int njobs, const vkcu_poly_job *one,
+		uint32_t log_n, int qclass, int sms, const vkcu_lift *lift, int b_ntt);
 /* A ragged batch of fused limb products of degrees 2^12 .. 2^16 as one
  * persistent launch (ntt_ragged.cu): items in decreasing size, the first
  * n_cluster_items of kind 16 (one product of 2^16 on a cluster of four CTAs)

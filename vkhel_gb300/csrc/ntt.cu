@@ -87,21 +87,20 @@ __global__ void k_ntt_inv_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
 
 // ---------------------------------------------------------------------------
 // Global-memory passes for n >= 2^18: the first (forward) or last (inverse)
-// log2(n) - 14 stages run over HBM in passes of KK <= 4 stages each, and
-// one CTA-resident kernel runs the other 14 stages on every 2^14-word
-// sub-block (sub-block r uses twiddle multiplier 2^(log2 n - 14) + r).  A
-// pass starting at stage s0 gives each thread one radix-2^KK group: the
-// 2^KK words at stride t = n >> (s0 + KK) inside one block of stage s0
-// (blocks of n >> s0 words), twiddle base 2^s0 + block (root index m + block
-// of the reference's stage loop, src/vector.c:536-566).  Consecutive threads
-// take consecutive offsets, so every load and store is coalesced.
+// stages run over HBM in passes of KK <= 4 stages each, and the CTA or cluster
+// kernels run the others on every sub-block (sub-block r uses twiddle
+// multiplier n / its size + r).  A pass starting at stage s0 gives each thread
+// one radix-2^KK group: the 2^KK words at stride t = n >> (s0 + KK) inside one
+// block of stage s0 (blocks of n >> s0 words), twiddle base 2^s0 + block (root
+// index m + block of the reference's stage loop, src/vector.c:536-566).
+// Consecutive threads take consecutive offsets, so every load and store is
+// coalesced.
 
 // Forward: stages s0 .. s0 + KK - 1, in -> out, forward-lazy; stage 0 takes
-// the reference's exact first-stage rule; the last pass (handoff) leaves
-// words below the sub-block kernels' first-stage fast-path bound.
+// the reference's exact first-stage rule.
 template <int KK, class M>
-__global__ void k_fwd_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int log_n, int s0,
-                             int handoff) {
+__global__ void __launch_bounds__(256)
+    k_fwd_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int log_n, int s0) {
   const int lt = log_n - s0 - KK;  // log2 of the stride
   const long groups = 1L << (log_n - KK);
   const long total = (long)njobs * groups;
@@ -116,31 +115,25 @@ __global__ void k_fwd_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, v
     u64 v[1 << KK];
 #pragma unroll
     for (int j = 0; j < (1 << KK); j++) v[j] = ld_stream(in + first + j * st);
-    const u32 base = (1u << s0) + (u32)blk;
-    if (s0 == 0) {
-      const ulonglong2 w0 = ld_tw(t.fwd + 1);
-#pragma unroll
-      for (int jj = 0; jj < (1 << (KK - 1)); jj++) ct_first<M>(v[jj], v[jj + (1 << (KK - 1))], w0.x, w0.y, t);
-      ct_group<M, KK, 1, 0>(v, RowTw{t.fwd, base}, t);
-    } else {
-      ct_group<M, KK, 0, 0>(v, RowTw{t.fwd, base}, t);
-    }
+    const RowTw tw{t.fwd, (1u << s0) + (u32)blk};
+    if (s0 == 0)
+      ct_first_group<M, KK, 0, true>(v, tw, t);
+    else
+      ct_first_group<M, KK, 0, false>(v, tw, t);
     u64* out = reinterpret_cast<u64*>(job.out);
-    if (handoff) {
-      const typename M::Out to(t);
-#pragma unroll
-      for (int j = 0; j < (1 << KK); j++) v[j] = to.handoff(v[j]);
-    }
 #pragma unroll
     for (int j = 0; j < (1 << KK); j++) out[first + j * st] = v[j];
   }
 }
 
 // Inverse: stages s0 + KK - 1 .. s0 on `out` in place (after the sub-block
-// kernels, which leave inverse-lazy words); the pass with s0 = 0 folds n^-1
-// into stage 0 and writes canonical words.
-template <int KK, class M>
-__global__ void k_inv_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int log_n, int s0) {
+// kernels, which leave words below one unit); the pass with s0 = 0 folds n^-1
+// into stage 0, writes canonical words and applies the epilogue (LIFT).
+// product: the sub-blocks' products were Product's (fold constants to match).
+template <int KK, class M, bool LIFT>
+__global__ void __launch_bounds__(256)
+    k_inv_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int log_n, int s0, int product,
+                 const __grid_constant__ vkcu_lift lift) {
   const int lt = log_n - s0 - KK;
   const long groups = 1L << (log_n - KK);
   const long total = (long)njobs * groups;
@@ -150,16 +143,18 @@ __global__ void k_inv_global(const vkcu_ntt_job* __restrict__ jobs, int njobs, v
     const long blk = g >> lt;
     const size_t first = ((size_t)blk << (log_n - s0)) | (size_t)(g & ((1L << lt) - 1));
     const size_t st = (size_t)1 << lt;
-    const Tw t = load_tw(job.tw);
+    const Tw t = product ? load_tw_product<M>(job.tw) : load_tw(job.tw);
     u64* out = reinterpret_cast<u64*>(job.out);
     u64 v[1 << KK];
 #pragma unroll
     for (int j = 0; j < (1 << KK); j++) v[j] = out[first + j * st];
-    const u32 base = (1u << s0) + (u32)blk;
-    if (s0 == 0)
-      gs_group<M, KK, 0, false, true>(v, RowTw{t.inv, base}, t);
-    else
-      gs_group<M, KK, 0, false, false>(v, RowTw{t.inv, base}, t);
+    const RowTw tw{t.inv, (1u << s0) + (u32)blk};
+    if (s0 == 0) {
+      gs_group<M, KK, 0, false, true>(v, tw, t);
+      if constexpr (LIFT) LiftFold(&lift, t.q).apply(v);
+    } else {
+      gs_group<M, KK, 0, false, false>(v, tw, t);
+    }
 #pragma unroll
     for (int j = 0; j < (1 << KK); j++) out[first + j * st] = v[j];
   }
@@ -189,42 +184,93 @@ static int simple(cudaStream_t st, bool inverse, const vkcu_ntt_job* jobs, int n
   return (int)cudaGetLastError();
 }
 
-// Stages of the global pass p (0-based, in forward order) for log_n: the
-// log_n - 14 global stages split into as few passes of <= 4 stages as
-// possible, sizes as equal as possible (2^21: 4 + 3).
-static int global_passes(int log_n) { return (log_n - kMaxCta + 3) / 4; }
-static void global_split(int log_n, int p, int* s0, int* kk) {
-  const int g = log_n - kMaxCta, np = global_passes(log_n), small = g / np, big = g % np;
-  *s0 = p * small + (p < big ? p : big);
-  *kk = small + (p < big ? 1 : 0);
+// The stages above the sub-blocks: `g` of them in as few passes of <= 4 as
+// possible, sizes as equal as possible (5: 3 + 2).
+struct GlobalPlan {
+  int g;
+  int passes() const { return (g + 3) / 4; }
+  void pass(int p, int* s0, int* kk) const {  // 0-based, in forward order
+    const int np = passes(), small = g / np, big = g % np;
+    *s0 = p * small + (p < big ? p : big);
+    *kk = small + (p < big ? 1 : 0);
+  }
+};
+
+// Blocks of 256 threads, of 64 where those would leave SMs without one.
+static int pass_threads(long work, int sms) { return work < (long)sms * 512 ? 64 : 256; }
+
+template <class M>
+static int forward_passes(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n,
+                          GlobalPlan plan, int sms) {
+  for (int p = 0; p < plan.passes(); p++) {
+    int s0, kk;
+    plan.pass(p, &s0, &kk);
+    const long work = (long)njobs << (log_n - kk);
+    const int threads = pass_threads(work, sms);
+    const long blocks = (work + threads - 1) / threads, cap = (long)sms * 8;
+    const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
+    switch (kk) {
+#define G(K)                                                                       \
+  case K:                                                                          \
+    k_fwd_global<K, M><<<grid, threads, 0, st>>>(jobs, njobs, one, log_n, s0);      \
+    break;
+      G(1)
+      G(2)
+      G(3)
+      G(4)
+#undef G
+      default:
+        return (int)cudaErrorInvalidValue;
+    }
+    vkcu_count_launches(1);
+    if (const int e = (int)cudaGetLastError()) return e;
+  }
+  return 0;
 }
 
 template <class M>
-static int global_pass(cudaStream_t st, bool inverse, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one,
-                       int log_n, int s0, int kk, int handoff, int sms) {
-  const long work = (long)njobs << (log_n - kk);
-  const int threads = 256;
-  long blocks = (work + threads - 1) / threads;
-  const long cap = (long)sms * 8;
-  if (blocks > cap) blocks = cap;
-  switch (kk) {
-#define G(K)                                                                                          \
-  case K:                                                                                             \
-    if (inverse)                                                                                      \
-      k_inv_global<K, M><<<(int)blocks, threads, 0, st>>>(jobs, njobs, one, log_n, s0);               \
-    else                                                                                              \
-      k_fwd_global<K, M><<<(int)blocks, threads, 0, st>>>(jobs, njobs, one, log_n, s0, handoff);      \
+static int inverse_passes(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n,
+                          GlobalPlan plan, int sms, int product, const vkcu_lift* lift) {
+  const vkcu_lift none{};
+  for (int p = plan.passes() - 1; p >= 0; p--) {
+    int s0, kk;
+    plan.pass(p, &s0, &kk);
+    const long work = (long)njobs << (log_n - kk);
+    const int threads = pass_threads(work, sms);
+    const long blocks = (work + threads - 1) / threads, cap = (long)sms * 8;
+    const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
+    switch (kk * 2 + (lift && s0 == 0 ? 1 : 0)) {
+#define G(K)                                                                                                     \
+  case 2 * K:                                                                                                    \
+    k_inv_global<K, M, false><<<grid, threads, 0, st>>>(jobs, njobs, one, log_n, s0, product, none);             \
+    break;                                                                                                       \
+  case 2 * K + 1:                                                                                                \
+    k_inv_global<K, M, true><<<grid, threads, 0, st>>>(jobs, njobs, one, log_n, s0, product, *lift);             \
     break;
-    G(1)
-    G(2)
-    G(3)
-    G(4)
+      G(1)
+      G(2)
+      G(3)
+      G(4)
 #undef G
-    default:
-      return (int)cudaErrorInvalidValue;
+      default:
+        return (int)cudaErrorInvalidValue;
+    }
+    vkcu_count_launches(1);
+    if (const int e = (int)cudaGetLastError()) return e;
   }
-  vkcu_count_launches(1);
-  return (int)cudaGetLastError();
+  return 0;
+}
+
+// log2 of the sub-blocks per transform of 2^log_n > 2^17 words: 2^16-word
+// sub-blocks on clusters of 4 CTAs (one radix-16 global pass at 2^20, and four
+// radix-16 passes inside), or 2^14-word ones on clusters of 8 small CTAs where
+// the former would leave half of the SMs idle.  Products, 4-CTA / 8-CTA: 1 of
+// 2^18 (4 sub-blocks of 2^16) 86 / 37 us, 4 of 2^18 (16) 94 / 66 us, 9 of 2^18
+// (36) 108 / 128 us, 15 of 2^20 (240) 722 / 907 us; forward transforms and
+// products on CTA-resident 2^14-word sub-blocks and more global passes before:
+// 90, 99, 121 and 885 us.
+static int sub_log_of(int njobs, int log_n, int sms) {
+  return ((long)njobs << (log_n - 16)) * 8 > (long)sms ? log_n - 16 : log_n - 14;
 }
 
 }  // namespace vk
@@ -287,22 +333,18 @@ static int forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
                  : e;
     }
     if (log_n <= (uint32_t)kMaxCta)
-      return fwd_cta<M>(st, jobs, njobs, o, (int)log_n, 0, sms, vkh_variant_jobs(1, (int)log_n, njobs, sms));
+      return fwd_cta<M>(st, jobs, njobs, o, (int)log_n, sms, vkh_variant_jobs(1, (int)log_n, njobs, sms));
     if (log_n <= (uint32_t)kMaxCluster) return fwd_cluster<M>(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta);
   }
-  const int np = global_passes((int)log_n);
-  for (int p = 0; p < np; p++) {
-    int s0, kk;
-    global_split((int)log_n, p, &s0, &kk);
-    const int e = global_pass<M>(st, false, jobs, njobs, o, (int)log_n, s0, kk, p == np - 1, sms);
-    if (e) return e;
+  if constexpr (kWide<M>) {
+    const int sub_log = (int)log_n - kMaxCta;
+    const int e = forward_passes<M>(st, jobs, njobs, o, (int)log_n, GlobalPlan{sub_log}, sms);
+    return e ? e : fwd_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms);
+  } else {
+    const int sub_log = sub_log_of(njobs, (int)log_n, sms);
+    const int e = forward_passes<M>(st, jobs, njobs, o, (int)log_n, GlobalPlan{sub_log}, sms);
+    return e ? e : fwd_cluster_sub<M>(st, jobs, njobs, o, (int)log_n, sub_log);
   }
-  const int sub_log = (int)log_n - kMaxCta;
-  if constexpr (kWide<M>)
-    return fwd_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms);
-  else
-    return fwd_cta<M>(st, jobs, njobs, o, kMaxCta, sub_log, sms,
-                      vkh_variant_jobs(1, kMaxCta, (long)njobs << sub_log, sms));
 }
 
 extern "C" int vkcu_ntt_forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
@@ -340,23 +382,21 @@ static int inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
       }
       if (log_n <= (uint32_t)kMaxCta) {
         if (lifted) return inv_cta_lift<M>(st, jobs, njobs, o, (int)log_n, sms, *lift);
-        return inv_cta<M>(st, jobs, njobs, o, (int)log_n, 0, sms, vkh_variant_jobs(2, (int)log_n, njobs, sms));
+        return inv_cta<M>(st, jobs, njobs, o, (int)log_n, sms, vkh_variant_jobs(2, (int)log_n, njobs, sms));
       }
       if (log_n <= (uint32_t)kMaxCluster) return inv_cluster<M>(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta, lp);
     }
-    const int sub_log = (int)log_n - kMaxCta;
-    if constexpr (kWide<M>)
+    int sub_log;
+    if constexpr (kWide<M>) {
+      sub_log = (int)log_n - kMaxCta;
       e = inv_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms, nullptr);
-    else
-      e = inv_cta<M>(st, jobs, njobs, o, kMaxCta, sub_log, sms,
-                     vkh_variant_jobs(2, kMaxCta, (long)njobs << sub_log, sms));
-    for (int p = global_passes((int)log_n) - 1; !e && p >= 0; p--) {
-      int s0, kk;
-      global_split((int)log_n, p, &s0, &kk);
-      e = global_pass<M>(st, true, jobs, njobs, o, (int)log_n, s0, kk, 0, sms);
+    } else {
+      sub_log = sub_log_of(njobs, (int)log_n, sms);
+      e = inv_cluster_sub<M>(st, jobs, njobs, o, (int)log_n, sub_log);
     }
+    return e ? e : inverse_passes<M>(st, jobs, njobs, o, (int)log_n, GlobalPlan{sub_log}, sms, 0, lp);
   }
-  // the multi-launch paths take the epilogue as one more element-wise launch
+  // the simple kernels take the epilogue as one more element-wise launch
   if (!e && lifted) e = vkcu_lift_jobs(stream, jobs, njobs, one, log_n, sms, lift);
   return e;
 }
@@ -408,6 +448,51 @@ extern "C" int vkcu_polymul_lift(void* stream, const vkcu_poly_job* jobs, int nj
 extern "C" int vkcu_polymul(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one,
                             uint32_t log_n, int qclass, int sms) {
   return vkcu_polymul_lift(stream, jobs, njobs, one, log_n, qclass, sms, nullptr, 0);
+}
+
+// A product past one cluster (2^18 .. 2^26, q < 2^62): the global passes of b
+// (into scratch) and of a (into c), one launch for every sub-block's forward,
+// product and inverse, the inverse global passes of c.  b, a and c give these
+// the jobs of the passes.
+template <class M>
+static int polymul_large(cudaStream_t st, const vkcu_poly_job* jobs, const vkcu_ntt_job* b, const vkcu_ntt_job* a,
+                         const vkcu_ntt_job* c, int njobs, const vkcu_poly_job& one, int log_n, int sms,
+                         const vkcu_lift* lift, int b_ntt) {
+  const vkcu_ntt_job ob{one.b, one.scratch, one.tw}, oa{one.a, one.c, one.tw}, oc{one.c, one.c, one.tw};
+  const int sub_log = sub_log_of(njobs, log_n, sms);
+  const GlobalPlan plan{sub_log};
+  int e = b_ntt ? 0 : forward_passes<M>(st, b, njobs, ob, log_n, plan, sms);
+  if (!e) e = forward_passes<M>(st, a, njobs, oa, log_n, plan, sms);
+  if (!e) e = poly_cluster_sub<M>(st, jobs, njobs, one, log_n, sub_log);
+  if (!e) e = inverse_passes<M>(st, c, njobs, oc, log_n, plan, sms, 1, lift);
+  return e;
+}
+
+// A product outside the single-launch degrees: past one cluster as above; for
+// n < 2^8, and q >= 2^62 past one cluster, forward(b), forward(a), pointwise,
+// inverse.
+extern "C" int vkcu_polymul_composed(void* stream, const vkcu_poly_job* jobs, const vkcu_ntt_job* b,
+                                     const vkcu_ntt_job* a, const vkcu_ntt_job* c, int njobs,
+                                     const vkcu_poly_job* one, uint32_t log_n, int qclass, int sms,
+                                     const vkcu_lift* lift, int b_ntt) {
+  cudaStream_t st = (cudaStream_t)stream;
+  const vkcu_poly_job o = one ? *one : vkcu_poly_job{};
+  if (log_n < 1 || log_n > (uint32_t)kMaxLogN || njobs < 1) return (int)cudaErrorInvalidValue;
+  if (has_lift(lift) && lift->count > VKCU_MAX_LIFT) return (int)cudaErrorInvalidValue;
+  const vkcu_lift* lp = has_lift(lift) ? lift : nullptr;
+  const bool aligned =
+      jobs != nullptr || (aligned32(o.a) && aligned32(o.b) && aligned32(o.c) && aligned32(o.scratch));
+  if (log_n > (uint32_t)kMaxCluster && !aligned) return (int)cudaErrorMisalignedAddress;
+  if (log_n > (uint32_t)kMaxCluster && qclass == VKCU_Q60)
+    return polymul_large<Mod60>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
+  if (log_n > (uint32_t)kMaxCluster && qclass == VKCU_Q62)
+    return polymul_large<Mod62>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
+  const vkcu_ntt_job ob{o.b, o.scratch, o.tw}, oa{o.a, o.c, o.tw}, oc{o.c, o.c, o.tw};
+  int e = b_ntt ? 0 : vkcu_ntt_forward(stream, b, njobs, &ob, log_n, qclass, sms);
+  if (!e) e = vkcu_ntt_forward(stream, a, njobs, &oa, log_n, qclass, sms);
+  if (!e) e = vkcu_pointwise(stream, jobs, njobs, one, log_n, qclass, sms);
+  if (!e) e = vkcu_ntt_inverse_lift(stream, c, njobs, &oc, log_n, qclass, sms, lift);
+  return e;
 }
 
 // The epilogue as its own element-wise pass: over `len` words at p, or over
@@ -601,13 +686,14 @@ extern "C" int vkcu_lift_jobs(void* stream, const vkcu_ntt_job* jobs, int njobs,
 // one job (the job's constants loaded once per chunk, not per word), each
 // thread two 16-byte pairs of c and of scratch per round, loads first.
 template <class M>
-__global__ void __launch_bounds__(256) k_pointwise(const vkcu_poly_job* __restrict__ jobs, int njobs, int log_n) {
+__global__ void __launch_bounds__(256)
+    k_pointwise(const vkcu_poly_job* __restrict__ jobs, int njobs, vkcu_poly_job one, int log_n) {
   const int lw = log_n < 11 ? log_n : 11;  // log2 of the words of a chunk
   const long cpj = 1L << (log_n - lw);    // chunks per job
   const long total = (long)njobs * cpj;
   const int pairs = 1 << (lw - 1);         // n >= 2
   for (long ch = blockIdx.x; ch < total; ch += gridDim.x) {
-    const vkcu_poly_job job = jobs[ch >> (log_n - lw)];
+    const vkcu_poly_job job = fetch_job(jobs, one, (int)(ch >> (log_n - lw)));
     const Tw t = load_tw(job.tw);
     const long base = (ch & (cpj - 1)) << lw;
     u64* c = reinterpret_cast<u64*>(job.c) + base;
@@ -630,13 +716,15 @@ __global__ void __launch_bounds__(256) k_pointwise(const vkcu_poly_job* __restri
   }
 }
 
-extern "C" int vkcu_pointwise(void* stream, const vkcu_poly_job* jobs, int njobs, uint32_t log_n, int qclass, int sms) {
-  if (njobs < 1 || !jobs || log_n < 1) return (int)cudaErrorInvalidValue;
+extern "C" int vkcu_pointwise(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one,
+                              uint32_t log_n, int qclass, int sms) {
+  if (njobs < 1 || (!jobs && !one) || log_n < 1) return (int)cudaErrorInvalidValue;
+  const vkcu_poly_job o = one ? *one : vkcu_poly_job{};
   const long chunks = (long)njobs << (log_n > 11 ? log_n - 11 : 0);
   long blocks = chunks;
   if (blocks > (long)sms * 8) blocks = (long)sms * 8;
   return by_class(qclass, [&](auto m) {
-    k_pointwise<decltype(m)><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(jobs, njobs, (int)log_n);
+    k_pointwise<decltype(m)><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(jobs, njobs, o, (int)log_n);
     vkcu_count_launches(1);
     return (int)cudaGetLastError();
   });

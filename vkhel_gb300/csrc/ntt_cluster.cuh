@@ -82,12 +82,13 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // first remote store (the fused polymul: 1-2.4 % faster; the forward
 // transform alone was 0.8 % slower this way and synchronizes before).
 // rbase: the cluster rank of this transform's CTA 0 (a larger cluster can
-// hold several transforms of C CTAs each).
-template <int LOGC, class S, bool SPLIT>
+// hold several transforms of C CTAs each).  SUB: a sub-block of a larger
+// transform after its global passes, twiddle multiplier `base`; its words are
+// forward-lazy already.
+template <int LOGC, class S, bool SPLIT, bool SUB = false>
 __device__ __forceinline__ void col_fwd(const u64* __restrict__ in, u64* sm, const cg::cluster_group& cl, int rank,
-                                        const Tw& t, int rbase = 0) {
+                                        const Tw& t, int rbase = 0, u32 base = 1u) {
   using K = Cols<LOGC, S>;
-  const ulonglong2 w0 = ld_tw(t.fwd + 1);
 #pragma unroll 1
   for (int k0 = 0; k0 < K::PER; k0 += K::H) {
     u64 v[K::H * K::W];
@@ -97,10 +98,7 @@ __device__ __forceinline__ void col_fwd(const u64* __restrict__ in, u64* sm, con
       for (int j = 0; j < K::W; j++) v[k * K::W + j] = ld_stream(in + K::col(rank, k0 + k) + (size_t)j * K::TM);
     static_for<0, K::H>([&](auto kc) {
       constexpr int k = decltype(kc)::value;
-#pragma unroll
-      for (int jj = 0; jj < K::W / 2; jj++)
-        ct_first<typename S::M>(v[k * K::W + jj], v[k * K::W + jj + K::W / 2], w0.x, w0.y, t);
-      ct_group<typename S::M, K::KK, 1, k * K::W>(v, RowTw{t.fwd, 1u}, t);
+      ct_first_group<typename S::M, K::KK, k * K::W, !SUB>(v, RowTw{t.fwd, base}, t);
     });
     if (SPLIT && k0 == 0) cluster_wait();
 #pragma unroll
@@ -113,10 +111,11 @@ __device__ __forceinline__ void col_fwd(const u64* __restrict__ in, u64* sm, con
 }
 
 // Inverse column pass: gather, global stages KK-1 .. 0 with n^-1 folded in,
-// canonical words to global memory; two rounds of H columns as above.
-template <int LOGC, class S, class Epi>
+// canonical words to global memory; two rounds of H columns as above.  SUB:
+// no fold, words below one unit.
+template <int LOGC, class S, bool SUB, class Epi>
 __device__ __forceinline__ void col_inv(u64* __restrict__ out, u64* sm, const cg::cluster_group& cl, int rank,
-                                        const Tw& t, const Epi& epi, int rbase = 0) {
+                                        const Tw& t, const Epi& epi, int rbase = 0, u32 base = 1u) {
   using K = Cols<LOGC, S>;
 #pragma unroll 1
   for (int k0 = 0; k0 < K::PER; k0 += K::H) {
@@ -129,7 +128,7 @@ __device__ __forceinline__ void col_inv(u64* __restrict__ out, u64* sm, const cg
     }
     static_for<0, K::H>([&](auto kc) {
       constexpr int k = decltype(kc)::value;
-      gs_group<typename S::M, K::KK, k * K::W, false, true>(v, RowTw{t.inv, 1u}, t);
+      gs_group<typename S::M, K::KK, k * K::W, false, !SUB>(v, RowTw{t.inv, base}, t);
     });
     epi.apply(v);
 #pragma unroll
@@ -158,33 +157,59 @@ __device__ __forceinline__ void sub_inv(u64* sm, const cg::cluster_group& cl, co
   cl.sync();
 }
 
-template <int LOGC, class S, bool LIFT>
+template <int LOGC, class S, bool LIFT, bool SUB = false>
 __device__ __forceinline__ void col_inv_out(u64* __restrict__ out, u64* sm, const cg::cluster_group& cl, int rank,
-                                            const Tw& t, const vkcu_lift* lift, int rbase = 0) {
+                                            const Tw& t, const vkcu_lift* lift, int rbase = 0, u32 base = 1u) {
   if constexpr (LIFT)
-    col_inv<LOGC, S>(out, sm, cl, rank, t, LiftFold(lift, t.q), rbase);
+    col_inv<LOGC, S, SUB>(out, sm, cl, rank, t, LiftFold(lift, t.q), rbase, base);
   else
-    col_inv<LOGC, S>(out, sm, cl, rank, t, NoLift{}, rbase);
+    col_inv<LOGC, S, SUB>(out, sm, cl, rank, t, NoLift{}, rbase, base);
 }
 
-template <int LOGC, class S>
+// Which cluster job (and, with SUB, which of its 2^sub_log sub-blocks) a
+// work item is: twiddle multiplier base, first word off, and the roots of the
+// last four stages for this CTA.
+template <int LOGC, class S, bool SUB>
+struct ClusterItem {
+  using K = Cols<LOGC, S>;
+  int job, sub, sub_log;
+  u32 base;
+  size_t off;
+  __device__ __forceinline__ ClusterItem(int w, int sub_log_)
+      : job(SUB ? w >> sub_log_ : w),
+        sub(SUB ? w & ((1 << sub_log_) - 1) : 0),
+        sub_log(SUB ? sub_log_ : 0),
+        base(SUB ? (1u << sub_log_) + (u32)sub : 1u),
+        off(SUB ? (size_t)sub * (K::C * K::SUB) : 0) {}
+  __device__ __forceinline__ u32 tw_mult(int rank) const { return base * K::C + (u32)rank; }
+  using Last = LastTable<SUB ? 0 : K::N16>;
+  __device__ __forceinline__ Last last(const ulonglong2* table, int rank) const {
+    return Last(table, sub * K::N16 + rank * (S::N / 16), (u32)K::N16 << sub_log);
+  }
+};
+
+template <int LOGC, class S, bool SUB = false>
 __global__ void __launch_bounds__(S::T, 1)
-    k_ntt_fwd_cluster(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one) {
+    k_ntt_fwd_cluster(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int sub_log) {
   using K = Cols<LOGC, S>;
   extern __shared__ u64 sm[];
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   const int ncl = (int)gridDim.x / K::C, cid = (int)blockIdx.x / K::C;
-  const u32 tw_mult = (u32)(K::C + rank);
+  const int items = SUB ? njobs << sub_log : njobs;
 #pragma unroll 1
-  for (int w = cid; w < njobs; w += ncl) {
-    const vkcu_ntt_job job = fetch_job(jobs, one, w);
+  for (int w = cid; w < items; w += ncl) {
+    const ClusterItem<LOGC, S, SUB> it(w, sub_log);
+    const vkcu_ntt_job job = fetch_job(jobs, one, it.job);
     const Tw t = load_tw(job.tw);
-    const LastTable<K::N16> last(t.fwd, rank * (S::N / 16), 0);
-    u64* out = reinterpret_cast<u64*>(job.out) + (size_t)rank * K::SUB;
+    const u32 tw_mult = it.tw_mult(rank);
+    const auto last = it.last(t.fwd, rank);
+    u64* out = reinterpret_cast<u64*>(job.out) + it.off;
+    const u64* in = SUB ? out : reinterpret_cast<const u64*>(job.in);
     cl.sync();
-    col_fwd<LOGC, S, false>(reinterpret_cast<const u64*>(job.in), sm, cl, rank, t);
+    col_fwd<LOGC, S, false, SUB>(in, sm, cl, rank, t, 0, it.base);
     sub_fwd<LOGC, S>(sm, cl, t, tw_mult);
+    out += (size_t)rank * K::SUB;
     fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
       const typename S::M::Out to(t);
 #pragma unroll
@@ -195,22 +220,23 @@ __global__ void __launch_bounds__(S::T, 1)
   cl.sync();
 }
 
-template <int LOGC, class S, bool LIFT>
+template <int LOGC, class S, bool LIFT, bool SUB = false>
 __global__ void __launch_bounds__(S::T, 1)
-    k_ntt_inv_cluster(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one,
+    k_ntt_inv_cluster(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int sub_log,
                       const __grid_constant__ vkcu_lift lift) {
   using K = Cols<LOGC, S>;
   extern __shared__ u64 sm[];
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   const int ncl = (int)gridDim.x / K::C, cid = (int)blockIdx.x / K::C;
-  const u32 tw_mult = (u32)(K::C + rank);
+  const int items = SUB ? njobs << sub_log : njobs;
 #pragma unroll 1
-  for (int w = cid; w < njobs; w += ncl) {
-    const vkcu_ntt_job job = fetch_job(jobs, one, w);
+  for (int w = cid; w < items; w += ncl) {
+    const ClusterItem<LOGC, S, SUB> it(w, sub_log);
+    const vkcu_ntt_job job = fetch_job(jobs, one, it.job);
     const Tw t = load_tw(job.tw);
-    const LastTable<K::N16> last(t.inv, rank * (S::N / 16), 0);
-    const u64* in = reinterpret_cast<const u64*>(job.in) + (size_t)rank * K::SUB;
+    const auto last = it.last(t.inv, rank);
+    const u64* in = reinterpret_cast<const u64*>(job.in) + it.off + (size_t)rank * K::SUB;
     cl.sync();
 #pragma unroll 1
     for (int i = 0; i < S::E / 16; i++) {
@@ -221,37 +247,45 @@ __global__ void __launch_bounds__(S::T, 1)
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
     }
-    sub_inv<LOGC, S>(sm, cl, t, tw_mult);
-    col_inv_out<LOGC, S, LIFT>(reinterpret_cast<u64*>(job.out), sm, cl, rank, t, &lift);
+    sub_inv<LOGC, S>(sm, cl, t, it.tw_mult(rank));
+    col_inv_out<LOGC, S, LIFT, SUB>(reinterpret_cast<u64*>(job.out) + it.off, sm, cl, rank, t, &lift, 0, it.base);
   }
   cl.sync();
 }
 
-template <int LOGC, class S, bool LIFT>
+// SUB: the sub-block products of a larger polymul: the global passes have left
+// their words of a in c and of b in scratch (b_ntt: NTT(b) whole in b).
+template <int LOGC, class S, bool LIFT, bool SUB = false>
 __global__ void __launch_bounds__(S::T, 1)
-    k_polymul_cluster(const vkcu_poly_job* __restrict__ jobs, int njobs, vkcu_poly_job one,
+    k_polymul_cluster(const vkcu_poly_job* __restrict__ jobs, int njobs, vkcu_poly_job one, int sub_log,
                       const __grid_constant__ vkcu_lift lift) {
   using K = Cols<LOGC, S>;
   extern __shared__ u64 sm[];
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   const int ncl = (int)gridDim.x / K::C, cid = (int)blockIdx.x / K::C;
-  const u32 tw_mult = (u32)(K::C + rank);
+  const int items = SUB ? njobs << sub_log : njobs;
   constexpr unsigned kSlice = (unsigned)(K::COLS * 8);
+  constexpr bool FLAGS = LIFT || SUB;  // the instantiations that read the job's flags
 #pragma unroll 1
-  for (int w = cid; w < njobs; w += ncl) {
-    const vkcu_poly_job job = fetch_job(jobs, one, w);
+  for (int w = cid; w < items; w += ncl) {
+    const ClusterItem<LOGC, S, SUB> it(w, sub_log);
+    const vkcu_poly_job job = fetch_job(jobs, one, it.job);
     const Tw t = load_tw_product<typename S::M>(job.tw);
-    // b holds NTT(b): phase 0 is skipped (read by the epilogue instantiations only)
-    const bool b_ntt = LIFT && (job.flags & VKCU_JOB_B_NTT);
-    u64* scratch = reinterpret_cast<u64*>(job.scratch) + (size_t)rank * K::SUB;
-    const LastTable<K::N16> last(t.fwd, rank * (S::N / 16), 0), last_inv(t.inv, rank * (S::N / 16), 0);
+    // b holds NTT(b): phase 0 is skipped
+    const bool b_ntt = FLAGS && (job.flags & VKCU_JOB_B_NTT);
+    const u32 tw_mult = it.tw_mult(rank);
+    const u64* a = (SUB ? reinterpret_cast<const u64*>(job.c) : reinterpret_cast<const u64*>(job.a)) + it.off;
+    const u64* b = (SUB && !b_ntt ? reinterpret_cast<const u64*>(job.scratch) : reinterpret_cast<const u64*>(job.b)) +
+                   it.off;
+    u64* scratch = reinterpret_cast<u64*>(job.scratch) + it.off + (size_t)rank * K::SUB;
+    const auto last = it.last(t.fwd, rank), last_inv = it.last(t.inv, rank);
     if ((int)threadIdx.x < K::W)  // this CTA's column slices of a, for phase 1
-      prefetch_l2(reinterpret_cast<const u64*>(job.a) + (size_t)threadIdx.x * K::TM + rank * K::COLS, kSlice);
+      prefetch_l2(a + (size_t)threadIdx.x * K::TM + rank * K::COLS, kSlice);
 #pragma unroll 1
     for (int ph = b_ntt ? 1 : 0; ph < 2; ph++) {
       cluster_arrive();  // done with every shared memory the column pass writes (col_fwd waits)
-      col_fwd<LOGC, S, true>(reinterpret_cast<const u64*>(ph ? job.a : job.b), sm, cl, rank, t);
+      col_fwd<LOGC, S, true, SUB>(ph ? a : b, sm, cl, rank, t, 0, it.base);
       sub_fwd<LOGC, S>(sm, cl, t, tw_mult);
       fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
         using M = typename S::M;
@@ -263,7 +297,7 @@ __global__ void __launch_bounds__(S::T, 1)
         } else {
           u64 bh[16];
           if (b_ntt) {
-            load16(bh, reinterpret_cast<const u64*>(job.b) + (size_t)rank * K::SUB + 16 * g);
+            load16(bh, b + (size_t)rank * K::SUB + 16 * g);
             reduce_operand16(bh, t);
           } else {
             unpark16(bh, scratch, g, S::N / 16);
@@ -278,7 +312,7 @@ __global__ void __launch_bounds__(S::T, 1)
         }
       });
     }
-    if (w + ncl < njobs && (int)threadIdx.x < K::W) {
+    if (!SUB && w + ncl < items && (int)threadIdx.x < K::W) {
       // the next job's b: its column slices, or (NTT(b) given) this CTA's sub-block
       const vkcu_poly_job nx = fetch_job(jobs, one, w + ncl);
       const size_t off = (LIFT && (nx.flags & VKCU_JOB_B_NTT)) ? (size_t)rank * K::SUB + (size_t)threadIdx.x * K::COLS
@@ -286,7 +320,7 @@ __global__ void __launch_bounds__(S::T, 1)
       prefetch_l2(reinterpret_cast<const u64*>(nx.b) + off, kSlice);
     }
     sub_inv<LOGC, S>(sm, cl, t, tw_mult);
-    col_inv_out<LOGC, S, LIFT>(reinterpret_cast<u64*>(job.c), sm, cl, rank, t, &lift);
+    col_inv_out<LOGC, S, LIFT, SUB>(reinterpret_cast<u64*>(job.c) + it.off, sm, cl, rank, t, &lift, 0, it.base);
   }
   cl.sync();
 }
@@ -380,7 +414,7 @@ int poly_cluster_lifted(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, c
 
 template <class M>
 int fwd_cluster(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int logc, int logs) {
-#define X(L, S) launch_cluster<L, S, k_ntt_fwd_cluster<L, S>>(st, njobs, jobs, njobs, one)
+#define X(L, S) launch_cluster<L, S, k_ntt_fwd_cluster<L, S>>(st, njobs, jobs, njobs, one, 0)
   VK_CLUSTER_SHAPES(X)
 #undef X
 }
@@ -390,7 +424,7 @@ int inv_cluster(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu
                 const vkcu_lift* lift) {
   if (lift) return inv_cluster_lifted<M>(st, jobs, njobs, one, logc, logs, *lift);
   const vkcu_lift l{};
-#define X(L, S) launch_cluster<L, S, k_ntt_inv_cluster<L, S, false>>(st, njobs, jobs, njobs, one, l)
+#define X(L, S) launch_cluster<L, S, k_ntt_inv_cluster<L, S, false>>(st, njobs, jobs, njobs, one, 0, l)
   VK_CLUSTER_SHAPES(X)
 #undef X
 }
@@ -400,8 +434,37 @@ int poly_cluster(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vk
                  const vkcu_lift* lift) {
   if (lift) return poly_cluster_lifted<M>(st, jobs, njobs, one, logc, logs, *lift);
   const vkcu_lift l{};
-#define X(L, S) launch_cluster<L, S, k_polymul_cluster<L, S, false>>(st, njobs, jobs, njobs, one, l)
+#define X(L, S) launch_cluster<L, S, k_polymul_cluster<L, S, false>>(st, njobs, jobs, njobs, one, 0, l)
   VK_CLUSTER_SHAPES(X)
+#undef X
+}
+
+// (log_n - sub_log is 16 or 14.)
+template <class M>
+int fwd_cluster_sub(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n,
+                    int sub_log) {
+#define X(L, S) launch_cluster<L, S, k_ntt_fwd_cluster<L, S, true>>(st, njobs << sub_log, jobs, njobs, one, sub_log)
+  return log_n - sub_log == 16 ? X(2, SubShape<M>) : X(3, Small11<M>);
+#undef X
+}
+
+template <class M>
+int inv_cluster_sub(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n,
+                    int sub_log) {
+  const vkcu_lift l{};
+#define X(L, S) \
+  launch_cluster<L, S, k_ntt_inv_cluster<L, S, false, true>>(st, njobs << sub_log, jobs, njobs, one, sub_log, l)
+  return log_n - sub_log == 16 ? X(2, SubShape<M>) : X(3, Small11<M>);
+#undef X
+}
+
+template <class M>
+int poly_cluster_sub(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int log_n,
+                     int sub_log) {
+  const vkcu_lift l{};
+#define X(L, S) \
+  launch_cluster<L, S, k_polymul_cluster<L, S, false, true>>(st, njobs << sub_log, jobs, njobs, one, sub_log, l)
+  return log_n - sub_log == 16 ? X(2, SubShape<M>) : X(3, Small11<M>);
 #undef X
 }
 

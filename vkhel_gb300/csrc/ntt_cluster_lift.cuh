@@ -7,7 +7,7 @@ namespace vk {
 template <class M>
 int inv_cluster_lifted(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int logc,
                        int logs, const vkcu_lift& l) {
-#define X(L, S) launch_cluster<L, S, k_ntt_inv_cluster<L, S, true>>(st, njobs, jobs, njobs, one, l)
+#define X(L, S) launch_cluster<L, S, k_ntt_inv_cluster<L, S, true>>(st, njobs, jobs, njobs, one, 0, l)
   VK_CLUSTER_SHAPES(X)
 #undef X
 }
@@ -15,7 +15,7 @@ int inv_cluster_lifted(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, con
 template <class M>
 int poly_cluster_lifted(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int logc,
                         int logs, const vkcu_lift& l) {
-#define X(L, S) launch_cluster<L, S, k_polymul_cluster<L, S, true>>(st, njobs, jobs, njobs, one, l)
+#define X(L, S) launch_cluster<L, S, k_polymul_cluster<L, S, true>>(st, njobs, jobs, njobs, one, 0, l)
   VK_CLUSTER_SHAPES(X)
 #undef X
 }

@@ -195,8 +195,8 @@ static __device__ __noinline__ U2 gs_first_slow63(u64 x, u64 y, u64 q) {
 //                bound); the sum, after sum(), is below sum_bound(B) units
 //   mul          the twiddle product of a difference, below one unit
 //   settle<B>    a word below B units brought below one unit
-//   Out          forward words -> canonical, parked (NTT(b) held for the
-//                pointwise product) or handed to the next kernel's first stage
+//   Out          forward words -> canonical, or parked (NTT(b) held for the
+//                pointwise product)
 //   Product      the pointwise product of a forward word and a parked or
 //                canonical one, below one unit (MONTGOMERY: times 2^-64)
 //   product_out  of two canonical words, the word the reference's elemmul stores
@@ -279,7 +279,6 @@ struct Mod60 {
       return pack(lo32(r), hi32(r) + k * hi32(nq));
     }
     __device__ __forceinline__ u64 canon(u64 x) const { return csub_sign(park(x), q); }
-    __device__ __forceinline__ u64 handoff(u64 x) const { return park(x); }
   };
   // x < 12q and y < 2q: (x y - ((x y) q^-1 mod 2^64) q) / 2^64 + q, below
   // 24 q q / 2^64 + q < 2.5q
@@ -328,7 +327,6 @@ struct Mod62 {
     __device__ __forceinline__ explicit Out(const Tw& t) : q(t.q), q2(t.q2) {}
     __device__ __forceinline__ u64 canon(u64 x) const { return canon4(x, q, q2); }
     __device__ __forceinline__ u64 park(u64 x) const { return canon(x); }
-    __device__ __forceinline__ u64 handoff(u64 x) const { return csub(x, q2); }
   };
   struct Product {
     u64 q, q2, mu;
@@ -377,7 +375,6 @@ struct Mod63 {
     __device__ __forceinline__ explicit Out(const Tw& t) : q(t.q) {}
     __device__ __forceinline__ u64 canon(u64 x) const { return csub(x, q); }
     __device__ __forceinline__ u64 park(u64 x) const { return csub(x, q); }
-    __device__ __forceinline__ u64 handoff(u64 x) const { return csub(x, q); }
   };
   // the reference's elemmul on canonical operands (its reduce64 returns them
   // unchanged): the full 128-bit product through reduce128
@@ -475,6 +472,20 @@ __device__ __forceinline__ void ct_group(u64 (&v)[NV], const R& tw, const Tw& t)
         M::template ct<M::reduce_at(u)>(v[G0 + r * 2 * half + jj], v[G0 + r * 2 * half + jj + half], w.x, w.y, t);
     });
   });
+}
+
+// The same from sub-stage 0, with the exact rule there where EXACT.
+template <class M, int KK, int G0, bool EXACT, int NV, class R>
+__device__ __forceinline__ void ct_first_group(u64 (&v)[NV], const R& tw, const Tw& t) {
+  if constexpr (EXACT) {
+    const ulonglong2 w0 = tw(0, 0);
+#pragma unroll
+    for (int jj = 0; jj < (1 << (KK - 1)); jj++)
+      ct_first<M>(v[G0 + jj], v[G0 + jj + (1 << (KK - 1))], w0.x, w0.y, t);
+    ct_group<M, KK, 1, G0>(v, tw, t);
+  } else {
+    ct_group<M, KK, 0, G0>(v, tw, t);
+  }
 }
 
 // Bound, in units, of word j of an inverse group of 2^KK words when sub-stage
@@ -609,10 +620,11 @@ constexpr int round_groups() {
 // First forward pass: this thread's words come from global memory (coalesced)
 // in rounds of 16 (all of a round's loads in flight at once; 32 words at once
 // would spill), then FIRSTK stages per group, results to shared memory.
-// The first sub-stage uses the exact first-stage rule; after the global pass
-// of a large transform the inputs always take its fast path.  The barrier that
-// frees the shared words comes after the first round's loads and butterflies.
-template <class S>
+// EXACT: the first sub-stage uses the exact first-stage rule (not after the
+// global passes of a large transform, whose words are forward-lazy already).
+// The barrier that frees the shared words comes after the first round's loads
+// and butterflies.
+template <class S, bool EXACT = true>
 __device__ __forceinline__ void fwd_first(u64* sm, const u64* __restrict__ in, const Tw& t, u32 tw_mult) {
   constexpr int KK = S::FIRSTK, G = S::E >> KK, TMIN = S::N >> KK;
   constexpr int GR = round_groups<KK, G>();
@@ -624,13 +636,9 @@ __device__ __forceinline__ void fwd_first(u64* sm, const u64* __restrict__ in, c
 #pragma unroll
       for (int j = 0; j < (1 << KK); j++)
         v[i * (1 << KK) + j] = ld_stream(in + S::tid() + (i0 + i) * S::T + j * TMIN);
-    const ulonglong2 w0 = ld_tw(t.fwd + tw_mult);
     static_for<0, GR>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
-#pragma unroll
-      for (int jj = 0; jj < (1 << (KK - 1)); jj++)
-        ct_first<typename S::M>(v[i * (1 << KK) + jj], v[i * (1 << KK) + jj + (1 << (KK - 1))], w0.x, w0.y, t);
-      ct_group<typename S::M, KK, 1, i * (1 << KK)>(v, RowTw{t.fwd, tw_mult}, t);
+      ct_first_group<typename S::M, KK, i * (1 << KK), EXACT>(v, RowTw{t.fwd, tw_mult}, t);
     });
     if (i0 == 0) __syncthreads();  // everyone is done with what the shared words held
 #pragma unroll
@@ -951,7 +959,7 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     u64* out = reinterpret_cast<u64*>(job.out) + ((size_t)sub << LOGN);
     const u64* in = sub_log ? out : reinterpret_cast<const u64*>(job.in);
     const u32 tw_mult = (1u << sub_log) + sub;
-    fwd_first<S>(sm, in, t, tw_mult);
+    fwd_first<S, !SUB>(sm, in, t, tw_mult);
     fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
       const typename M::Out to(t);
 #pragma unroll
@@ -1072,11 +1080,11 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
 // variant: 0 = default shape, 1 = two radix-16 groups per thread in flight,
 // 2 = the other words-per-thread shape (2^10..2^13 only); others -> 0.
 template <class M>
-int fwd_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sub_log,
-            int sms, int variant);
+int fwd_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sms,
+            int variant);
 template <class M>
-int inv_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sub_log,
-            int sms, int variant);
+int inv_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sms,
+            int variant);
 template <class M>
 int poly_cta(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int log_n, int sms,
              int variant);
@@ -1098,6 +1106,19 @@ int inv_cluster(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu
 template <class M>
 int poly_cluster(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int logc, int logs,
                  const vkcu_lift* lift = nullptr);
+
+// The sub-blocks of 2^(log_n - sub_log) words of transforms and products past
+// one cluster, between their global passes (in place in out, or from c and
+// scratch to c): 2^16 words on 4 CTAs, or 2^14 words on 8.
+template <class M>
+int fwd_cluster_sub(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n,
+                    int sub_log);
+template <class M>
+int inv_cluster_sub(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n,
+                    int sub_log);
+template <class M>
+int poly_cluster_sub(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int log_n,
+                     int sub_log);
 
 // The same families for 2^62 <= q < 2^63 (Mod63), default shape of each
 // degree, sub-blocks of 2^14 words for the cluster kernels (translation units

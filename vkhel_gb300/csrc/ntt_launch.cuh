@@ -6,14 +6,9 @@
 
 namespace vk {
 
-// sub_log > 0 only with log_n = 14 (the sub-blocks of larger transforms).
 template <class M>
-int fwd_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sub_log,
-            int sms, int variant) {
-#define X(L, E, U) \
-  launch_cta<Shape<L, E, U, M>, k_ntt_fwd<L, E, U, M, true>>(st, (long)njobs << sub_log, sms, jobs, njobs, one, sub_log)
-  if (sub_log) return variant == 1 ? X(14, 32, 2) : X(14, 32, 1);
-#undef X
+int fwd_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sms,
+            int variant) {
 retry:
 #define X(L, E, U) launch_cta<Shape<L, E, U, M>, k_ntt_fwd<L, E, U, M>>(st, (long)njobs, sms, jobs, njobs, one, 0)
   VK_FOR_LOGN(X)
@@ -21,14 +16,9 @@ retry:
 }
 
 template <class M>
-int inv_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sub_log,
-            int sms, int variant) {
+int inv_cta(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int log_n, int sms,
+            int variant) {
   const vkcu_lift none{};
-#define X(L, E, U)                                                                                                   \
-  launch_cta<Shape<L, E, U, M>, k_ntt_inv<L, E, U, false, M, true>>(st, (long)njobs << sub_log, sms, jobs, njobs, one, \
-                                                                     sub_log, none)
-  if (sub_log) return variant == 1 ? X(14, 32, 2) : X(14, 32, 1);
-#undef X
 retry:
 #define X(L, E, U) \
   launch_cta<Shape<L, E, U, M>, k_ntt_inv<L, E, U, false, M>>(st, (long)njobs, sms, jobs, njobs, one, 0, none)

@@ -11,10 +11,9 @@ int inv_cluster_wide(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const
   switch (logc * 2 + (lift ? 1 : 0)) {
 #define X(L)                                                                                                  \
   case 2 * L:                                                                                                 \
-    return launch_cluster<L, SubShape<Mod63>, k_ntt_inv_cluster<L, SubShape<Mod63>, false>>(st, njobs, jobs, njobs, one, \
-                                                                                  none);                      \
+    return launch_cluster<L, SubShape<Mod63>, k_ntt_inv_cluster<L, SubShape<Mod63>, false>>(st, njobs, jobs, njobs, one, 0, none); \
   case 2 * L + 1:                                                                                             \
-    return launch_cluster<L, SubShape<Mod63>, k_ntt_inv_cluster<L, SubShape<Mod63>, true>>(st, njobs, jobs, njobs, one, *lift);
+    return launch_cluster<L, SubShape<Mod63>, k_ntt_inv_cluster<L, SubShape<Mod63>, true>>(st, njobs, jobs, njobs, one, 0, *lift);
     X(1)
     X(2)
     X(3)
@@ -30,11 +29,9 @@ int poly_cluster_wide(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, con
   switch (logc * 2 + (lift ? 1 : 0)) {
 #define X(L)                                                                                                    \
   case 2 * L:                                                                                                   \
-    return launch_cluster<L, SubShape<Mod63>, k_polymul_cluster<L, SubShape<Mod63>, false>>(st, njobs, jobs, njobs, one,   \
-                                                                                  none);                        \
+    return launch_cluster<L, SubShape<Mod63>, k_polymul_cluster<L, SubShape<Mod63>, false>>(st, njobs, jobs, njobs, one, 0, none); \
   case 2 * L + 1:                                                                                               \
-    return launch_cluster<L, SubShape<Mod63>, k_polymul_cluster<L, SubShape<Mod63>, true>>(st, njobs, jobs, njobs, one,    \
-                                                                                 *lift);
+    return launch_cluster<L, SubShape<Mod63>, k_polymul_cluster<L, SubShape<Mod63>, true>>(st, njobs, jobs, njobs, one, 0, *lift);
     X(1)
     X(2)
     X(3)

@@ -22,7 +22,7 @@ int fwd_cluster_wide(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const
   switch (logc) {
 #define X(L) \
   case L:    \
-    return launch_cluster<L, SubShape<Mod63>, k_ntt_fwd_cluster<L, SubShape<Mod63>>>(st, njobs, jobs, njobs, one);
+    return launch_cluster<L, SubShape<Mod63>, k_ntt_fwd_cluster<L, SubShape<Mod63>>>(st, njobs, jobs, njobs, one, 0);
     X(1)
     X(2)
     X(3)
