@@ -916,16 +916,22 @@ __device__ __forceinline__ void unpark16(u64 (&v)[16], const u64* p, int g, int 
 }
 
 // Resident CTAs per SM the register budget is sized for: 512 threads per SM
-// (128 registers per thread, 16 warps) for the 32-words-per-thread shapes and
-// for the 16-words-per-thread transforms from n = 2^9 and polymuls from
-// n = 2^12; 384 threads (about 170 registers) for the other 16-word shapes.
-// Left at 384, the 2^12 shapes took 222 registers (one CTA of 256 threads per
-// SM): 128 made them 9 % (polymul) and 17 % (transforms) faster; the 2^9 ..
-// 2^11 transforms gained 4 %, the polymuls of those sizes lost 2-3 %, and
-// n = 2^8 (16-thread CTAs) spills above 384.
+// (128 registers per thread, 16 warps) for the 32-words-per-thread shapes, the
+// 16-words-per-thread transforms of n >= 2^12 and polymuls of n >= 2^12; 640
+// threads (102 registers, 20 warps) for the 16-word transforms of 2^9 .. 2^11;
+// 384 threads (about 170 registers) for the other 16-word shapes.  Measured:
+// the 2^12 shapes at 384 took 222 registers (one CTA of 256 threads per SM),
+// 128 made them 9 % (polymul) and 17 % (transforms) faster; 640 against 512
+// makes the transforms of 2^9 .. 2^11 5-6 % faster (16384 forward ones of 2^10
+// 114.6 -> 108.8 us, inverse 123.0 -> 116.9) but the polymuls slower wherever
+// the jobs are few (2048 of 2^10 47.8 -> 52.9 us, 54.1 at 512), whose rounds
+// then wait on one thread's chain; n = 2^8 (16-thread CTAs) spills above 384.
 template <int LOGN, int E, bool POLY = false>
 constexpr int min_blocks() {
-  constexpr int budget = E >= 32 || LOGN >= (POLY ? 12 : 9) ? 512 : 384;
+  constexpr int budget = E >= 32                              ? 512
+                         : !POLY && LOGN >= 9 && LOGN <= 11    ? 640
+                         : LOGN >= 12                          ? 512
+                                                               : 384;
   return (budget / ((1 << LOGN) / E)) < 1 ? 1 : (budget / ((1 << LOGN) / E));
 }
 
