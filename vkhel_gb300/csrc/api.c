@@ -510,7 +510,8 @@ static void forward_impl(const struct vkhel_vector *a, struct vkhel_vector *res,
 	if (t->n == 1)
 		return; /* the stage loop of src/vector.c:537 runs zero times */
 	const vkcu_ntt_job job = {a->dev, res->dev, d->dev_set};
-	finish(res->ctx, vkcu_ntt_forward(res->ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), res->ctx->sms),
+	finish(res->ctx, vkcu_ntt_forward(res->ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), res->ctx->sms,
+			res->ctx->sms),
 			"forward_transform");
 }
 
@@ -535,7 +536,7 @@ static int inverse_impl(const struct vkhel_vector *a, struct vkhel_vector *res, 
 	int e = 0;
 	if (t->n > 1) {
 		const vkcu_ntt_job job = {a->dev, res->dev, d->dev_set};
-		e = vkcu_ntt_inverse_lift(ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms, lp);
+		e = vkcu_ntt_inverse_lift(ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms, ctx->sms, lp);
 	}
 	/* src/vector.c:635-638 scales result->length words by n^-1: words past n
 	 * (and, for n == 1, the untouched result) are scaled here. */
@@ -688,7 +689,7 @@ static int polymul_impl(const struct vkhel_vector *a, const struct vkhel_vector 
 	int e;
 	if (fused) {
 		const vkcu_poly_job job = {a->dev, b->dev, res->dev, scratch, d->dev_set, b_ntt ? VKCU_JOB_B_NTT : 0};
-		e = vkcu_polymul_lift(ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms, lp, b_ntt);
+		e = vkcu_polymul_lift(ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms, ctx->sms, lp, b_ntt);
 	} else {
 		const vkcu_poly_job job = {a->dev, b->dev, res->dev, scratch, d->dev_set, b_ntt ? VKCU_JOB_B_NTT : 0};
 		e = vkcu_polymul_composed(ctx->stream, NULL, NULL, NULL, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms,

@@ -287,7 +287,7 @@ static int cmp_rec(const void *x, const void *y) {
  * product (b -> scratch, a -> c, product, inverse of c) over the class's slice
  * of the ntt-job array (laid out at 3 * first: b jobs, a jobs, c jobs).  A
  * class's epilogue rides on its last launch. */
-int vkh_issue_classes(void *stream, int sms, const vkcu_poly_job *dev_poly, const vkcu_ntt_job *dev_ntt,
+int vkh_issue_classes(void *stream, int sms, int avail, const vkcu_poly_job *dev_poly, const vkcu_ntt_job *dev_ntt,
 		const struct vkh_job_class *classes, uint32_t nclasses, const vkcu_lift *lifts) {
 	for (uint32_t k = 0; k < nclasses; k++) {
 		const struct vkh_job_class *cl = &classes[k];
@@ -295,12 +295,13 @@ int vkh_issue_classes(void *stream, int sms, const vkcu_poly_job *dev_poly, cons
 		const vkcu_ntt_job *tj = dev_ntt + 3 * (size_t) cl->first;
 		int e;
 		if (cl->kind == VKH_JOB_FORWARD) {
-			e = vkcu_ntt_forward(stream, tj, (int) cl->count, NULL, cl->log_n, cl->qclass, sms);
+			e = vkcu_ntt_forward(stream, tj, (int) cl->count, NULL, cl->log_n, cl->qclass, sms, avail);
 		} else if (cl->kind == VKH_JOB_INVERSE) {
-			e = vkcu_ntt_inverse_lift(stream, tj, (int) cl->count, NULL, cl->log_n, cl->qclass, sms, lift);
+			e = vkcu_ntt_inverse_lift(stream, tj, (int) cl->count, NULL, cl->log_n, cl->qclass, sms, avail,
+					lift);
 		} else if (cl->fused) {
 			e = vkcu_polymul_lift(stream, dev_poly + cl->first, (int) cl->count, NULL, cl->log_n, cl->qclass, sms,
-					lift, (int) cl->b_ntt);
+					avail, lift, (int) cl->b_ntt);
 		} else {
 			e = vkcu_polymul_composed(stream, dev_poly + cl->first, tj, tj + cl->count, tj + 2 * (size_t) cl->count,
 					(int) cl->count, NULL, cl->log_n, cl->qclass, sms, lift, (int) cl->b_ntt);
@@ -336,6 +337,13 @@ void vkh_fill_ntt_jobs(const vkcu_poly_job *poly, vkcu_ntt_job *ntt, const struc
 	}
 }
 
+/* Butterflies of a class, up to a common factor: its share of the SMs beside
+ * the classes that run with it. */
+static uint64_t class_work(const struct vkh_job_class *cl) {
+	const uint64_t transforms = cl->kind != VKH_JOB_POLYMUL ? 1 : cl->b_ntt ? 2 : 3;
+	return transforms * cl->log_n * ((uint64_t) cl->count << cl->log_n);
+}
+
 /* Same, with class k > 0 on aux[k - 1]: the auxiliary streams wait for
  * `fork` recorded on `stream`, and `stream` waits for each join[k - 1], so
  * the classes run concurrently and the whole still ends on `stream` (this is
@@ -344,12 +352,16 @@ int vkh_issue_classes_forked(void *stream, void *const *aux, void *fork, void *c
 		const vkcu_poly_job *dev_poly, const vkcu_ntt_job *dev_ntt, const struct vkh_job_class *classes,
 		uint32_t nclasses, const vkcu_lift *lifts) {
 	if (nclasses < 2)
-		return vkh_issue_classes(stream, sms, dev_poly, dev_ntt, classes, nclasses, lifts);
+		return vkh_issue_classes(stream, sms, sms, dev_poly, dev_ntt, classes, nclasses, lifts);
 	int e = vkcu_event_record(fork, stream);
 	for (uint32_t k = 1; !e && k < nclasses; k++)
 		e = vkcu_stream_wait(aux[k - 1], fork);
+	uint64_t total = 0;
+	for (uint32_t k = 0; k < nclasses; k++)
+		total += class_work(&classes[k]);
 	for (uint32_t k = 0; !e && k < nclasses; k++)
-		e = vkh_issue_classes(k ? aux[k - 1] : stream, sms, dev_poly, dev_ntt, &classes[k], 1, lifts);
+		e = vkh_issue_classes(k ? aux[k - 1] : stream, sms, (int) (class_work(&classes[k]) * sms / total), dev_poly,
+				dev_ntt, &classes[k], 1, lifts);
 	for (uint32_t k = 1; !e && k < nclasses; k++) {
 		e = vkcu_event_record(join[k - 1], aux[k - 1]);
 		if (!e)
@@ -370,7 +382,7 @@ static int issue(struct vkhel_batch *b) {
 	if (b->naux)
 		return vkh_issue_classes_forked(b->ctx->stream, b->aux, b->fork, b->join, b->ctx->sms, b->dev_poly,
 				b->dev_ntt, b->classes, b->nclasses, b->lifts);
-	return vkh_issue_classes(b->ctx->stream, b->ctx->sms, b->dev_poly, b->dev_ntt, b->classes, b->nclasses,
+	return vkh_issue_classes(b->ctx->stream, b->ctx->sms, b->ctx->sms, b->dev_poly, b->dev_ntt, b->classes, b->nclasses,
 			b->lifts);
 }
 

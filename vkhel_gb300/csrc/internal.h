@@ -110,8 +110,9 @@ struct vkh_job_class {
 	uint32_t lift;         /* index into the lift table, 0 = none */
 	uint32_t b_ntt;        /* polymul jobs whose b holds NTT(b) (VKCU_JOB_B_NTT) */
 };
-/* lifts: table indexed by vkh_job_class.lift (NULL when no class has one) */
-int vkh_issue_classes(void *stream, int sms, const vkcu_poly_job *dev_poly, const vkcu_ntt_job *dev_ntt,
+/* lifts: table indexed by vkh_job_class.lift (NULL when no class has one);
+ * avail: the SMs these classes may count on beside concurrent ones */
+int vkh_issue_classes(void *stream, int sms, int avail, const vkcu_poly_job *dev_poly, const vkcu_ntt_job *dev_ntt,
 		const struct vkh_job_class *classes, uint32_t nclasses, const vkcu_lift *lifts);
 int vkh_issue_classes_forked(void *stream, void *const *aux, void *fork, void *const *join, int sms,
 		const vkcu_poly_job *dev_poly, const vkcu_ntt_job *dev_ntt, const struct vkh_job_class *classes,

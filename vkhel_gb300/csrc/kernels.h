@@ -195,7 +195,9 @@ typedef struct vkcu_lift {
 /* ---- transforms (ntt.cu) ----
  * `jobs` is a device array of `njobs` jobs that all share log_n and the
  * modulus class, or NULL to launch the single job `one` passed by value.
- * `qclass` names the butterfly arithmetic (ntt_core.cuh): how far above q a
+ * `avail` of the GPU's `sms` SMs is what the launch may count on when it
+ * splits few jobs over more of them (all, or a class's share of concurrent
+ * ones).  `qclass` names the butterfly arithmetic (ntt_core.cuh): how far above q a
  * lazy word may go in 64 bits. */
 enum {
 	VKCU_Q60 = 0,                /* odd q < 2^60: words below 12q */
@@ -206,9 +208,7 @@ static inline int vkcu_qclass(uint64_t q) {
 	return q < ((uint64_t) 1 << 60) && (q & 1) ? VKCU_Q60 : q < ((uint64_t) 1 << 62) ? VKCU_Q62 : VKCU_Q63;
 }
 int vkcu_ntt_forward(void *stream, const vkcu_ntt_job *jobs, int njobs,
-		const vkcu_ntt_job *one, uint32_t log_n, int qclass, int sms);
-int vkcu_ntt_inverse(void *stream, const vkcu_ntt_job *jobs, int njobs,
-		const vkcu_ntt_job *one, uint32_t log_n, int qclass, int sms);
+		const vkcu_ntt_job *one, uint32_t log_n, int qclass, int sms, int avail);
 int vkcu_polymul(void *stream, const vkcu_poly_job *jobs, int njobs,
 		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms);
 /* The same with an epilogue (`lift` NULL or count 0: none); fused into the
@@ -217,9 +217,9 @@ int vkcu_polymul(void *stream, const vkcu_poly_job *jobs, int njobs,
  * the fused kernels read that flag, so such jobs run those (with no steps
  * when `lift` has none) and the plain kernels stay as lean as before. */
 int vkcu_ntt_inverse_lift(void *stream, const vkcu_ntt_job *jobs, int njobs,
-		const vkcu_ntt_job *one, uint32_t log_n, int qclass, int sms, const vkcu_lift *lift);
+		const vkcu_ntt_job *one, uint32_t log_n, int qclass, int sms, int avail, const vkcu_lift *lift);
 int vkcu_polymul_lift(void *stream, const vkcu_poly_job *jobs, int njobs,
-		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms, const vkcu_lift *lift, int b_ntt);
+		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms, int avail, const vkcu_lift *lift, int b_ntt);
 /* The epilogue alone, in place on `len` words at p (modulus q for TABLE_Q
  * steps), or on the n output words of every job. */
 int vkcu_lift_range(void *stream, uint64_t *p, uint64_t len, uint64_t q, int sms, const vkcu_lift *lift);

@@ -286,20 +286,59 @@ static bool jobs_aligned(const vkcu_ntt_job* jobs, const vkcu_ntt_job* one) {
   return jobs != nullptr || (aligned32(one->in) && aligned32(one->out));
 }
 
-// Few jobs of n = 2^12 .. 2^16 (at most one per 8 SMs, e.g. a single call):
-// each runs on a cluster of 8 CTAs with 2^9 .. 2^13-word sub-blocks instead
-// of one CTA (n <= 2^14) or a cluster of 2 / 4 CTAs (n = 2^15 / 2^16), so it
-// uses 8 SMs.  Tuning entry (family 3, log_n 1) = 1 turns this off.
-// Cluster size (log2) for a few jobs of n = 2^12 .. 2^16, 0 for none: 8
-// CTAs when there is at most one job per 8 SMs; 16 for a single call (one
-// job passed by value) of n >= 2^14 (tuning entry (3, 3) = 1 keeps it on 8).
-// Batches and server micro-batches keep 8: their classes run beside other
-// kernels, and a 16-CTA cluster can only start once 16 SMs of one GPC are
-// free at the same time.
-static int split_small(int njobs, uint32_t log_n, int sms, bool single) {
+// log2 of the CTAs that share a job where a launch has fewer jobs than the SMs
+// it may count on (`avail`: all, or its share of a batch's concurrent classes),
+// 0 for the degree's own kernel (one CTA to 2^14, 2 / 4 CTAs at 2^15 / 2^16).
+// A single call (one job passed by value) of n >= 2^14 takes 16 CTAs; batches
+// and server micro-batches keep to 8, since their classes run beside other
+// kernels and a 16-CTA cluster can only start once 16 SMs of one GPC are free
+// at the same time.  Tuning entry (3, 1) = 1 turns the split off, (3, 3) = 1
+// keeps single calls on 8.  The lines, from products timed per job count and
+// split on 152 SMs (us; the kernel without a split / on 2 / 4 / 8 CTAs a job):
+//   2^13: 30 jobs 33 / 25 / 21 / 21, 60: 33 / 25 / 25 / 25, 76: 33 / 25 / 41 / 41,
+//         100: 33 / 37 / 43 / 43
+//   2^14: 30 jobs 64 / 45 / 27 / 27, 50: 66 / 45 / 40 / 45, 76: 66 / 47 / 57 / 67,
+//         100: 66 / 70 / 57 / 72
+//   2^15: (2 / 4 / 8) 19 jobs 70 / 47 / 41, 50: 72 / 75 / 62, 60: 72 / 76 / 88
+//   2^16: (4 / 8) 19 jobs 78 / 78, 24: 78 / 86
+static int split_log(long njobs, uint32_t log_n, long avail, bool single) {
   if (log_n < 12 || log_n > 16 || vkh_variant(3, 1) != 0) return 0;
-  if (single && log_n >= 14 && (long)njobs * 16 <= (long)sms && vkh_variant(3, 3) == 0) return 4;
-  return (long)njobs * 8 <= (long)sms ? 3 : 0;
+  if (single && log_n >= 14 && njobs * 16 <= avail && vkh_variant(3, 3) == 0) return 4;
+  switch (log_n) {
+    case 13: return njobs * 4 <= avail ? 3 : njobs * 2 <= avail ? 1 : 0;
+    case 14: return njobs * 5 <= avail ? 3 : njobs * 5 <= 2 * avail ? 2 : njobs * 2 <= avail ? 1 : 0;
+    case 15: return njobs * 3 <= avail ? 3 : 0;
+    default: return njobs * 8 <= avail ? 3 : 0;
+  }
+}
+
+// The last jobs of a launch whose kernel runs `round` jobs at a time, one per
+// SM or SM pair: those past the whole rounds, where a split finishes them
+// sooner than a round of their own.  Only where the launch has the GPU to
+// itself -- concurrent classes fill a partial round anyway.  Products of 2^14
+// in us, without / with the split tail: 160 (8 past the round) 129 / 91, 200
+// (48) 131 / 108, 344 (40) 193 / 172; of 2^15, 80 (4) 139 / 103, 160 (8) 207 /
+// 172, 120 (44) 142 / 135.  A tail of 77 .. 106 products of 2^14 on 4 CTAs each
+// still gains (256 products 131.6 -> 128.2), the shorter transforms and
+// products with NTT(b) given lose 2-4 % there, as do 48 products of 2^15 with
+// NTT(b) given.
+struct Tail {
+  int jobs = 0, lc = 0;
+  // `long_job`: a product with both forward transforms
+  Tail(bool batch, int njobs, uint32_t log_n, int round, int sms, int avail, bool long_job) {
+    if (!batch || avail < sms || round < 1 || njobs <= round || vkh_variant(3, 1) != 0) return;
+    const int r = njobs % round;
+    if (r == 0 || (log_n == 15 && r * 10 > 3 * sms)) return;
+    lc = split_log(r, log_n, sms, false);
+    if (!lc && log_n == 14 && long_job && r * 10 <= 7 * sms) lc = 2;
+    if (lc) jobs = r;
+  }
+};
+// Jobs of one round: 2^14 words take an SM each (139 KB of shared memory),
+// 2^13 ones in the 512-thread shape (variant 2) too, 2^15 ones two SMs; 0
+// for the others, whose rounds overlap.
+static int round_jobs(uint32_t log_n, int variant, int sms) {
+  return log_n == 14 || (log_n == 13 && variant == 2) ? sms : log_n == 15 ? sms / 2 : 0;
 }
 
 // f(M{}) for the modulus class's M; the wide class has launchers of its own.
@@ -313,7 +352,7 @@ static int by_class(int qclass, F&& f) {
 
 template <class M>
 static int forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one, uint32_t log_n,
-                   int sms) {
+                   int sms, int avail) {
   cudaStream_t st = (cudaStream_t)stream;
   const vkcu_ntt_job o = one ? *one : vkcu_ntt_job{};
   if (log_n < 1 || log_n > (uint32_t)kMaxLogN || njobs < 1) return (int)cudaErrorInvalidValue;
@@ -325,16 +364,21 @@ static int forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
     if (log_n <= (uint32_t)kMaxCta) return fwd_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms);
     if (log_n <= (uint32_t)kMaxCluster) return fwd_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta);
   } else {
-    if (const int lc = split_small(njobs, log_n, sms, jobs == nullptr)) {
+    if (const int lc = split_log(njobs, log_n, avail, jobs == nullptr)) {
       const int e = fwd_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc);
       // a GPU that cannot host 16-CTA clusters: the set-up refuses before any launch
       return e == (int)cudaErrorInvalidConfiguration && lc == 4
                  ? fwd_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3)
                  : e;
     }
-    if (log_n <= (uint32_t)kMaxCta)
-      return fwd_cta<M>(st, jobs, njobs, o, (int)log_n, sms, vkh_variant_jobs(1, (int)log_n, njobs, sms));
-    if (log_n <= (uint32_t)kMaxCluster) return fwd_cluster<M>(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta);
+    if (log_n <= (uint32_t)kMaxCluster) {
+      const int variant = log_n <= (uint32_t)kMaxCta ? vkh_variant_jobs(1, (int)log_n, njobs, sms) : 0;
+      const Tail tail(jobs != nullptr, njobs, log_n, round_jobs(log_n, variant, sms), sms, avail, false);
+      const int main = njobs - tail.jobs;
+      const int e = log_n <= (uint32_t)kMaxCta ? fwd_cta<M>(st, jobs, main, o, (int)log_n, sms, variant)
+                                               : fwd_cluster<M>(st, jobs, main, o, (int)log_n - kMaxCta, kMaxCta);
+      return e || !tail.jobs ? e : fwd_cluster<M>(st, jobs + main, tail.jobs, o, tail.lc, (int)log_n - tail.lc);
+    }
   }
   if constexpr (kWide<M>) {
     const int sub_log = (int)log_n - kMaxCta;
@@ -348,15 +392,15 @@ static int forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
 }
 
 extern "C" int vkcu_ntt_forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
-                                uint32_t log_n, int qclass, int sms) {
-  return by_class(qclass, [&](auto m) { return forward<decltype(m)>(stream, jobs, njobs, one, log_n, sms); });
+                                uint32_t log_n, int qclass, int sms, int avail) {
+  return by_class(qclass, [&](auto m) { return forward<decltype(m)>(stream, jobs, njobs, one, log_n, sms, avail); });
 }
 
 static bool has_lift(const vkcu_lift* lift) { return lift && lift->count > 0; }
 
 template <class M>
 static int inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one, uint32_t log_n, int sms,
-                   const vkcu_lift* lift) {
+                   int avail, const vkcu_lift* lift) {
   cudaStream_t st = (cudaStream_t)stream;
   const vkcu_ntt_job o = one ? *one : vkcu_ntt_job{};
   if (log_n < 1 || log_n > (uint32_t)kMaxLogN || njobs < 1) return (int)cudaErrorInvalidValue;
@@ -374,17 +418,22 @@ static int inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
       if (log_n <= (uint32_t)kMaxCta) return inv_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms, lp);
       if (log_n <= (uint32_t)kMaxCluster) return inv_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta, lp);
     } else {
-      if (const int lc = split_small(njobs, log_n, sms, jobs == nullptr)) {
+      if (const int lc = split_log(njobs, log_n, avail, jobs == nullptr)) {
         const int r = inv_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc, lp);
         return r == (int)cudaErrorInvalidConfiguration && lc == 4
                    ? inv_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3, lp)
                    : r;
       }
-      if (log_n <= (uint32_t)kMaxCta) {
-        if (lifted) return inv_cta_lift<M>(st, jobs, njobs, o, (int)log_n, sms, *lift);
-        return inv_cta<M>(st, jobs, njobs, o, (int)log_n, sms, vkh_variant_jobs(2, (int)log_n, njobs, sms));
+      if (log_n <= (uint32_t)kMaxCluster) {
+        // the lifted CTA kernels run in the default shape
+        const int variant = log_n <= (uint32_t)kMaxCta && !lifted ? vkh_variant_jobs(2, (int)log_n, njobs, sms) : 0;
+        const Tail tail(jobs != nullptr, njobs, log_n, round_jobs(log_n, variant, sms), sms, avail, false);
+        const int main = njobs - tail.jobs;
+        const int r = log_n > (uint32_t)kMaxCta ? inv_cluster<M>(st, jobs, main, o, (int)log_n - kMaxCta, kMaxCta, lp)
+                      : lifted                  ? inv_cta_lift<M>(st, jobs, main, o, (int)log_n, sms, *lift)
+                                                : inv_cta<M>(st, jobs, main, o, (int)log_n, sms, variant);
+        return r || !tail.jobs ? r : inv_cluster<M>(st, jobs + main, tail.jobs, o, tail.lc, (int)log_n - tail.lc, lp);
       }
-      if (log_n <= (uint32_t)kMaxCluster) return inv_cluster<M>(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta, lp);
     }
     int sub_log;
     if constexpr (kWide<M>) {
@@ -402,18 +451,14 @@ static int inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
 }
 
 extern "C" int vkcu_ntt_inverse_lift(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
-                                     uint32_t log_n, int qclass, int sms, const vkcu_lift* lift) {
-  return by_class(qclass, [&](auto m) { return inverse<decltype(m)>(stream, jobs, njobs, one, log_n, sms, lift); });
-}
-
-extern "C" int vkcu_ntt_inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job* one,
-                                uint32_t log_n, int qclass, int sms) {
-  return vkcu_ntt_inverse_lift(stream, jobs, njobs, one, log_n, qclass, sms, nullptr);
+                                     uint32_t log_n, int qclass, int sms, int avail, const vkcu_lift* lift) {
+  return by_class(qclass,
+                  [&](auto m) { return inverse<decltype(m)>(stream, jobs, njobs, one, log_n, sms, avail, lift); });
 }
 
 template <class M>
 static int polymul(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one, uint32_t log_n,
-                   int sms, const vkcu_lift* lift, int b_ntt) {
+                   int sms, int avail, const vkcu_lift* lift, int b_ntt) {
   cudaStream_t st = (cudaStream_t)stream;
   const vkcu_poly_job o = one ? *one : vkcu_poly_job{};
   if (log_n < 8 || log_n > (uint32_t)kMaxCluster || njobs < 1) return (int)cudaErrorInvalidValue;
@@ -424,30 +469,31 @@ static int polymul(void* stream, const vkcu_poly_job* jobs, int njobs, const vkc
     if (log_n <= (uint32_t)kMaxCta) return poly_cta_wide(st, jobs, njobs, o, (int)log_n, sms, lp);
     return poly_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta, lp);
   } else {
-    if (const int lc = split_small(njobs, log_n, sms, jobs == nullptr)) {
+    if (const int lc = split_log(njobs, log_n, avail, jobs == nullptr)) {
       const int e = poly_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc, lp);
       return e == (int)cudaErrorInvalidConfiguration && lc == 4
                  ? poly_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3, lp)
                  : e;
     }
-    if (log_n <= (uint32_t)kMaxCta) {
-      const int variant = vkh_variant_jobs(0, (int)log_n, njobs, sms);
-      if (lp) return poly_cta_lift<M>(st, jobs, njobs, o, (int)log_n, sms, variant, *lp);
-      return poly_cta<M>(st, jobs, njobs, o, (int)log_n, sms, variant);
-    }
-    return poly_cluster<M>(st, jobs, njobs, o, (int)log_n - kMaxCta, kMaxCta, lp);
+    const int variant = log_n <= (uint32_t)kMaxCta ? vkh_variant_jobs(0, (int)log_n, njobs, sms) : 0;
+    const Tail tail(jobs != nullptr, njobs, log_n, round_jobs(log_n, variant, sms), sms, avail, !b_ntt);
+    const int main = njobs - tail.jobs;
+    const int e = log_n > (uint32_t)kMaxCta ? poly_cluster<M>(st, jobs, main, o, (int)log_n - kMaxCta, kMaxCta, lp)
+                  : lp                      ? poly_cta_lift<M>(st, jobs, main, o, (int)log_n, sms, variant, *lp)
+                                            : poly_cta<M>(st, jobs, main, o, (int)log_n, sms, variant);
+    return e || !tail.jobs ? e : poly_cluster<M>(st, jobs + main, tail.jobs, o, tail.lc, (int)log_n - tail.lc, lp);
   }
 }
 
 extern "C" int vkcu_polymul_lift(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one,
-                                 uint32_t log_n, int qclass, int sms, const vkcu_lift* lift, int b_ntt) {
-  return by_class(qclass,
-                  [&](auto m) { return polymul<decltype(m)>(stream, jobs, njobs, one, log_n, sms, lift, b_ntt); });
+                                 uint32_t log_n, int qclass, int sms, int avail, const vkcu_lift* lift, int b_ntt) {
+  return by_class(
+      qclass, [&](auto m) { return polymul<decltype(m)>(stream, jobs, njobs, one, log_n, sms, avail, lift, b_ntt); });
 }
 
 extern "C" int vkcu_polymul(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one,
                             uint32_t log_n, int qclass, int sms) {
-  return vkcu_polymul_lift(stream, jobs, njobs, one, log_n, qclass, sms, nullptr, 0);
+  return vkcu_polymul_lift(stream, jobs, njobs, one, log_n, qclass, sms, sms, nullptr, 0);
 }
 
 // A product past one cluster (2^18 .. 2^26, q < 2^62): the global passes of b
@@ -488,10 +534,10 @@ extern "C" int vkcu_polymul_composed(void* stream, const vkcu_poly_job* jobs, co
   if (log_n > (uint32_t)kMaxCluster && qclass == VKCU_Q62)
     return polymul_large<Mod62>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
   const vkcu_ntt_job ob{o.b, o.scratch, o.tw}, oa{o.a, o.c, o.tw}, oc{o.c, o.c, o.tw};
-  int e = b_ntt ? 0 : vkcu_ntt_forward(stream, b, njobs, &ob, log_n, qclass, sms);
-  if (!e) e = vkcu_ntt_forward(stream, a, njobs, &oa, log_n, qclass, sms);
+  int e = b_ntt ? 0 : vkcu_ntt_forward(stream, b, njobs, &ob, log_n, qclass, sms, sms);
+  if (!e) e = vkcu_ntt_forward(stream, a, njobs, &oa, log_n, qclass, sms, sms);
   if (!e) e = vkcu_pointwise(stream, jobs, njobs, one, log_n, qclass, sms);
-  if (!e) e = vkcu_ntt_inverse_lift(stream, c, njobs, &oc, log_n, qclass, sms, lift);
+  if (!e) e = vkcu_ntt_inverse_lift(stream, c, njobs, &oc, log_n, qclass, sms, sms, lift);
   return e;
 }
 

@@ -188,8 +188,18 @@ struct ClusterItem {
   }
 };
 
+// CTAs per SM the register budget is sized for: two of 256 threads (128
+// registers), so that an SM holds a CTA of each of two clusters (19 products
+// of 2^15 words on 8 CTAs each 54 -> 42 us, 19 of 2^16 100 -> 78 us); the
+// smaller shapes are single calls first of all, and 128 registers cost those
+// 4-10 % (one product of 2^13 19.7 -> 20.5 us).
+template <class S>
+constexpr int cluster_blocks() {
+  return S::T == 256 ? 2 : 1;
+}
+
 template <int LOGC, class S, bool SUB = false>
-__global__ void __launch_bounds__(S::T, 1)
+__global__ void __launch_bounds__(S::T, cluster_blocks<S>())
     k_ntt_fwd_cluster(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int sub_log) {
   using K = Cols<LOGC, S>;
   extern __shared__ u64 sm[];
@@ -221,7 +231,7 @@ __global__ void __launch_bounds__(S::T, 1)
 }
 
 template <int LOGC, class S, bool LIFT, bool SUB = false>
-__global__ void __launch_bounds__(S::T, 1)
+__global__ void __launch_bounds__(S::T, cluster_blocks<S>())
     k_ntt_inv_cluster(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one, int sub_log,
                       const __grid_constant__ vkcu_lift lift) {
   using K = Cols<LOGC, S>;
@@ -256,7 +266,7 @@ __global__ void __launch_bounds__(S::T, 1)
 // SUB: the sub-block products of a larger polymul: the global passes have left
 // their words of a in c and of b in scratch (b_ntt: NTT(b) whole in b).
 template <int LOGC, class S, bool LIFT, bool SUB = false>
-__global__ void __launch_bounds__(S::T, 1)
+__global__ void __launch_bounds__(S::T, cluster_blocks<S>())
     k_polymul_cluster(const vkcu_poly_job* __restrict__ jobs, int njobs, vkcu_poly_job one, int sub_log,
                       const __grid_constant__ vkcu_lift lift) {
   using K = Cols<LOGC, S>;
@@ -383,22 +393,26 @@ using Small12 = Shape<12, 16, 1, M>;
 template <class M>
 using Small13 = Shape<13, 32, 1, M>;
 
-// logc: cluster size 2^logc; logs: sub-block size 2^logs (14, or 9 .. 13
-// with logc = 3, or 10 .. 12 with logc = 4: n = 2^14 .. 2^16 on 16 CTAs, a
-// cluster size the GPU allows on request).
+// logc: cluster size 2^logc; logs: sub-block size 2^logs: 14, or, for fewer
+// jobs than SMs, 9 .. 13 with logc = 3, 12 / 13 with logc = 1 or 2 (n = 2^13,
+// 2^14), 10 .. 12 with logc = 4 (n = 2^14 .. 2^16 on 16 CTAs, a cluster size
+// the GPU allows on request).
 #define VK_CLUSTER_SHAPES(X)                                 \
   switch (logc * 32 + logs) {                                \
-    case 1 * 32 + 14: return X(1, SubShape<M>);                 \
-    case 2 * 32 + 14: return X(2, SubShape<M>);                 \
-    case 3 * 32 + 14: return X(3, SubShape<M>);                 \
-    case 3 * 32 + 9: return X(3, Small9<M>);                    \
-    case 3 * 32 + 10: return X(3, Small10<M>);                  \
-    case 3 * 32 + 11: return X(3, Small11<M>);                  \
-    case 3 * 32 + 12: return X(3, Small12<M>);                  \
-    case 3 * 32 + 13: return X(3, Small13<M>);                  \
-    case 4 * 32 + 10: return X(4, Small10<M>);                  \
-    case 4 * 32 + 11: return X(4, Small11<M>);                  \
-    case 4 * 32 + 12: return X(4, Small12<M>);                  \
+    case 1 * 32 + 14: return X(1, SubShape<M>);              \
+    case 2 * 32 + 14: return X(2, SubShape<M>);              \
+    case 3 * 32 + 14: return X(3, SubShape<M>);              \
+    case 3 * 32 + 9: return X(3, Small9<M>);                 \
+    case 1 * 32 + 12: return X(1, Small12<M>);               \
+    case 1 * 32 + 13: return X(1, Small13<M>);               \
+    case 2 * 32 + 12: return X(2, Small12<M>);               \
+    case 3 * 32 + 10: return X(3, Small10<M>);               \
+    case 3 * 32 + 11: return X(3, Small11<M>);               \
+    case 3 * 32 + 12: return X(3, Small12<M>);               \
+    case 3 * 32 + 13: return X(3, Small13<M>);               \
+    case 4 * 32 + 10: return X(4, Small10<M>);               \
+    case 4 * 32 + 11: return X(4, Small11<M>);               \
+    case 4 * 32 + 12: return X(4, Small12<M>);               \
     default: return (int)cudaErrorInvalidValue;              \
   }
 

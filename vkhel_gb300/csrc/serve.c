@@ -237,7 +237,7 @@ static int issue_chunk(struct vkhel_server *s, struct srv_slot *sl, uint32_t c, 
 	if (!e) /* a whole micro-batch: its classes on concurrent streams when tuned so */
 		e = s->forked && nchunks == 1 && nclasses <= SRV_AUX + 1
 				? vkh_issue_classes_forked(cs, s->aux, s->fork, s->join, ctx->sms, dpoly, dntt, classes, nclasses, NULL)
-				: vkh_issue_classes(cs, ctx->sms, dpoly, dntt, classes, nclasses, NULL);
+				: vkh_issue_classes(cs, ctx->sms, ctx->sms, dpoly, dntt, classes, nclasses, NULL);
 	if (!e)
 		e = vkcu_event_record(sl->ev_comp[c], cs);
 	if (!e)
@@ -400,7 +400,7 @@ static int upload_operand(struct vkhel_server *s, struct srv_operand *op) {
 			break;
 		uint64_t *p = (uint64_t *) op->dev + (uint64_t) k * op->n;
 		const vkcu_ntt_job j = {p, p, d->dev_set};
-		e = vkcu_ntt_forward(s->s_in, NULL, 1, &j, op->log_n, vkcu_qclass(op->tables[k]->q), ctx->sms);
+		e = vkcu_ntt_forward(s->s_in, NULL, 1, &j, op->log_n, vkcu_qclass(op->tables[k]->q), ctx->sms, ctx->sms);
 	}
 	const int se = vkcu_sync(s->s_in);
 	if (!e)
