@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 LIFT = [("elemmod", 65537, 0)]
 # on 152 SMs: the last count of each choice and the first of the next, then
 # counts past one or two rounds of one job per SM (2^14, 2^13) or SM pair (2^15)
-COUNTS = [(12, 19), (12, 20), (13, 38), (13, 39), (13, 76), (13, 77), (13, 160),
+COUNTS = [(12, 19), (12, 20), (13, 30), (13, 31), (13, 76), (13, 77), (13, 160),
           (14, 30), (14, 31), (14, 60), (14, 61), (14, 76), (14, 77), (14, 153), (14, 182), (14, 212), (14, 228),
           (14, 256), (14, 259), (14, 304), (15, 50), (15, 51), (15, 77), (15, 121), (15, 122), (15, 153),
           (16, 19), (16, 20)]

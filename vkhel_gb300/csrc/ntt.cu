@@ -295,17 +295,18 @@ static bool jobs_aligned(const vkcu_ntt_job* jobs, const vkcu_ntt_job* one) {
 // at the same time.  Tuning entry (3, 1) = 1 turns the split off, (3, 3) = 1
 // keeps single calls on 8.  The lines, from products timed per job count and
 // split on 152 SMs (us; the kernel without a split / on 2 / 4 / 8 CTAs a job):
-//   2^13: 30 jobs 33 / 25 / 21 / 21, 60: 33 / 25 / 25 / 25, 76: 33 / 25 / 41 / 41,
+//   2^13: 30 jobs 33 / 25 / 21 / 18, 38: 33 / 25 / 25 / 29, 76: 33 / 25 / 41 / 41,
 //         100: 33 / 37 / 43 / 43
 //   2^14: 30 jobs 64 / 45 / 27 / 27, 50: 66 / 45 / 40 / 45, 76: 66 / 47 / 57 / 67,
 //         100: 66 / 70 / 57 / 72
 //   2^15: (2 / 4 / 8) 19 jobs 70 / 47 / 41, 50: 72 / 75 / 62, 60: 72 / 76 / 88
 //   2^16: (4 / 8) 19 jobs 78 / 78, 24: 78 / 86
 static int split_log(long njobs, uint32_t log_n, long avail, bool single) {
-  if (log_n < 12 || log_n > 16 || vkh_variant(3, 1) != 0) return 0;
+  if (log_n < 12 || log_n > 17 || vkh_variant(3, 1) != 0) return 0;
   if (single && log_n >= 14 && njobs * 16 <= avail && vkh_variant(3, 3) == 0) return 4;
+  if (log_n == 17) return 0;  // 8 CTAs in any case
   switch (log_n) {
-    case 13: return njobs * 4 <= avail ? 3 : njobs * 2 <= avail ? 1 : 0;
+    case 13: return njobs * 5 <= avail ? 3 : njobs * 2 <= avail ? 1 : 0;
     case 14: return njobs * 5 <= avail ? 3 : njobs * 5 <= 2 * avail ? 2 : njobs * 2 <= avail ? 1 : 0;
     case 15: return njobs * 3 <= avail ? 3 : 0;
     default: return njobs * 8 <= avail ? 3 : 0;

@@ -50,16 +50,18 @@ using SubShape = Shape<14, 32, 1, M>;  // the large-n sub-block
 template <int LOGC, class S>
 struct Cols {
   static constexpr int C = 1 << LOGC, SUB = S::N;
-  static constexpr bool MERGED = LOGC + S::FIRSTK <= 4;
+  static constexpr bool MERGED = S::R == 4 && LOGC + S::FIRSTK <= 4;
   static constexpr int LJ = MERGED ? S::FIRSTK : 0;
   static constexpr int KK = LOGC + LJ, W = 1 << KK;
   static constexpr int TM = SUB >> LJ;
   static constexpr int COLS = TM >> LOGC;   // groups per CTA
-  static constexpr int PER = COLS / S::T;   // groups per thread
-  static constexpr int H = PER >= 2 ? PER / 2 : 1;  // of them in flight at once
+  static constexpr int PER = COLS >= S::T ? COLS / S::T : 1;  // groups per thread
+  static constexpr int H = PER >= 2 ? PER / 2 : 1;            // of them in flight at once
   static constexpr int N16 = C * SUB / 16;  // groups of the last four stages
-  static_assert(PER * W == S::E, "a column pass moves E words per thread");
+  static_assert(COLS >= S::T ? PER * W == S::E : COLS % 32 == 0, "whole warps move the columns");
   static_assert(W <= S::T, "a thread per slice prefetches");
+  // with fewer columns than threads (radix-4 shapes) the first warps have one each
+  __device__ __forceinline__ static bool active() { return COLS >= S::T || (int)threadIdx.x < COLS; }
   __device__ __forceinline__ static int col(int rank, int k) { return rank * COLS + (int)threadIdx.x + k * S::T; }
   // word j of column c: its CTA (static) and its place there
   static constexpr int cta(int j) { return j >> LJ; }
@@ -89,9 +91,7 @@ template <int LOGC, class S, bool SPLIT, bool SUB = false>
 __device__ __forceinline__ void col_fwd(const u64* __restrict__ in, u64* sm, const cg::cluster_group& cl, int rank,
                                         const Tw& t, int rbase = 0, u32 base = 1u) {
   using K = Cols<LOGC, S>;
-#pragma unroll 1
-  for (int k0 = 0; k0 < K::PER; k0 += K::H) {
-    u64 v[K::H * K::W];
+  auto load = [&](u64(&v)[K::H * K::W], int k0) {
 #pragma unroll
     for (int k = 0; k < K::H; k++)
 #pragma unroll
@@ -100,13 +100,28 @@ __device__ __forceinline__ void col_fwd(const u64* __restrict__ in, u64* sm, con
       constexpr int k = decltype(kc)::value;
       ct_first_group<typename S::M, K::KK, k * K::W, !SUB>(v, RowTw{t.fwd, base}, t);
     });
-    if (SPLIT && k0 == 0) cluster_wait();
+  };
+  auto scatter = [&](const u64(&v)[K::H * K::W], int k0) {
 #pragma unroll
     for (int j = 0; j < K::W; j++) {
       u64* rem = cl.map_shared_rank(sm, rbase + K::cta(j));
 #pragma unroll
       for (int k = 0; k < K::H; k++) rem[K::local(K::col(rank, k0 + k), j)] = v[k * K::W + j];
     }
+  };
+  if constexpr (K::COLS >= S::T) {
+#pragma unroll 1
+    for (int k0 = 0; k0 < K::PER; k0 += K::H) {
+      u64 v[K::H * K::W];
+      load(v, k0);
+      if (SPLIT && k0 == 0) cluster_wait();
+      scatter(v, k0);
+    }
+  } else {
+    u64 v[K::H * K::W];
+    if (K::active()) load(v, 0);
+    if (SPLIT) cluster_wait();  // every thread's
+    if (K::active()) scatter(v, 0);
   }
 }
 
@@ -117,6 +132,7 @@ template <int LOGC, class S, bool SUB, class Epi>
 __device__ __forceinline__ void col_inv(u64* __restrict__ out, u64* sm, const cg::cluster_group& cl, int rank,
                                         const Tw& t, const Epi& epi, int rbase = 0, u32 base = 1u) {
   using K = Cols<LOGC, S>;
+  if (!K::active()) return;
 #pragma unroll 1
   for (int k0 = 0; k0 < K::PER; k0 += K::H) {
     u64 v[K::H * K::W];
@@ -147,9 +163,10 @@ __device__ __forceinline__ void sub_fwd(u64* sm, const cg::cluster_group& cl, co
   if constexpr (!Cols<LOGC, S>::MERGED) fwd_first_smem<S>(sm, t, tw_mult);
 }
 
-template <int LOGC, class S>
-__device__ __forceinline__ void sub_inv(u64* sm, const cg::cluster_group& cl, const Tw& t, u32 tw_mult) {
-  inv_passes<S>(sm, t, tw_mult, S::HEAD - 4);
+template <int LOGC, class S, class L>
+__device__ __forceinline__ void sub_inv(u64* sm, const cg::cluster_group& cl, const Tw& t, u32 tw_mult,
+                                        const L& last_inv) {
+  inv_passes<S>(sm, t, tw_mult, last_inv);
   if constexpr (!Cols<LOGC, S>::MERGED) {
     __syncthreads();
     inv_last_smem<S>(sm, t, tw_mult);
@@ -220,11 +237,11 @@ __global__ void __launch_bounds__(S::T, cluster_blocks<S>())
     col_fwd<LOGC, S, false, SUB>(in, sm, cl, rank, t, 0, it.base);
     sub_fwd<LOGC, S>(sm, cl, t, tw_mult);
     out += (size_t)rank * K::SUB;
-    fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
+    fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[S::W]) {
       const typename S::M::Out to(t);
 #pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = to.canon(v[j]);
-      store16(v, out + 16 * g);
+      for (int j = 0; j < S::W; j++) v[j] = to.canon(v[j]);
+      store_group(v, out + S::W * g);
     });
   }
   cl.sync();
@@ -249,15 +266,15 @@ __global__ void __launch_bounds__(S::T, cluster_blocks<S>())
     const u64* in = reinterpret_cast<const u64*>(job.in) + it.off + (size_t)rank * K::SUB;
     cl.sync();
 #pragma unroll 1
-    for (int i = 0; i < S::E / 16; i++) {
+    for (int i = 0; i < S::GROUPS; i++) {
       const int g = S::group(i);
-      u64 v[16];
-      load16(v, in + 16 * g);
-      gs_group<typename S::M, 4, 0, true, false>(v, last.at(g), t);
+      u64 v[S::W];
+      load_group(v, in + S::W * g);
+      gs_group<typename S::M, S::R, 0, true, false>(v, last.template at<4 - S::R>(g), t);
 #pragma unroll
-      for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
+      for (int j = 0; j < S::W; j++) sm[pad(S::W * g) + j] = v[j];
     }
-    sub_inv<LOGC, S>(sm, cl, t, it.tw_mult(rank));
+    sub_inv<LOGC, S>(sm, cl, t, it.tw_mult(rank), last);
     col_inv_out<LOGC, S, LIFT, SUB>(reinterpret_cast<u64*>(job.out) + it.off, sm, cl, rank, t, &lift, 0, it.base);
   }
   cl.sync();
@@ -297,28 +314,28 @@ __global__ void __launch_bounds__(S::T, cluster_blocks<S>())
       cluster_arrive();  // done with every shared memory the column pass writes (col_fwd waits)
       col_fwd<LOGC, S, true, SUB>(ph ? a : b, sm, cl, rank, t, 0, it.base);
       sub_fwd<LOGC, S>(sm, cl, t, tw_mult);
-      fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
+      fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[S::W]) {
         using M = typename S::M;
         if (ph == 0) {
           const typename M::Out to(t);
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
-          park16(v, scratch, g, S::N / 16);
+          for (int j = 0; j < S::W; j++) v[j] = to.park(v[j]);
+          park_group(v, scratch, g, S::N / S::W);
         } else {
-          u64 bh[16];
+          u64 bh[S::W];
           if (b_ntt) {
-            load16(bh, b + (size_t)rank * K::SUB + 16 * g);
-            reduce_operand16(bh, t);
+            load_group(bh, b + (size_t)rank * K::SUB + S::W * g);
+            reduce_operands(bh, t);
           } else {
-            unpark16(bh, scratch, g, S::N / 16);
+            unpark_group(bh, scratch, g, S::N / S::W);
           }
           const typename M::Product product(t);
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
+          for (int j = 0; j < S::W; j++) v[j] = product(v[j], bh[j]);
           // the sub-block's first inverse pass (stages HEAD + 3 .. HEAD) on the same words
-          gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.at(g), t);
+          gs_group<M, S::R, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.template at<4 - S::R>(g), t);
 #pragma unroll
-          for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
+          for (int j = 0; j < S::W; j++) sm[pad(S::W * g) + j] = v[j];
         }
       });
     }
@@ -329,7 +346,7 @@ __global__ void __launch_bounds__(S::T, cluster_blocks<S>())
                                                      : (size_t)threadIdx.x * K::TM + rank * K::COLS;
       prefetch_l2(reinterpret_cast<const u64*>(nx.b) + off, kSlice);
     }
-    sub_inv<LOGC, S>(sm, cl, t, tw_mult);
+    sub_inv<LOGC, S>(sm, cl, t, tw_mult, last_inv);
     col_inv_out<LOGC, S, LIFT, SUB>(reinterpret_cast<u64*>(job.c) + it.off, sm, cl, rank, t, &lift, 0, it.base);
   }
   cl.sync();
@@ -380,12 +397,13 @@ static int launch_cluster(cudaStream_t st, int njobs, Args... args) {
   return (int)e;
 }
 
-// Sub-blocks of 2^9 .. 2^13 words for n = 2^12 .. 2^16 on 8 CTAs (16 words
-// per thread; 32 at 2^13, so that 256 threads fit the register file).
+// Sub-blocks of 2^9 .. 2^13 words for n = 2^12 .. 2^16 on 8 CTAs: 4 words per
+// thread and radix-4 passes to 2^10, 16 words per thread above (32 at 2^13, so
+// that 256 threads fit the register file).
 template <class M>
-using Small9 = Shape<9, 16, 1, M>;
+using Small9 = Shape<9, 4, 1, M, false, 2>;
 template <class M>
-using Small10 = Shape<10, 16, 1, M>;
+using Small10 = Shape<10, 4, 1, M, false, 2>;
 template <class M>
 using Small11 = Shape<11, 16, 1, M>;
 template <class M>
@@ -395,7 +413,7 @@ using Small13 = Shape<13, 32, 1, M>;
 
 // logc: cluster size 2^logc; logs: sub-block size 2^logs: 14, or, for fewer
 // jobs than SMs, 9 .. 13 with logc = 3, 12 / 13 with logc = 1 or 2 (n = 2^13,
-// 2^14), 10 .. 12 with logc = 4 (n = 2^14 .. 2^16 on 16 CTAs, a cluster size
+// 2^14), 10 .. 13 with logc = 4 (n = 2^14 .. 2^17 on 16 CTAs, a cluster size
 // the GPU allows on request).
 #define VK_CLUSTER_SHAPES(X)                                 \
   switch (logc * 32 + logs) {                                \
@@ -412,6 +430,7 @@ using Small13 = Shape<13, 32, 1, M>;
     case 3 * 32 + 13: return X(3, Small13<M>);               \
     case 4 * 32 + 10: return X(4, Small10<M>);               \
     case 4 * 32 + 11: return X(4, Small11<M>);               \
+    case 4 * 32 + 13: return X(4, Small13<M>);               \
     case 4 * 32 + 12: return X(4, Small12<M>);               \
     default: return (int)cudaErrorInvalidValue;              \
   }

@@ -137,11 +137,12 @@ __device__ __forceinline__ Tw load_tw_product(const vkcu_twset* p) {
 
 // A caller-supplied NTT(b) operand reduced as the reference's elemmul reduces
 // its operands (reduce64, elemmul.comp:36-47): canonical words pass through.
-__device__ __forceinline__ void reduce_operand16(u64 (&v)[16], const Tw& t) {
+template <int K>
+__device__ __forceinline__ void reduce_operands(u64 (&v)[K], const Tw& t) {
   const u64 mu = t.mu();
   const u32 qbits = t.qbits();
 #pragma unroll
-  for (int j = 0; j < 16; j++) v[j] = ref_reduce64_maybe(v[j], t.q, mu, qbits);
+  for (int j = 0; j < K; j++) v[j] = ref_reduce64_maybe(v[j], t.q, mu, qbits);
 }
 
 // ---------------------------------------------------------------------------
@@ -440,25 +441,28 @@ struct RowTw {
 // The roots of the last four stages, from the table's rows (vkcu_tw_slot): a
 // warp's 32 groups read 32 neighbouring entries, 4 wavefronts a load instead
 // of up to 32.  N16 = n/16 for the whole transform, 0 where it is known at run
-// time only.
-template <int N16>
+// time only.  A pass from the V-th of these stages on: p its group's column,
+// x its block within the 16 words.
+template <int N16, int V>
 struct LastTw {
-  const ulonglong2* p;  // the group's column
-  u32 n16;
+  const ulonglong2* p;
+  u32 n16, x;
   __device__ __forceinline__ ulonglong2 operator()(int u, int r) const {
-    return ld_tw(p + ((1u << u) + (u32)r) * (N16 ? (u32)N16 : n16));
+    return ld_tw(p + ((1u << (V + u)) + (V ? x << u : 0u) + (u32)r) * (N16 ? (u32)N16 : n16));
   }
 };
-// Those of a sub-block: at(g) for its group g.
+// Those of a sub-block: at<V>(b) for block b (within it) of the V-th stage.
 template <int N16>
 struct LastTable {
   const ulonglong2* p;  // the sub-block's first column
   u32 n16;
   __device__ __forceinline__ LastTable(const ulonglong2* table, int first_group, u32 n16_)
       : p(table + first_group), n16(n16_) {}
-  __device__ __forceinline__ LastTw<N16> at(int g) const { return LastTw<N16>{p + g, n16}; }
+  template <int V>
+  __device__ __forceinline__ LastTw<N16, V> at(int b) const {
+    return LastTw<N16, V>{p + (b >> V), n16, (u32)b & ((1u << V) - 1)};
+  }
 };
-
 template <class M, int KK, int U0, int G0, int NV, class R>
 __device__ __forceinline__ void ct_group(u64 (&v)[NV], const R& tw, const Tw& t) {
   static_for<U0, KK>([&](auto uc) {
@@ -554,19 +558,31 @@ __device__ __forceinline__ void gs_group(u64 (&v)[NV], const R& tw, const Tw& t)
 // a direction share one loop body (the stage offset is a runtime value), and
 // the fused polymul runs its two forward transforms through the same code.
 
-template <int LOGN_, int E_, int U_ = 1, class M_ = Mod60, bool DUAL_ = false>
+// R: stages of a pass (radix 2^R groups of W words).  4 everywhere but in the
+// small sub-blocks of single calls, which run radix-4 passes with 4 words per
+// thread: a radix-16 group is 32 butterflies one after another in one thread
+// (about 1200 cycles of its SM sub-partition's multiplier), and with 16 words
+// per thread a 2^9- or 2^10-word sub-block is one or two warps, so that half or
+// more of the SM's four sub-partitions had nothing to do: one product of 2^12
+// words 24.5 -> 19.5 us a call, of 2^13 26 -> 21.4, of 2^14 27.5 -> 24.4 (10 us
+// of a call are its launch and wait).  With 16 warps the radix-16 passes win:
+// 2^11-word sub-blocks, 25 products of 2^14 27 us against 37.
+template <int LOGN_, int E_, int U_ = 1, class M_ = Mod60, bool DUAL_ = false, int R_ = 4>
 struct Shape {
   using M = M_;  // modulus class
+  static constexpr int R = R_, W = 1 << R_;
   // DUAL: the CTA holds 2 T threads running two transforms of this shape in
   // step, thread t on the one of half t / T (shared barriers, separate words)
   static constexpr bool DUAL = DUAL_;
   static constexpr int LOGN = LOGN_, E = E_;
-  static constexpr int U = U_;  // radix-16 groups of a thread in flight at once (1 or 2)
+  static constexpr int U = U_;  // groups of a thread in flight at once (1 or 2)
   static constexpr int N = 1 << LOGN, T = N / E;
-  static constexpr int HEAD = LOGN - 4;  // first stage of the last pass
-  static constexpr int FIRSTK = HEAD % 4 == 0 ? 4 : HEAD % 4;
+  static constexpr int HEAD = LOGN - R;  // first stage of the last pass
+  static constexpr int FIRSTK = HEAD % R == 0 ? R : HEAD % R;
+  static constexpr int GROUPS = E >> R;  // of a thread in a pass
   static constexpr int SMEM_BYTES = (N + N / 16) * 8;
-  static_assert(E >= 16 && (E % 16) == 0 && HEAD >= 1 && T >= 1, "unsupported shape");
+  static_assert((R == 4 || R == 2) && GROUPS >= 1 && (E % W) == 0 && HEAD >= FIRSTK + (R == 2 ? 2 : 0) && T >= 1,
+                "unsupported shape");
   // this thread's index within its transform
   __device__ __forceinline__ static int tid() { return DUAL ? (int)(threadIdx.x & (T - 1)) : (int)threadIdx.x; }
   // its i-th group in the radix-16 passes: a warp's groups are consecutive, so
@@ -574,7 +590,7 @@ struct Shape {
   // threads in every such pass
   __device__ __forceinline__ static int group(int i) {
     const int t = tid();
-    return (t >> 5) * (2 * E) + (t & 31) + 32 * i;
+    return (t >> 5) * (32 * GROUPS) + (t & 31) + 32 * i;
   }
   // Barrier of the threads that share this thread's block of 2^lb words.  A
   // pass mixes words inside its blocks only, so a CTA-wide barrier is needed
@@ -587,24 +603,28 @@ struct Shape {
   __device__ __forceinline__ static void sync_block(int lb) {
     if ((1 << lb) <= 32 * E) {
       __syncwarp(T < 32 ? (1u << (T & 31)) - 1u : 0xffffffffu);
-    } else if ((1 << lb) == N) {
-      __syncthreads();
     } else {
+      // parts of the CTA: barriers k .. 2k - 1 for k parts, so that no barrier
+      // serves blocks of two sizes (15 is the last there is)
       static_assert(!DUAL || N <= 32 * E * 16, "a part of half a CTA");
-      const int threads = (1 << lb) / E;
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + tid() / threads), "r"(threads) : "memory");
+      const int threads = (1 << lb) / E, parts = T / threads;
+      if (parts == 1 || parts > 8)
+        __syncthreads();
+      else
+        asm volatile("bar.sync %0, %1;" ::"r"(parts + tid() / threads), "r"(threads) : "memory");
     }
   }
 };
 
-// A radix-16 pass starting at stage s0 of an n = 2^logn transform: group g
+// A radix-2^R pass starting at stage s0 of an n = 2^LOGN transform: group g
 // has block g >> lt (lt = log2 t_min), first word (g >> lt) << lb | (g & mask)
 // with lb = log2(n >> s0), words at stride t_min, twiddle base tw0 + block.
-struct Pass16 {
+template <class S>
+struct Pass {
   int lt, lb;
   u32 tw0;
-  __device__ __forceinline__ Pass16(int logn, int s0, u32 tw_mult)
-      : lt(logn - s0 - 4), lb(logn - s0), tw0(tw_mult << s0) {}
+  __device__ __forceinline__ Pass(int s0, u32 tw_mult)
+      : lt(S::LOGN - s0 - S::R), lb(S::LOGN - s0), tw0(tw_mult << s0) {}
   __device__ __forceinline__ int first(int g) const { return ((g >> lt) << lb) | (g & ((1 << lt) - 1)); }
   __device__ __forceinline__ u32 base(int g) const { return tw0 + (u32)(g >> lt); }
 };
@@ -672,59 +692,77 @@ __device__ __forceinline__ void fwd_first_smem(u64* sm, const Tw& t, u32 tw_mult
   __syncthreads();
 }
 
-// Radix-16 forward passes s0 = FIRSTK, FIRSTK + 4, ..., HEAD on shared
-// memory.  The last pass hands each group (words 16g .. 16g+15) to epi(g, v)
-// instead of storing it back.  No barrier at the end.
+// Forward passes s0 = FIRSTK, FIRSTK + R, ..., HEAD on shared memory.  The
+// last pass hands each group (words W g .. W g + W - 1) to epi(g, v) instead
+// of storing it back.  No barrier at the end.
+template <class S, class Tws>
+__device__ __forceinline__ void fwd_pass(u64* sm, const Tw& t, const Pass<S>& ps, const Tws& tws) {
+  const int st = 1 << ps.lt;
+#pragma unroll(S::U)
+  for (int i = 0; i < S::GROUPS; i++) {
+    const int g = S::group(i);
+    const int a0 = ps.first(g);
+    u64 v[S::W];
+#pragma unroll
+    for (int j = 0; j < S::W; j++) v[j] = sm[pad(a0 + j * st)];
+    ct_group<typename S::M, S::R, 0, 0>(v, tws(g), t);
+#pragma unroll
+    for (int j = 0; j < S::W; j++) sm[pad(a0 + j * st)] = v[j];
+  }
+  S::sync_block(ps.lb);
+}
+
 template <class S, class L, class Epi>
 __device__ __forceinline__ void fwd_passes(u64* sm, const Tw& t, u32 tw_mult, const L& last, Epi&& epi) {
+  // radix 4: the pass before the last is one of the last four stages too
+  constexpr int ROWS = S::R == 4 ? S::HEAD : S::HEAD - 2;
 #pragma unroll 1
-  for (int s0 = S::FIRSTK; s0 < S::HEAD; s0 += 4) {
-    const Pass16 ps(S::LOGN, s0, tw_mult);
-    const int st = 1 << ps.lt;
-#pragma unroll(S::U)
-    for (int i = 0; i < S::E / 16; i++) {
-      const int g = S::group(i);
-      const int a0 = ps.first(g);
-      u64 v[16];
-#pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = sm[pad(a0 + j * st)];
-      ct_group<typename S::M, 4, 0, 0>(v, RowTw{t.fwd, ps.base(g)}, t);
-#pragma unroll
-      for (int j = 0; j < 16; j++) sm[pad(a0 + j * st)] = v[j];
-    }
-    S::sync_block(ps.lb);
+  for (int s0 = S::FIRSTK; s0 < ROWS; s0 += S::R) {
+    const Pass<S> ps(s0, tw_mult);
+    fwd_pass<S>(sm, t, ps, [&](int g) { return RowTw{t.fwd, ps.base(g)}; });
   }
+  if constexpr (S::R == 2)
+    fwd_pass<S>(sm, t, Pass<S>(ROWS, tw_mult), [&](int g) { return last.template at<0>(g >> 2); });
 #pragma unroll(S::U)
-  for (int i = 0; i < S::E / 16; i++) {
+  for (int i = 0; i < S::GROUPS; i++) {
     const int g = S::group(i);
-    u64 v[16];
+    u64 v[S::W];
 #pragma unroll
-    for (int j = 0; j < 16; j++) v[j] = sm[17 * g + j];  // pad(16 g + j)
-    ct_group<typename S::M, 4, 0, 0>(v, last.at(g), t);
+    for (int j = 0; j < S::W; j++) v[j] = sm[pad(S::W * g) + j];
+    ct_group<typename S::M, S::R, 0, 0>(v, last.template at<4 - S::R>(g), t);
     epi(g, v);
   }
 }
 
-// Radix-16 inverse passes s0 = s_top, s_top - 4, ..., FIRSTK on shared
-// memory, each preceded by a barrier of its blocks; no barrier at the end.
-template <class S>
-__device__ __forceinline__ void inv_passes(u64* sm, const Tw& t, u32 tw_mult, int s_top) {
-#pragma unroll 1
-  for (int s0 = s_top; s0 >= S::FIRSTK; s0 -= 4) {
-    const Pass16 ps(S::LOGN, s0, tw_mult);
-    const int st = 1 << ps.lt;
-    S::sync_block(ps.lb);
+// Inverse passes s0 = HEAD - R, ..., FIRSTK on shared memory (the one at HEAD
+// is the caller's), each preceded by a barrier of its blocks; no barrier at
+// the end.
+template <class S, class Tws>
+__device__ __forceinline__ void inv_pass(u64* sm, const Tw& t, const Pass<S>& ps, const Tws& tws) {
+  const int st = 1 << ps.lt;
+  S::sync_block(ps.lb);
 #pragma unroll(S::U)
-    for (int i = 0; i < S::E / 16; i++) {
-      const int g = S::group(i);
-      const int a0 = ps.first(g);
-      u64 v[16];
+  for (int i = 0; i < S::GROUPS; i++) {
+    const int g = S::group(i);
+    const int a0 = ps.first(g);
+    u64 v[S::W];
 #pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = sm[pad(a0 + j * st)];
-      gs_group<typename S::M, 4, 0, false, false>(v, RowTw{t.inv, ps.base(g)}, t);
+    for (int j = 0; j < S::W; j++) v[j] = sm[pad(a0 + j * st)];
+    gs_group<typename S::M, S::R, 0, false, false>(v, tws(g), t);
 #pragma unroll
-      for (int j = 0; j < 16; j++) sm[pad(a0 + j * st)] = v[j];
-    }
+    for (int j = 0; j < S::W; j++) sm[pad(a0 + j * st)] = v[j];
+  }
+}
+
+template <class S, class L>
+__device__ __forceinline__ void inv_passes(u64* sm, const Tw& t, u32 tw_mult, const L& last_inv) {
+  constexpr int ROWS = S::R == 4 ? S::HEAD : S::HEAD - 2;
+  if constexpr (S::R == 2)
+    inv_pass<S>(sm, t, Pass<S>(ROWS, tw_mult), [&](int g) { return last_inv.template at<0>(g >> 2); });
+#pragma unroll 1
+  for (int s0 = ROWS - S::R; s0 >= S::FIRSTK; s0 -= S::R) {
+    const Pass<S> ps(s0, tw_mult);
+    inv_pass<S>(sm, t, ps, [&](int g) { return RowTw{t.inv, ps.base(g)}; });
   }
 }
 
@@ -886,30 +924,34 @@ __device__ __forceinline__ void inv_last(u64* sm, const Tw& t, u32 tw_mult, u64*
     inv_last_epi<S>(sm, t, tw_mult, out, fold, NoLift{});
 }
 
-// Register groups of 16 consecutive words <-> global memory (32-byte vectors).
-__device__ __forceinline__ void load16(u64 (&v)[16], const u64* p) {
+// Register groups of K consecutive words <-> global memory (32-byte vectors).
+template <int K>
+__device__ __forceinline__ void load_group(u64 (&v)[K], const u64* p) {
 #pragma unroll
-  for (int h = 0; h < 4; h++) ld4(p + 4 * h, v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+  for (int h = 0; h < K / 4; h++) ld4(p + 4 * h, v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
 }
 
-__device__ __forceinline__ void store16(const u64 (&v)[16], u64* p) {
+template <int K>
+__device__ __forceinline__ void store_group(const u64 (&v)[K], u64* p) {
 #pragma unroll
-  for (int h = 0; h < 4; h++) st4(p + 4 * h, v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+  for (int h = 0; h < K / 4; h++) st4(p + 4 * h, v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
 }
 
 // NTT(b) parked between the phases of a fused product: 16-byte pairs, pair jj
 // of group g (of G) at jj G + g, so that a warp moves whole lines (each thread
 // reads back what it wrote).
-__device__ __forceinline__ void park16(const u64 (&v)[16], u64* p, int g, int G) {
+template <int K>
+__device__ __forceinline__ void park_group(const u64 (&v)[K], u64* p, int g, int G) {
 #pragma unroll
-  for (int jj = 0; jj < 8; jj++)
+  for (int jj = 0; jj < K / 2; jj++)
     asm volatile("st.global.v2.u64 [%0], {%1,%2};" ::"l"(p + 2 * (jj * G + g)), "l"(v[2 * jj]), "l"(v[2 * jj + 1])
                  : "memory");
 }
 
-__device__ __forceinline__ void unpark16(u64 (&v)[16], const u64* p, int g, int G) {
+template <int K>
+__device__ __forceinline__ void unpark_group(u64 (&v)[K], const u64* p, int g, int G) {
 #pragma unroll
-  for (int jj = 0; jj < 8; jj++)
+  for (int jj = 0; jj < K / 2; jj++)
     asm volatile("ld.global.v2.u64 {%0,%1}, [%2];"
                  : "=l"(v[2 * jj]), "=l"(v[2 * jj + 1])
                  : "l"(p + 2 * (jj * G + g)));
@@ -970,7 +1012,7 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
       const typename M::Out to(t);
 #pragma unroll
       for (int j = 0; j < 16; j++) v[j] = to.canon(v[j]);
-      store16(v, out + 16 * g);
+      store_group(v, out + 16 * g);
     });
   }
 }
@@ -1008,13 +1050,13 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     for (int i = 0; i < S::E / 16; i++) {
       const int g = S::group(i);
       u64 v[16];
-      load16(v, in + 16 * g);
-      gs_group<M, 4, 0, true, false>(v, last.at(g), t);
+      load_group(v, in + 16 * g);
+      gs_group<M, 4, 0, true, false>(v, last.template at<0>(g), t);
       if (i == 0) __syncthreads();  // the last job's words are read
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
     }
-    inv_passes<S>(sm, t, tw_mult, S::HEAD - 4);
+    inv_passes<S>(sm, t, tw_mult, last);
     __syncthreads();
     inv_last<S, LIFT>(sm, t, tw_mult, out, sub_log == 0, &lift);
   }
@@ -1054,26 +1096,26 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
           const typename M::Out to(t);
 #pragma unroll
           for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
-          park16(v, scratch, g, S::N / 16);
+          park_group(v, scratch, g, S::N / 16);
         } else {
           u64 bh[16];
           if (b_ntt) {
-            load16(bh, reinterpret_cast<const u64*>(job.b) + 16 * g);
-            reduce_operand16(bh, t);
+            load_group(bh, reinterpret_cast<const u64*>(job.b) + 16 * g);
+            reduce_operands(bh, t);
           } else {
-            unpark16(bh, scratch, g, S::N / 16);
+            unpark_group(bh, scratch, g, S::N / 16);
           }
           const typename M::Product product(t);
 #pragma unroll
           for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
           // the first inverse pass (stages HEAD + 3 .. HEAD) on the same 16 words
-          gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.at(g), t);
+          gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.template at<0>(g), t);
 #pragma unroll
           for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
         }
       });
     }
-    inv_passes<S>(sm, t, 1u, S::HEAD - 4);
+    inv_passes<S>(sm, t, 1u, last_inv);
     __syncthreads();
     inv_last<S, LIFT>(sm, t, 1u, reinterpret_cast<u64*>(job.c), true, &lift);
   }

@@ -45,20 +45,20 @@ __device__ __noinline__ void ragged_cta_product(u64* sm, const vkcu_poly_job& jo
         const typename M::Out to(t);
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
-        park16(v, scratch, g, S::N / 16);
+        park_group(v, scratch, g, S::N / 16);
       } else {
         u64 bh[16];
-        unpark16(bh, scratch, g, S::N / 16);
+        unpark_group(bh, scratch, g, S::N / 16);
         const typename M::Product product(t);
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
-        gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.at(g), t);
+        gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.template at<0>(g), t);
 #pragma unroll
         for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
       }
     });
   }
-  inv_passes<S>(sm, t, 1u, S::HEAD - 4);
+  inv_passes<S>(sm, t, 1u, last_inv);
   __syncthreads();
   inv_last<S>(sm, t, 1u, reinterpret_cast<u64*>(job.c), true);
   __syncthreads();
@@ -86,20 +86,20 @@ __device__ __noinline__ void ragged_cluster_product(u64* sm, const cg::cluster_g
         const typename M::Out to(t);
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = to.park(v[j]);
-        park16(v, scratch, g, S::N / 16);
+        park_group(v, scratch, g, S::N / 16);
       } else {
         u64 bh[16];
-        unpark16(bh, scratch, g, S::N / 16);
+        unpark_group(bh, scratch, g, S::N / 16);
         const typename M::Product product(t);
 #pragma unroll
         for (int j = 0; j < 16; j++) v[j] = product(v[j], bh[j]);
-        gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.at(g), t);
+        gs_group<M, 4, 0, M::EXACT_AFTER_PRODUCT, false>(v, last_inv.template at<0>(g), t);
 #pragma unroll
         for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
       }
     });
   }
-  sub_inv<LOGC, S>(sm, cl, t, tw_mult);
+  sub_inv<LOGC, S>(sm, cl, t, tw_mult, last_inv);
   col_inv_out<LOGC, S, false>(reinterpret_cast<u64*>(job.c), sm, cl, rank, t, nullptr, rbase);
 }
 
