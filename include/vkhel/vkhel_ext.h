@@ -108,9 +108,10 @@ void vkhel_vector_elemfma_canonical(const struct vkhel_vector *a,
 		uint64_t multiplier, uint64_t mod);
 /* Negacyclic product result = a * b mod (X^n + 1, q) of the first n words,
  * equal to the reference composition forward(a), forward(b), elemmul,
- * inverse.  One fused launch for 256 <= n <= 131072 (one CTA, or a cluster
- * of CTAs sharing the polynomial through distributed shared memory).
- * Returns a status. */
+ * inverse.  One fused launch for 256 <= n <= 65536 (one CTA, or a cluster of
+ * CTAs sharing the polynomial through distributed shared memory); at 131072
+ * too where a buffer of n words for the faster global passes cannot be had
+ * (memory, the context's budget).  Returns a status. */
 int vkhel_vector_polymul(const struct vkhel_vector *a,
 		const struct vkhel_vector *b, struct vkhel_vector *result,
 		struct vkhel_ntt_tables *ntt);
@@ -127,7 +128,7 @@ int vkhel_vector_polymul_ntt(const struct vkhel_vector *a,
 /* ---- centred-lift epilogues ----
  * Up to VKHEL_MAX_LIFT_STEPS of the reference's element-wise ops applied, in
  * order, to the output of an inverse transform or polymul, inside the same
- * kernel for 256 <= n <= 131072 (a separate element-wise launch otherwise).
+ * kernel for n >= 256 (a separate element-wise launch below).
  * Results equal calling the reference functions one after another on the
  * result vector (src/vector.c:342-386, 429-511):
  *   VKHEL_LIFT_ELEMMOD    p0 = mod, p1 = q          vkhel_vector_elemmod
@@ -277,12 +278,13 @@ void vkhel_elem_batch_destroy(struct vkhel_elem_batch *batch);
  * of which one to launch is read once per process from $VKHEL_TUNE_TABLE or
  * from tuning/gb300.txt beside the package (written by vkhel_gb300.autotune).
  * Family VKHEL_TUNE_BATCH, log_n 0: 1 = run the degree classes of a batch on
- * concurrent streams; log_n 1: 1 = never split a few n = 2^12 .. 2^16 jobs
- * (at most one per 8 SMs, e.g. a single call) over clusters (the default, 0,
- * splits them: over 16 CTAs for n >= 2^14 with at most one job per 16 SMs,
- * otherwise over 8); log_n 2: 1 = run a ragged batch of fused products of
- * 2^12 .. 2^16 as one persistent launch; log_n 3: 1 = split over 8 CTAs
- * only. */
+ * concurrent streams; log_n 1: 1 = never split few jobs of n = 2^12 .. 2^17
+ * (fewer than the SMs, e.g. a single call, or those past a launch's whole
+ * rounds) over more CTAs than their degree's own kernel (the default, 0,
+ * splits them: single calls of n >= 2^14 over 16 CTAs, others over 2, 4 or 8
+ * by degree and count); log_n 2: 1 = run a ragged batch of fused products of
+ * 2^12 .. 2^16 as one persistent launch; log_n 3: 1 = single calls over 8
+ * CTAs only. */
 enum vkhel_tune_family {
 	VKHEL_TUNE_POLYMUL = 0,
 	VKHEL_TUNE_FORWARD = 1,

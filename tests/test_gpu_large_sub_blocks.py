@@ -77,3 +77,45 @@ def test_single_calls_in_place(vk, ctx, oracle, log_n):
     a = vk.Vector(ctx, a_h)
     vk.polymul(a, b, b, t)
     np.testing.assert_array_equal(b.download(), ref)
+
+
+@pytest.mark.parametrize("bits", [60, 62])
+@pytest.mark.parametrize("jobs", [1, 9, 10])
+def test_few_of_the_largest_cluster_degree(vk, ctx, oracle, jobs, bits):
+    """2^17: few jobs in global passes and sub-blocks, more on 8-CTA clusters;
+    and where the context's budget leaves no room for the passes' scratch."""
+    n = 1 << 17
+    q = workloads.ntt_primes(n, 1, bound=1 << bits)[0]
+    w = workloads.root_for(n, q)
+    t = vk.NttTables(n, q, w)
+    rng = np.random.default_rng(jobs)
+    a_h, b_h = workloads.uniform(rng, q, jobs * n), workloads.uniform(rng, q, jobs * n)
+    part = [slice(k * n, (k + 1) * n) for k in range(jobs)]
+    want = np.concatenate([oracle.polymul(a_h[s], b_h[s], n, q, w)[0] for s in part])
+    own = vk.Context()
+    a, b, c, f = vk.Vector(own, a_h), vk.Vector(own, b_h), vk.Vector(own, jobs * n), vk.Vector(own, jobs * n)
+
+    def run(add):
+        bt = vk.Batch(own)
+        add(bt)
+        bt.commit(graph=True)
+        bt.run()
+        bt.close()
+
+    run(lambda bt: bt.add_transform([t] * jobs, b, f))
+    np.testing.assert_array_equal(f.download(n), oracle.forward(b_h[:n], n, q, w)[0])
+    run(lambda bt: bt.add_polymul([t] * jobs, a, f, c, b_ntt=True))
+    np.testing.assert_array_equal(c.download(), want, err_msg="NTT(b) given")
+    run(lambda bt: bt.add_transform([t] * jobs, f, f, inverse=True, lift=LIFT))
+    np.testing.assert_array_equal(f.download(), _lift(oracle, b_h, q))
+    for budget in (0, own.bytes_in_use + 4096 * jobs):  # room for the job table alone
+        own.set_budget(budget)
+        run(lambda bt: bt.add_polymul([t] * jobs, a, b, c, lift=LIFT))
+        np.testing.assert_array_equal(c.download(), _lift(oracle, want, q), err_msg=f"budget {budget}")
+        if jobs == 1:
+            vk.polymul(a, b, c, t)
+            np.testing.assert_array_equal(c.download(), want, err_msg=f"one call, budget {budget}")
+            vk.forward_transform(b, f, t)
+            vk.polymul_ntt(a, f, c, t)
+            np.testing.assert_array_equal(c.download(), want, err_msg="one call, NTT(b) given")
+    own.close()

@@ -93,6 +93,14 @@ int vkh_dev_alloc(struct vkhel_ctx *ctx, uint64_t bytes, void **ptr) {
 	return VKHEL_OK;
 }
 
+int vkh_dev_try_alloc(struct vkhel_ctx *ctx, uint64_t bytes, void **ptr) {
+	if (vkh_inject_alloc_failure() || (ctx->budget && ctx->in_use + bytes > ctx->budget) ||
+			vkcu_alloc(ctx->pool, ctx->stream, bytes, ptr) != 0)
+		return 0;
+	ctx->in_use += bytes;
+	return 1;
+}
+
 void vkh_dev_free(struct vkhel_ctx *ctx, void *ptr, uint64_t bytes) {
 	if (!ptr)
 		return;
@@ -686,8 +694,15 @@ static int polymul_impl(const struct vkhel_vector *a, const struct vkhel_vector 
 			return st;
 		scratch = tmp;
 	}
+	/* one product of the largest fused degree is faster in global passes and
+	 * sub-blocks over more SMs, which need a buffer for b's; without one (the
+	 * budget, a full device) the fused kernel does */
+	const int passes = vkcu_few_composed(1, t->log_n, vkcu_qclass(t->q), ctx->sms) &&
+			(b_ntt || tmp || vkh_dev_try_alloc(ctx, bytes, &tmp));
+	if (tmp)
+		scratch = tmp;
 	int e;
-	if (fused) {
+	if (fused && !passes) {
 		const vkcu_poly_job job = {a->dev, b->dev, res->dev, scratch, d->dev_set, b_ntt ? VKCU_JOB_B_NTT : 0};
 		e = vkcu_polymul_lift(ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms, ctx->sms, lp, b_ntt);
 	} else {

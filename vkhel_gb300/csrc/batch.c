@@ -28,6 +28,7 @@ struct job_rec {
 	uint32_t kind;         /* VKH_JOB_* */
 	uint32_t log_n;
 	uint32_t needs_scratch;
+	uint32_t extra_scratch; /* also where its class runs composed though it need not */
 	uint32_t lift;         /* index into the batch's lift table, 0 = none */
 	uint32_t qclass;       /* modulus class, VKCU_Q60 .. VKCU_Q63 */
 	uint32_t b_ntt;        /* b holds NTT(b) (VKCU_JOB_B_NTT) */
@@ -501,6 +502,7 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 	b->nclasses = 0;
 	for (uint32_t i = 0; i < b->njobs; i++) {
 		struct job_rec *r = &b->recs[i];
+		r->extra_scratch = 0;
 		if (b->nclasses == 0 || b->classes[b->nclasses - 1].kind != r->kind ||
 				b->classes[b->nclasses - 1].log_n != r->log_n || b->classes[b->nclasses - 1].qclass != (int) r->qclass ||
 				b->classes[b->nclasses - 1].lift != r->lift || b->classes[b->nclasses - 1].b_ntt != r->b_ntt) {
@@ -527,15 +529,45 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 		if (r->needs_scratch)
 			scratch_words += slice_words(r->log_n);
 	}
-	if (scratch_words) {
+	/* classes that run faster composed, where their scratch can be had (not
+	 * under tuning entry (3, 2), which asks for as few launches as possible) */
+	uint64_t work = 0, extra_words = 0;
+	for (uint32_t k = 0; k < b->nclasses; k++)
+		work += class_work(&b->classes[k]);
+	for (int pass = vkh_variant(3, 2) == 1 ? 2 : 0; pass < 2; pass++) { /* 0: those with NTT(b) given and the words of the others, 1: the others */
+		for (uint32_t k = 0; k < b->nclasses; k++) {
+			struct vkh_job_class *cl = &b->classes[k];
+			const int avail = vkh_variant(3, 0) == 1 ? (int) (class_work(cl) * ctx->sms / work) : ctx->sms;
+			if (cl->kind != VKH_JOB_POLYMUL || !cl->fused ||
+					!vkcu_few_composed(cl->count, cl->log_n, cl->qclass, avail))
+				continue;
+			if (pass == 1 || cl->b_ntt)
+				cl->fused = 0;
+			for (uint32_t i = cl->first; !cl->b_ntt && i < cl->first + cl->count; i++) {
+				if (pass == 0 && !b->recs[i].needs_scratch)
+					extra_words += slice_words(cl->log_n);
+				b->recs[i].extra_scratch = pass == 1;
+			}
+		}
+		if (pass == 0 && extra_words) {
+			b->scratch_bytes = (scratch_words + extra_words) * sizeof(uint64_t);
+			if (!vkh_dev_try_alloc(ctx, b->scratch_bytes, &b->scratch)) {
+				b->scratch_bytes = 0;
+				break;
+			}
+		}
+	}
+	if (scratch_words && !b->scratch) {
 		b->scratch_bytes = scratch_words * sizeof(uint64_t);
 		int st = vkh_dev_alloc(ctx, b->scratch_bytes, &b->scratch);
 		if (st)
 			return st;
+	}
+	if (b->scratch) {
 		uint64_t off = 0;
 		for (uint32_t i = 0; i < b->njobs; i++) {
 			struct job_rec *r = &b->recs[i];
-			if (r->needs_scratch) {
+			if (r->needs_scratch || r->extra_scratch) {
 				r->job.scratch = (uint64_t *) b->scratch + off;
 				off += slice_words(r->log_n);
 			}

@@ -86,6 +86,8 @@ uint64_t vkh_invmod(uint64_t a, uint64_t mod);
 int vkh_fail(struct vkhel_ctx *ctx, int code, const char *fmt, ...);
 int vkh_cuda(struct vkhel_ctx *ctx, int cuda_err, const char *what);
 int vkh_dev_alloc(struct vkhel_ctx *ctx, uint64_t bytes, void **ptr);
+/* The same for memory the caller can do without: 1, or 0 with no error recorded. */
+int vkh_dev_try_alloc(struct vkhel_ctx *ctx, uint64_t bytes, void **ptr);
 void vkh_dev_free(struct vkhel_ctx *ctx, void *ptr, uint64_t bytes);
 /* tables.c -- device table cache */
 int vkh_devtab_get(struct vkhel_ctx *ctx, const struct vkhel_ntt_tables *t,

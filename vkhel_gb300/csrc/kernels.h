@@ -230,7 +230,10 @@ int vkcu_lift_jobs(void *stream, const vkcu_ntt_job *jobs, int njobs, const vkcu
  * polymul that is not fused. */
 int vkcu_pointwise(void *stream, const vkcu_poly_job *jobs, int njobs,
 		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms);
-/* Products outside the single-launch degrees.  b, a and c are the jobs'
+/* 1 where a class of products of a single-launch degree is faster through
+ * vkcu_polymul_composed (few of the largest one): needs scratch for b. */
+int vkcu_few_composed(long njobs, uint32_t log_n, int qclass, int avail);
+/* Products outside the single-launch degrees, and those.  b, a and c are the jobs'
  * transforms b -> scratch, a -> c and c -> c (device arrays, or NULL with a
  * single job `one`). */
 int vkcu_polymul_composed(void *stream, const vkcu_poly_job *jobs, const vkcu_ntt_job *b,

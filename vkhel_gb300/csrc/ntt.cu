@@ -270,7 +270,7 @@ static int inverse_passes(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, 
 // products on CTA-resident 2^14-word sub-blocks and more global passes before:
 // 90, 99, 121 and 885 us.
 static int sub_log_of(int njobs, int log_n, int sms) {
-  return ((long)njobs << (log_n - 16)) * 8 > (long)sms ? log_n - 16 : log_n - 14;
+  return log_n > 17 && ((long)njobs << (log_n - 16)) * 8 > (long)sms ? log_n - 16 : log_n - 14;
 }
 
 }  // namespace vk
@@ -304,13 +304,21 @@ static bool jobs_aligned(const vkcu_ntt_job* jobs, const vkcu_ntt_job* one) {
 static int split_log(long njobs, uint32_t log_n, long avail, bool single) {
   if (log_n < 12 || log_n > 17 || vkh_variant(3, 1) != 0) return 0;
   if (single && log_n >= 14 && njobs * 16 <= avail && vkh_variant(3, 3) == 0) return 4;
-  if (log_n == 17) return 0;  // 8 CTAs in any case
+  if (log_n == 17) return 0;
   switch (log_n) {
     case 13: return njobs * 5 <= avail ? 3 : njobs * 2 <= avail ? 1 : 0;
     case 14: return njobs * 5 <= avail ? 3 : njobs * 5 <= 2 * avail ? 2 : njobs * 2 <= avail ? 1 : 0;
     case 15: return njobs * 3 <= avail ? 3 : 0;
     default: return njobs * 8 <= avail ? 3 : 0;
   }
+}
+
+// Few transforms and products of 2^17 take the path of larger degrees: a global
+// pass and 2^14-word sub-blocks on 8 small CTAs, 64 SMs a job instead of 8 or
+// 16 (forward transforms, 8-CTA clusters / so: 1 33 / 12 us, 4 33 / 16, 9 35 /
+// 27; products 1 83 / 29 us, 4 83 / 37, 9 85 / 63; 12 jobs are even).
+static bool few_of_17(long njobs, uint32_t log_n, long avail) {
+  return log_n == 17 && njobs * 16 <= avail && vkh_variant(3, 1) == 0;
 }
 
 // The last jobs of a launch whose kernel runs `round` jobs at a time, one per
@@ -365,14 +373,14 @@ static int forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
     if (log_n <= (uint32_t)kMaxCta) return fwd_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms);
     if (log_n <= (uint32_t)kMaxCluster) return fwd_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta);
   } else {
-    if (const int lc = split_log(njobs, log_n, avail, jobs == nullptr)) {
+    if (const int lc = few_of_17(njobs, log_n, avail) ? 0 : split_log(njobs, log_n, avail, jobs == nullptr)) {
       const int e = fwd_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc);
       // a GPU that cannot host 16-CTA clusters: the set-up refuses before any launch
       return e == (int)cudaErrorInvalidConfiguration && lc == 4
                  ? fwd_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3)
                  : e;
     }
-    if (log_n <= (uint32_t)kMaxCluster) {
+    if (log_n <= (uint32_t)kMaxCluster && !few_of_17(njobs, log_n, avail)) {
       const int variant = log_n <= (uint32_t)kMaxCta ? vkh_variant_jobs(1, (int)log_n, njobs, sms) : 0;
       const Tail tail(jobs != nullptr, njobs, log_n, round_jobs(log_n, variant, sms), sms, avail, false);
       const int main = njobs - tail.jobs;
@@ -419,13 +427,13 @@ static int inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
       if (log_n <= (uint32_t)kMaxCta) return inv_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms, lp);
       if (log_n <= (uint32_t)kMaxCluster) return inv_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta, lp);
     } else {
-      if (const int lc = split_log(njobs, log_n, avail, jobs == nullptr)) {
+      if (const int lc = few_of_17(njobs, log_n, avail) ? 0 : split_log(njobs, log_n, avail, jobs == nullptr)) {
         const int r = inv_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc, lp);
         return r == (int)cudaErrorInvalidConfiguration && lc == 4
                    ? inv_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3, lp)
                    : r;
       }
-      if (log_n <= (uint32_t)kMaxCluster) {
+      if (log_n <= (uint32_t)kMaxCluster && !few_of_17(njobs, log_n, avail)) {
         // the lifted CTA kernels run in the default shape
         const int variant = log_n <= (uint32_t)kMaxCta && !lifted ? vkh_variant_jobs(2, (int)log_n, njobs, sms) : 0;
         const Tail tail(jobs != nullptr, njobs, log_n, round_jobs(log_n, variant, sms), sms, avail, false);
@@ -455,6 +463,24 @@ extern "C" int vkcu_ntt_inverse_lift(void* stream, const vkcu_ntt_job* jobs, int
                                      uint32_t log_n, int qclass, int sms, int avail, const vkcu_lift* lift) {
   return by_class(qclass,
                   [&](auto m) { return inverse<decltype(m)>(stream, jobs, njobs, one, log_n, sms, avail, lift); });
+}
+
+// A product of 2^17 .. 2^26, q < 2^62: the global passes of b
+// (into scratch) and of a (into c), one launch for every sub-block's forward,
+// product and inverse, the inverse global passes of c.  b, a and c give these
+// the jobs of the passes.
+template <class M>
+static int polymul_large(cudaStream_t st, const vkcu_poly_job* jobs, const vkcu_ntt_job* b, const vkcu_ntt_job* a,
+                         const vkcu_ntt_job* c, int njobs, const vkcu_poly_job& one, int log_n, int sms,
+                         const vkcu_lift* lift, int b_ntt) {
+  const vkcu_ntt_job ob{one.b, one.scratch, one.tw}, oa{one.a, one.c, one.tw}, oc{one.c, one.c, one.tw};
+  const int sub_log = sub_log_of(njobs, log_n, sms);
+  const GlobalPlan plan{sub_log};
+  int e = b_ntt ? 0 : forward_passes<M>(st, b, njobs, ob, log_n, plan, sms);
+  if (!e) e = forward_passes<M>(st, a, njobs, oa, log_n, plan, sms);
+  if (!e) e = poly_cluster_sub<M>(st, jobs, njobs, one, log_n, sub_log);
+  if (!e) e = inverse_passes<M>(st, c, njobs, oc, log_n, plan, sms, 1, lift);
+  return e;
 }
 
 template <class M>
@@ -497,27 +523,13 @@ extern "C" int vkcu_polymul(void* stream, const vkcu_poly_job* jobs, int njobs, 
   return vkcu_polymul_lift(stream, jobs, njobs, one, log_n, qclass, sms, sms, nullptr, 0);
 }
 
-// A product past one cluster (2^18 .. 2^26, q < 2^62): the global passes of b
-// (into scratch) and of a (into c), one launch for every sub-block's forward,
-// product and inverse, the inverse global passes of c.  b, a and c give these
-// the jobs of the passes.
-template <class M>
-static int polymul_large(cudaStream_t st, const vkcu_poly_job* jobs, const vkcu_ntt_job* b, const vkcu_ntt_job* a,
-                         const vkcu_ntt_job* c, int njobs, const vkcu_poly_job& one, int log_n, int sms,
-                         const vkcu_lift* lift, int b_ntt) {
-  const vkcu_ntt_job ob{one.b, one.scratch, one.tw}, oa{one.a, one.c, one.tw}, oc{one.c, one.c, one.tw};
-  const int sub_log = sub_log_of(njobs, log_n, sms);
-  const GlobalPlan plan{sub_log};
-  int e = b_ntt ? 0 : forward_passes<M>(st, b, njobs, ob, log_n, plan, sms);
-  if (!e) e = forward_passes<M>(st, a, njobs, oa, log_n, plan, sms);
-  if (!e) e = poly_cluster_sub<M>(st, jobs, njobs, one, log_n, sub_log);
-  if (!e) e = inverse_passes<M>(st, c, njobs, oc, log_n, plan, sms, 1, lift);
-  return e;
-}
-
-// A product outside the single-launch degrees: past one cluster as above; for
+// A product outside the single-launch degrees (or few of 2^17): as above; for
 // n < 2^8, and q >= 2^62 past one cluster, forward(b), forward(a), pointwise,
 // inverse.
+extern "C" int vkcu_few_composed(long njobs, uint32_t log_n, int qclass, int avail) {
+  return qclass != VKCU_Q63 && few_of_17(njobs, log_n, avail);
+}
+
 extern "C" int vkcu_polymul_composed(void* stream, const vkcu_poly_job* jobs, const vkcu_ntt_job* b,
                                      const vkcu_ntt_job* a, const vkcu_ntt_job* c, int njobs,
                                      const vkcu_poly_job* one, uint32_t log_n, int qclass, int sms,
@@ -529,10 +541,10 @@ extern "C" int vkcu_polymul_composed(void* stream, const vkcu_poly_job* jobs, co
   const vkcu_lift* lp = has_lift(lift) ? lift : nullptr;
   const bool aligned =
       jobs != nullptr || (aligned32(o.a) && aligned32(o.b) && aligned32(o.c) && aligned32(o.scratch));
-  if (log_n > (uint32_t)kMaxCluster && !aligned) return (int)cudaErrorMisalignedAddress;
-  if (log_n > (uint32_t)kMaxCluster && qclass == VKCU_Q60)
+  if (log_n >= (uint32_t)kMaxCluster && !aligned) return (int)cudaErrorMisalignedAddress;
+  if (log_n >= (uint32_t)kMaxCluster && qclass == VKCU_Q60)
     return polymul_large<Mod60>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
-  if (log_n > (uint32_t)kMaxCluster && qclass == VKCU_Q62)
+  if (log_n >= (uint32_t)kMaxCluster && qclass == VKCU_Q62)
     return polymul_large<Mod62>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
   const vkcu_ntt_job ob{o.b, o.scratch, o.tw}, oa{o.a, o.c, o.tw}, oc{o.c, o.c, o.tw};
   int e = b_ntt ? 0 : vkcu_ntt_forward(stream, b, njobs, &ob, log_n, qclass, sms, sms);

@@ -74,7 +74,9 @@ extern "C" int vkcu_pool_independent_streams(void* pool) {
 
 extern "C" int vkcu_alloc(void* pool, void* stream, size_t bytes, void** ptr) {
   *ptr = nullptr;
-  return (int)cudaMallocFromPoolAsync(ptr, bytes ? bytes : 8, (cudaMemPool_t)pool, (cudaStream_t)stream);
+  const cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes ? bytes : 8, (cudaMemPool_t)pool, (cudaStream_t)stream);
+  if (e != cudaSuccess) cudaGetLastError();  // the caller reports it, or does without the memory
+  return (int)e;
 }
 
 extern "C" int vkcu_free(void* stream, void* ptr) {
