@@ -35,7 +35,7 @@ POLYMUL, FORWARD, INVERSE, BATCH = 0, 1, 2, 3
 # a variant replaces the incumbent (variant 0 for the many-jobs bucket, the
 # many-jobs choice for the other buckets) only when it is this much faster:
 # smaller gaps are within run-to-run noise
-MARGIN = 0.02
+MARGIN = 0.015
 # jobs per SM timed for each bucket of the table (<= 1, <= 2, <= 4, more)
 BUCKET_JOBS_PER_SM = (1.0, 1.5, 3.0, 8.0)
 VARIANTS = {8: [0, 1], 9: [0, 1], 10: [0, 1, 2], 11: [0, 1, 2], 12: [0, 1, 2], 13: [0, 1, 2], 14: [0, 1]}
