@@ -269,7 +269,10 @@ __global__ void __launch_bounds__(S::T, cluster_blocks<S>())
     for (int i = 0; i < S::GROUPS; i++) {
       const int g = S::group(i);
       u64 v[S::W];
-      load_group(v, in + S::W * g);
+      if constexpr (staged_loads<S>())
+        load_group_staged<S>(v, in, sm, g, [] {});
+      else
+        load_group(v, in + S::W * g);
       gs_group<typename S::M, S::R, 0, true, false>(v, last.template at<4 - S::R>(g), t);
 #pragma unroll
       for (int j = 0; j < S::W; j++) sm[pad(S::W * g) + j] = v[j];

@@ -937,6 +937,57 @@ __device__ __forceinline__ void store_group(const u64 (&v)[K], u64* p) {
   for (int h = 0; h < K / 4; h++) st4(p + 4 * h, v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
 }
 
+// The same for a warp's 32 neighbouring radix-16 groups (512 consecutive
+// words), through the shared words of those groups, which the warp must be
+// done with: a lane's 32-byte pieces of its own group lie 128 bytes from the
+// next lane's, so that a load or store of them costs the LSU about 60
+// wavefronts; 16-byte pairs over whole lines and a turn through shared memory
+// cost 8 + 8.  g is the lane's group; `sync` runs before the words are written.
+// Measured: inverse transforms of 2^11 .. 2^14 3-9 % faster with staged loads
+// (1024 of 2^14 175.6 -> 160.0 us, 2048 of 2^13 167.5 -> 151.8; 2^10 even);
+// forward ones of 2^9 .. 2^13 0.5-2 % with staged stores, but 2.4 % slower at
+// 2^14, where a CTA has its SM to itself and nothing overlaps the turn.  A given
+// NTT(b) is staged in the CTA products (480 of 2^14 182.6 -> 179.5 us) and not
+// in the cluster ones (150 of 2^15 104.5 -> 106.4).
+template <class S>
+constexpr bool staged_loads() {
+  return S::R == 4 && S::LOGN >= 11;
+}
+template <class S>
+constexpr bool staged_stores() {
+  return S::R == 4 && S::LOGN >= 9 && S::LOGN <= 13;
+}
+
+template <class S, class Sync>
+__device__ __forceinline__ void load_group_staged(u64 (&v)[16], const u64* p, u64* sm, int g, Sync&& sync) {
+  const int lane = (int)threadIdx.x & 31, w0 = (g - lane) * 16 + 2 * lane;
+  ulonglong2 x[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    asm volatile("ld.global.L1::no_allocate.v2.u64 {%0,%1}, [%2];" : "=l"(x[k].x), "=l"(x[k].y) : "l"(p + w0 + 64 * k));
+  sync();
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    sm[pad(w0 + 64 * k)] = x[k].x;
+    sm[pad(w0 + 64 * k) + 1] = x[k].y;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 16; j++) v[j] = sm[pad(16 * g) + j];
+}
+
+// A warp's words of all its groups, already in shared memory, to p.
+template <class S>
+__device__ __forceinline__ void store_staged(u64* p, const u64* sm) {
+  __syncwarp();
+  const int w0 = (S::tid() >> 5) * (32 * S::E) + 2 * (S::tid() & 31);
+#pragma unroll 8
+  for (int k = 0; k < S::E / 2; k++) {
+    const int i = w0 + 64 * k;
+    asm volatile("st.global.v2.u64 [%0], {%1,%2};" ::"l"(p + i), "l"(sm[pad(i)]), "l"(sm[pad(i) + 1]) : "memory");
+  }
+}
+
 // NTT(b) parked between the phases of a fused product: 16-byte pairs, pair jj
 // of group g (of G) at jj G + g, so that a warp moves whole lines (each thread
 // reads back what it wrote).
@@ -1012,8 +1063,14 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
       const typename M::Out to(t);
 #pragma unroll
       for (int j = 0; j < 16; j++) v[j] = to.canon(v[j]);
-      store_group(v, out + 16 * g);
+      if constexpr (staged_stores<S>()) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) sm[pad(16 * g) + j] = v[j];
+      } else {
+        store_group(v, out + 16 * g);
+      }
     });
+    if constexpr (staged_stores<S>()) store_staged<S>(out, sm);
   }
 }
 
@@ -1050,9 +1107,15 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     for (int i = 0; i < S::E / 16; i++) {
       const int g = S::group(i);
       u64 v[16];
-      load_group(v, in + 16 * g);
+      auto free_words = [&] {
+        if (i == 0) __syncthreads();  // the last job's words are read
+      };
+      if constexpr (staged_loads<S>())
+        load_group_staged<S>(v, in, sm, g, free_words);
+      else
+        load_group(v, in + 16 * g);
       gs_group<M, 4, 0, true, false>(v, last.template at<0>(g), t);
-      if (i == 0) __syncthreads();  // the last job's words are read
+      if constexpr (!staged_loads<S>()) free_words();
 #pragma unroll
       for (int j = 0; j < 16; j++) sm[pad(16 * g + j)] = v[j];
     }
@@ -1100,7 +1163,10 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E, true>())
         } else {
           u64 bh[16];
           if (b_ntt) {
-            load_group(bh, reinterpret_cast<const u64*>(job.b) + 16 * g);
+            if constexpr (staged_loads<S>())
+              load_group_staged<S>(bh, reinterpret_cast<const u64*>(job.b), sm, g, [] { __syncwarp(); });
+            else
+              load_group(bh, reinterpret_cast<const u64*>(job.b) + 16 * g);
             reduce_operands(bh, t);
           } else {
             unpark_group(bh, scratch, g, S::N / 16);
