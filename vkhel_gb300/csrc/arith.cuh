@@ -163,6 +163,16 @@ __device__ __forceinline__ u64 ref_reduce64(u64 x, u64 mod, u64 mu, u32 n) {
   return z >= mod ? z - mod : z;
 }
 
+// The same with the products as chains, for the epilogues inside the
+// transforms (480 inverse transforms of 2^14 words with one step 106.4 -> 102.7
+// us with these and no branches; the element-wise kernels are bound by memory).
+__device__ __forceinline__ u64 ref_reduce64_chain(u64 x, u64 mod, u64 mu, u32 n) {
+  const u64 qh = mulhi_chain(x >> (n - 2), mu), nm = 0 - mod;
+  const u64 r = mad_wide(lo32(qh), lo32(nm), x);
+  const u64 z = pack(lo32(r), hi32(r) + lo32(qh) * hi32(nm) + hi32(qh) * lo32(nm));
+  return z >= mod ? z - mod : z;
+}
+
 // The same for operands that are usually reduced already.  For x < mod the
 // estimate floor(k mu / 2^64), k = x >> (n - 2) <= 3, mu <= 2^63, is 0: it
 // needs k mu >= 2^64, i.e. k = 2 with mod = 2^(n-1) (but x < mod gives

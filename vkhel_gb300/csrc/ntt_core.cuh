@@ -874,7 +874,11 @@ struct LiftFold {
       } else if (kind == VKCU_LIFT_GTSUB) {
         const u64 d = tq ? ref_reduce64(q, mod, mu, bits) : st.d;
 #pragma unroll
-        for (int k = 0; k < K; k++) v[k] = ref_gtsub(v[k], bound, d, mod, mu, bits);
+        for (int k = 0; k < K; k++) {  // ref_gtsub, without its branches
+          const u64 r = ref_reduce64_chain(v[k], mod, mu, bits);
+          const u64 z = r + mod - d, zr = z >= mod ? z - mod : z;
+          v[k] = v[k] > bound ? zr : r;
+        }
       } else {
         const u64 d = st.d;
 #pragma unroll
