@@ -241,7 +241,10 @@ __global__ void __launch_bounds__(S::T, cluster_blocks<S>())
       const typename S::M::Out to(t);
 #pragma unroll
       for (int j = 0; j < S::W; j++) v[j] = to.canon(v[j]);
-      store_group(v, out + S::W * g);
+      if constexpr (staged_stores<S>())
+        store_group_staged(v, out, sm, g);
+      else
+        store_group(v, out + S::W * g);
     });
   }
   cl.sync();

@@ -949,8 +949,9 @@ __device__ __forceinline__ void store_group(const u64 (&v)[K], u64* p) {
 // cost 8 + 8.  g is the lane's group; `sync` runs before the words are written.
 // Measured: inverse transforms of 2^11 .. 2^14 3-9 % faster with staged loads
 // (1024 of 2^14 175.6 -> 160.0 us, 2048 of 2^13 167.5 -> 151.8; 2^10 even);
-// forward ones of 2^9 .. 2^13 0.5-2 % with staged stores, but 2.4 % slower at
-// 2^14, where a CTA has its SM to itself and nothing overlaps the turn.  A given
+// forward ones 0.5-2 % to 2^13 and 4 % from 2^14 on with staged stores (1000 of
+// 2^14 163.9 -> 157.6 us, 512 of 2^15 187.4 -> 179.8; storing after all groups
+// instead of group by group made 2^14 2.4 % slower than unstaged).  A given
 // NTT(b) is staged in the CTA products (480 of 2^14 182.6 -> 179.5 us) and not
 // in the cluster ones (150 of 2^15 104.5 -> 106.4).
 template <class S>
@@ -959,7 +960,7 @@ constexpr bool staged_loads() {
 }
 template <class S>
 constexpr bool staged_stores() {
-  return S::R == 4 && S::LOGN >= 9 && S::LOGN <= 13;
+  return S::R == 4 && S::LOGN >= 9;  // whole warps
 }
 
 template <class S, class Sync>
@@ -980,13 +981,14 @@ __device__ __forceinline__ void load_group_staged(u64 (&v)[16], const u64* p, u6
   for (int j = 0; j < 16; j++) v[j] = sm[pad(16 * g) + j];
 }
 
-// A warp's words of all its groups, already in shared memory, to p.
-template <class S>
-__device__ __forceinline__ void store_staged(u64* p, const u64* sm) {
+// (The warp is done with these words: every lane has read its own.)
+__device__ __forceinline__ void store_group_staged(const u64 (&v)[16], u64* p, u64* sm, int g) {
+#pragma unroll
+  for (int j = 0; j < 16; j++) sm[pad(16 * g) + j] = v[j];
   __syncwarp();
-  const int w0 = (S::tid() >> 5) * (32 * S::E) + 2 * (S::tid() & 31);
-#pragma unroll 8
-  for (int k = 0; k < S::E / 2; k++) {
+  const int lane = (int)threadIdx.x & 31, w0 = (g - lane) * 16 + 2 * lane;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
     const int i = w0 + 64 * k;
     asm volatile("st.global.v2.u64 [%0], {%1,%2};" ::"l"(p + i), "l"(sm[pad(i)]), "l"(sm[pad(i) + 1]) : "memory");
   }
@@ -1067,14 +1069,11 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
       const typename M::Out to(t);
 #pragma unroll
       for (int j = 0; j < 16; j++) v[j] = to.canon(v[j]);
-      if constexpr (staged_stores<S>()) {
-#pragma unroll
-        for (int j = 0; j < 16; j++) sm[pad(16 * g) + j] = v[j];
-      } else {
+      if constexpr (staged_stores<S>())
+        store_group_staged(v, out, sm, g);
+      else
         store_group(v, out + 16 * g);
-      }
     });
-    if constexpr (staged_stores<S>()) store_staged<S>(out, sm);
   }
 }
 
