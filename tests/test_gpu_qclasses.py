@@ -116,3 +116,25 @@ def test_batch_of_both_classes_and_an_even_modulus(vk, ctx, oracle, log_n):
     x, y = vk.Vector(ctx, x_h), vk.Vector(ctx, n)
     vk.forward_transform(x, y, t)
     np.testing.assert_array_equal(y.download(), oracle.forward(x_h, n, q, 5)[0])
+
+
+@pytest.mark.parametrize("which", ["top60", "past60", "bits31", "least"])
+@pytest.mark.parametrize("log_n", [3, 9, 10, 12, 14, 15, 17, 18])
+def test_single_words_past_the_inverse_group_check(vk, ctx, oracle, log_n, which):
+    """The inverse's first sub-stage checks its group's words against 2^bits(q)
+    together: words on both sides of that and of 2q, one in 97 among words below
+    q.  (2^64 - 1 only where the butterfly subtracts from it: the reference's
+    subtraction loop wraps past 2^64 before it reaches it as the other operand.)"""
+    n = 1 << log_n
+    q = _modulus(n, which)
+    w = workloads.root_for(n, q)
+    t = vk.NttTables(n, q, w)
+    rng = np.random.default_rng(97 + log_n)
+    top = 1 << q.bit_length()
+    edges = np.array([q, top - 1, top, 2 * q - 1, 2 * q, 3 * q, (1 << 64) - 1], np.uint64)
+    a_h = workloads.uniform(rng, q, n)
+    a_h[::97] = rng.choice(edges, len(a_h[::97]))
+    a_h[1::2] = np.minimum(a_h[1::2], np.uint64(3 * q))
+    a, r = vk.Vector(ctx, a_h), vk.Vector(ctx, n)
+    vk.inverse_transform(a, r, t)
+    np.testing.assert_array_equal(r.download(), oracle.inverse(a_h, n, q, w)[0])

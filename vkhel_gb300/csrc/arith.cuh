@@ -145,14 +145,6 @@ __device__ __forceinline__ void ct_bfly(u64& x, u64& y, u64 w, u64 wp, u64 q, u6
   y = xr - t + q2;
 }
 
-// Gentleman-Sande butterfly on lazy values: X, Y in [0, 2q) -> [0, 2q).
-__device__ __forceinline__ void gs_bfly(u64& x, u64& y, u64 w, u64 wp, u64 q, u64 q2) {
-  const u64 s = x + y;
-  const u64 d = x - y + q2;
-  x = csub(s, q2);
-  y = shoup_lazy(d, w, wp, q);
-}
-
 // ---- reference-exact Barrett (alpha = 62, beta = -2) ----------------------
 // n = bit length of mod (>= 2), mu = floor(2^(n+62) / mod).
 
