@@ -1093,6 +1093,12 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     u64* out = reinterpret_cast<u64*>(job.out) + ((size_t)sub << LOGN);
     const u64* in = sub_log ? out : reinterpret_cast<const u64*>(job.in);
     const u32 tw_mult = (1u << sub_log) + sub;
+    // the next transform's words into L2 (1000 of 2^14 157.9 -> 156.2 us; even
+    // at 2^13, and before the outputs left in whole lines 1 % slower)
+    if (!SUB && LOGN == 14 && w + (int)gridDim.x < total && threadIdx.x < 4) {
+      const vkcu_ntt_job nx = fetch_job(jobs, one, w + (int)gridDim.x);
+      prefetch_l2(reinterpret_cast<const char*>(nx.in) + threadIdx.x * (S::N * 2), S::N * 2);
+    }
     fwd_first<S, !SUB>(sm, in, t, tw_mult);
     fwd_passes<S>(sm, t, tw_mult, last, [&](int g, u64(&v)[16]) {
       const typename M::Out to(t);
@@ -1124,7 +1130,7 @@ __global__ void __launch_bounds__((1 << LOGN) / E, min_blocks<LOGN, E>())
     const u64* in = reinterpret_cast<const u64*>(job.in) + ((size_t)sub << LOGN);
     u64* out = reinterpret_cast<u64*>(job.out) + ((size_t)sub << LOGN);
     // the next work item's words into L2 while this one runs (2.6-3.4 % on
-    // batched inverse transforms; the forward kernel measured no better so)
+    // batched inverse transforms)
     if (w + (int)gridDim.x < total && threadIdx.x < 4) {
       const int w2 = w + (int)gridDim.x, sub2 = w2 & ((1 << sub_log) - 1);
       const vkcu_ntt_job nx = fetch_job(jobs, one, w2 >> sub_log);
