@@ -14,8 +14,10 @@ the device so that a profiler capture of one launch ends quickly.
   fwd_cluster   64 forward transforms of n = 2^16 (batch)       k_ntt_fwd_cluster<2,..>
   inv_cluster   64 inverse transforms of n = 2^16 (batch)       k_ntt_inv_cluster<2,..>
   twiddles      device twiddle tables for n = 2^20              k_twiddles
-  global        16 forward + 16 inverse transforms of n = 2^20  k_fwd_global, k_inv_global
-  pointwise     32 polymuls of n = 2^18 (composed path)         k_pointwise
+  global        16 forward + 16 inverse transforms of n = 2^20  k_fwd_global, k_inv_global,
+                k_ntt_{fwd,inv}_cluster<2,..> on the 2^16-word sub-blocks
+  pointwise     32 polymuls of n = 2^18                         k_fwd_global, k_polymul_cluster<2,..>
+                on the 2^16-word sub-blocks, k_inv_global
   simple        4096 forward + inverse transforms of n = 2^7    k_ntt_fwd_simple, k_ntt_inv_simple
   wide_polymul  256 polymuls of n = 2^14, 63-bit primes         k_polymul<14,..,Mod63>
   cluster_polymul  64 polymuls of n = 2^16 (single-limb batch)  k_polymul_cluster<2,..>
@@ -28,7 +30,7 @@ the device so that a profiler capture of one launch ends quickly.
   ntt_operand   256 polymuls of n = 2^14 with b given as NTT(b)  k_polymul<14,..,true> (the
                 epilogue instantiation, no steps)
   lift_jobs     32 inverse transforms of n = 2^20 with a two-step centred lift
-                k_inv_global, k_ntt_inv<14,..>, k_lift_stream (the epilogue pass)
+                k_ntt_inv_cluster<2,..>, k_inv_global (the epilogue in its last pass)
   single_call_n65536  one polymul and one forward transform of n = 2^16 as single calls
                 k_polymul_cluster<4, Shape<12,16>>, k_ntt_fwd_cluster<4, ..> (16-CTA clusters)
 """
@@ -220,9 +222,7 @@ def case_wide_transforms(ctx):
 
 def case_lift_jobs(ctx):
     """32 inverse transforms of n = 2^20 (256 MB) with the centred-lift
-    epilogue: the global passes leave the words in HBM and k_lift_stream
-    applies the steps (elemmod 65537, elemgtadd) as its own element-wise
-    pass."""
+    epilogue (elemmod 65537, elemgtadd), applied by the last global pass."""
     n, jobs, primes = 1 << 20, 32, 4
     qs, tabs = _tabs(n, primes)
     x = _operands(ctx, n, qs, jobs, 5)

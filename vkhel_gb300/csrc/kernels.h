@@ -221,7 +221,8 @@ int vkcu_ntt_inverse_lift(void *stream, const vkcu_ntt_job *jobs, int njobs,
 int vkcu_polymul_lift(void *stream, const vkcu_poly_job *jobs, int njobs,
 		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms, int avail, const vkcu_lift *lift, int b_ntt);
 /* The epilogue alone, in place on `len` words at p (modulus q for TABLE_Q
- * steps), or on the n output words of every job. */
+ * steps), or on the n output words of every job (those of the simple kernels;
+ * the others lift in their last pass). */
 int vkcu_lift_range(void *stream, uint64_t *p, uint64_t len, uint64_t q, int sms, const vkcu_lift *lift);
 int vkcu_lift_jobs(void *stream, const vkcu_ntt_job *jobs, int njobs, const vkcu_ntt_job *one,
 		uint32_t log_n, int sms, const vkcu_lift *lift);
@@ -254,8 +255,8 @@ int vkcu_polymul_ragged(void *stream, const vkcu_ragged_item *items, int n_clust
 
 /* Kernel variant table (tuning.c): family 0 = fused polymul, 1 = forward,
  * 2 = inverse, 3 = batch options (log_n 0: concurrent degree classes, 1:
- * no split of single jobs over 8 CTAs, 2: ragged batches as one launch);
- * per degree and, for a launch of njobs jobs
+ * no split of few jobs over clusters, 2: ragged batches as one launch, 3:
+ * single calls on at most 8 CTAs); per degree and, for a launch of njobs jobs
  * on sms SMs, per job-count bucket (vkh_variant: the many-jobs entry). */
 int vkh_variant(int family, int log_n);
 int vkh_variant_jobs(int family, int log_n, long njobs, int sms);

@@ -591,10 +591,9 @@ __global__ void __launch_bounds__(256) k_lift_range(u64* __restrict__ p, u64 len
   if ((rest & 1) && first) a[rest - 1] = lr(a[rest - 1]);
 }
 
-// Jobs of up to 2^11 words: one block per job (grid-stride over the jobs),
-// blockDim sized to the job; longer jobs take k_lift_stream below.
-static constexpr int kLiftSmallLog = 11;
-
+// The epilogue of the simple kernels' jobs (n < 2^8, and to 2^14 when a pointer
+// is off the 32-byte grid): one block per job (grid-stride over the jobs),
+// blockDim sized to the job.  Every other path lifts in its last pass.
 template <class L>
 __device__ __forceinline__ void lift_segment(u64* __restrict__ out, long words, const L& lr) {
   if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
@@ -611,81 +610,6 @@ __global__ void __launch_bounds__(256) k_lift_jobs(const vkcu_ntt_job* __restric
     const vkcu_ntt_job job = fetch_job(jobs, one, w);
     const LiftRun lr(&lift, load_tw(job.tw).q);
     lift_segment(reinterpret_cast<u64*>(job.out), 1L << log_n, lr);
-  }
-}
-
-// Long jobs (n >= 2^12), up to kLiftStreamJobs per launch: the jobs' words
-// laid end to end are walked in 128-word warp chunks, chunk c by warp c mod W
-// (W warps in the grid), so that the whole grid streams through adjacent
-// memory at any time (a block per contiguous range, 608 blocks reading from
-// 608 places, reached 0.71 of HBM against 0.91 so on 32 jobs of 2^20
-// words); each job's output pointer and step constants are staged in shared
-// memory once per block.  Two pairs per lane per chunk, the next chunk's
-// loads issued before this chunk is lifted; word by word when an output is
-// off the 16-byte grid.
-static constexpr int kLiftStreamJobs = 256;
-
-__global__ void __launch_bounds__(256) k_lift_stream(const vkcu_ntt_job* __restrict__ jobs, int njobs,
-                                                     vkcu_ntt_job one, int log_n,
-                                                     const __grid_constant__ vkcu_lift lift) {
-  __shared__ u64 s_out[kLiftStreamJobs];
-  __shared__ u64 s_c[kLiftStreamJobs][2 * VKCU_MAX_LIFT];
-  __shared__ int s_unaligned;
-  if (threadIdx.x == 0) s_unaligned = 0;
-  __syncthreads();
-  for (int j = threadIdx.x; j < njobs; j += blockDim.x) {
-    const vkcu_ntt_job job = fetch_job(jobs, one, j);
-    const LiftRun lr(&lift, load_tw(job.tw).q);
-    s_out[j] = reinterpret_cast<u64>(job.out);
-    if (s_out[j] & 15) atomicOr(&s_unaligned, 1);
-#pragma unroll
-    for (int k = 0; k < VKCU_MAX_LIFT; k++) {
-      s_c[j][k] = lr.bound[k];
-      s_c[j][VKCU_MAX_LIFT + k] = lr.d[k];
-    }
-  }
-  __syncthreads();
-  const int cl = log_n - 7;  // log2 of the chunks of a job
-  const long chunks = (long)njobs << cl;
-  const long nw = (long)gridDim.x * (blockDim.x >> 5);
-  const int lane = threadIdx.x & 31;
-  auto base = [&](long c) {
-    return reinterpret_cast<u64*>(s_out[c >> cl]) + ((c & ((1L << cl) - 1)) << 7) + 2 * lane;
-  };
-  long c = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (s_unaligned) {  // an output off the 16-byte grid: word by word
-    for (; c < chunks; c += nw) {
-      u64* pw = base(c);
-      const u64* cj = s_c[c >> cl];
-      const LiftRun lr(&lift, cj, cj + VKCU_MAX_LIFT);
-      pw[0] = lr(pw[0]);
-      pw[1] = lr(pw[1]);
-      pw[64] = lr(pw[64]);
-      pw[65] = lr(pw[65]);
-    }
-    return;
-  }
-  if (c >= chunks) return;
-  u64* p = base(c);
-  ulonglong2 x0 = ld2(p), x1 = ld2(p + 64);
-  for (; c < chunks; c += nw) {
-    const long cn = c + nw;
-    u64* pn = p;
-    ulonglong2 y0 = x0, y1 = x1;
-    if (cn < chunks) {
-      pn = base(cn);
-      y0 = ld2(pn);
-      y1 = ld2(pn + 64);
-    }
-    const u64* cj = s_c[c >> cl];
-    const LiftRun lr(&lift, cj, cj + VKCU_MAX_LIFT);
-    u64 v[4] = {x0.x, x0.y, x1.x, x1.y};
-    lr.apply(v);
-    st2(p, v[0], v[1]);
-    st2(p + 64, v[2], v[3]);
-    p = pn;
-    x0 = y0;
-    x1 = y1;
   }
 }
 
@@ -715,27 +639,13 @@ extern "C" int vkcu_lift_jobs(void* stream, const vkcu_ntt_job* jobs, int njobs,
   if (!has_lift(lift)) return 0;
   if (njobs < 1 || log_n > (uint32_t)kMaxLogN || lift->count > VKCU_MAX_LIFT) return (int)cudaErrorInvalidValue;
   const vkcu_ntt_job o = one ? *one : vkcu_ntt_job{};
-  if ((int)log_n <= kLiftSmallLog) {  // one block per job, a thread per pair up to 256
-    const long pairs = (1L << log_n) / 2;
-    const int threads = pairs <= 32 ? 32 : pairs >= 256 ? 256 : (int)pairs;
-    const long cap = (long)(sms > 0 ? sms : 1) * 16;
-    const long blocks = njobs < cap ? njobs : cap;
-    k_lift_jobs<<<(unsigned)blocks, threads, 0, (cudaStream_t)stream>>>(jobs, njobs, o, (int)log_n, *lift);
-    vkcu_count_launches(1);
-    return (int)cudaGetLastError();
-  }
-  // long jobs: one streaming launch per kLiftStreamJobs jobs (a single job by value: one)
-  for (int g = 0; g < njobs; g += kLiftStreamJobs) {
-    const int cnt = njobs - g < kLiftStreamJobs ? njobs - g : kLiftStreamJobs;
-    long blocks = (((long)cnt << log_n) + 1023) / 1024;
-    const long cap = resident_blocks<k_lift_stream>(sms);
-    if (blocks > cap) blocks = cap;
-    k_lift_stream<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(jobs ? jobs + g : nullptr, cnt, o, (int)log_n,
-                                                                     *lift);
-    vkcu_count_launches(1);
-    if (const int e = (int)cudaGetLastError()) return e;
-  }
-  return 0;
+  const long pairs = (1L << log_n) / 2;  // a thread per pair up to 256
+  const int threads = pairs <= 32 ? 32 : pairs >= 256 ? 256 : (int)pairs;
+  const long cap = (long)(sms > 0 ? sms : 1) * 16;
+  const long blocks = njobs < cap ? njobs : cap;
+  k_lift_jobs<<<(unsigned)blocks, threads, 0, (cudaStream_t)stream>>>(jobs, njobs, o, (int)log_n, *lift);
+  vkcu_count_launches(1);
+  return (int)cudaGetLastError();
 }
 
 // Pointwise step of a composed polymul: c = c * scratch mod q over njobs

@@ -9,7 +9,9 @@
 //                             runs the radix-C network in registers and writes
 //                             output j of every column into CTA j's shared
 //                             memory (DSMEM);
-//             row passes   -- each CTA then runs the remaining 14 stages on its
+//                             (and the sub-block's first pass with them where
+//                             both fit one radix-16 group: Cols below);
+//             row passes   -- each CTA then runs the remaining stages on its
 //                             own 2^14-word sub-block, which is the contiguous
 //                             words [r 2^14, (r+1) 2^14) of the bit-reversed
 //                             output; the twiddle of local stage m' and local
@@ -19,8 +21,12 @@
 //             stages with n^-1 folded in, writing global memory coalesced.
 //
 // The sub-block is 2^14 words (n = 2^15 .. 2^17, one CTA per SM), or 2^9 ..
-// 2^13 words for n = 2^12 .. 2^16 split over 8 CTAs when there are too few
-// jobs to fill the GPU otherwise (single calls, small server micro-batches).
+// 2^13 words for n = 2^12 .. 2^17 split over 2 .. 16 CTAs when there are too
+// few jobs to fill the GPU otherwise (single calls, small batches, server
+// micro-batches, the jobs past a batch's whole rounds: split_log and Tail in
+// ntt.cu).  Past one cluster (n >= 2^18, and few jobs of 2^17) the same kernels
+// run the sub-blocks that the global passes leave (SUB: 2^16 words on 4 CTAs,
+// or 2^14 on 8).
 //
 // Cluster barriers separate the phases: before a forward column pass writes
 // another CTA's shared memory (its owner has finished reading it; in the
