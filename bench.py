@@ -991,7 +991,7 @@ def main():
     int_ach_eff = modmuls / (eff_ms * 1e-3) / 1e9
     roofline = {"bound": "int", "achieved": int_ach, "peak": bfly_peak / 1e9, "unit": "Gmodmul/s",
                 "frac": int_ach / (bfly_peak / 1e9), "traffic": traffic,
-                "kernel": "k_polymul<14,32,1>", "launch_ms": kernel_ms,
+                "kernel": "k_polymul<14> (whole rounds), k_polymul_cluster<2> (the jobs past them)", "launch_ms": kernel_ms,
                 "launch_ms_source": "mean CUDA-event duration of isolated launches (one stream)",
                 "modmuls_per_launch": modmuls,
                 "modmuls_per_unit": "3 (n/2) log2 n + n per limb product (n/2 log2 n Shoup products per "
@@ -1123,7 +1123,7 @@ def main():
         "config": CONFIG,
         "setup": {"primes": [str(q) for q in qs],
                   "l2": f"{ROTATE} input batches rotate (4 x 96 MB > 129 MB L2); no flush needed",
-                  "launch": "one fused persistent kernel per step (CUDA graph replay); consecutive steps "
+                  "launch": "two fused kernels per step, whole rounds and the jobs past them (CUDA graph replay); consecutive steps "
                             "alternate between two streams and overlap",
                   "timing": f"blocks of {args.steps} steps repeated for >= {MIN_TIMED_S} s "
                             f"({len(block_ms)} blocks); ms_per_step from the median block",
