@@ -503,6 +503,9 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 	for (uint32_t i = 0; i < b->njobs; i++) {
 		struct job_rec *r = &b->recs[i];
 		r->extra_scratch = 0;
+		/* where a commit that failed may have pointed it, that memory is gone */
+		if (r->kind == VKH_JOB_POLYMUL)
+			r->job.scratch = r->b_ntt ? (uint64_t *) r->job.b : r->job.c;
 		if (b->nclasses == 0 || b->classes[b->nclasses - 1].kind != r->kind ||
 				b->classes[b->nclasses - 1].log_n != r->log_n || b->classes[b->nclasses - 1].qclass != (int) r->qclass ||
 				b->classes[b->nclasses - 1].lift != r->lift || b->classes[b->nclasses - 1].b_ntt != r->b_ntt) {
