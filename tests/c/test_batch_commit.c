@@ -238,6 +238,24 @@ static void retry_with_other_tuning(void) {
 	CHECK(fused_launches == 1 && composed_launches == 0);
 }
 
+/* Room for the passes' scratch or the job table, not both: the batch runs fused. */
+static void no_room_beside_the_table(void) {
+	mem_limit = used + N * sizeof(uint64_t) + 64;
+	CHECK(vkhel_batch_commit(bt, VKHEL_BATCH_GRAPH) == VKHEL_OK);
+	CHECK(fused_launches == 1 && composed_launches == 0);
+}
+
+/* What a budget leaves beside the job table stays free for later vectors. */
+static void budget_for_a_later_vector(void) {
+	const uint64_t before = vkhel_ctx_bytes_in_use(ctx);
+	CHECK(vkhel_ctx_set_budget(ctx, before + N * sizeof(uint64_t) + 4096) == VKHEL_OK);
+	CHECK(vkhel_batch_commit(bt, VKHEL_BATCH_GRAPH) == VKHEL_OK);
+	struct vkhel_vector *v = vkhel_vector_create2(ctx, N, true);
+	CHECK(v != NULL);
+	vkhel_vector_destroy(v);
+	CHECK(fused_launches == 1 && composed_launches == 0);
+}
+
 static void composed_where_there_is_room(void) {
 	CHECK(vkhel_batch_commit(bt, VKHEL_BATCH_GRAPH) == VKHEL_OK);
 	CHECK(fused_launches == 0 && composed_launches == 1);
@@ -250,6 +268,8 @@ int main(int argc, char **argv) {
 	} scenarios[] = {
 		{"retry_without_scratch", retry_without_scratch},
 		{"retry_with_other_tuning", retry_with_other_tuning},
+		{"no_room_beside_the_table", no_room_beside_the_table},
+		{"budget_for_a_later_vector", budget_for_a_later_vector},
 		{"composed_where_there_is_room", composed_where_there_is_room},
 	};
 	if (argc != 4)

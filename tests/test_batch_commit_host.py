@@ -23,7 +23,8 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["composed_where_there_is_room", "retry_without_scratch",
-                                      "retry_with_other_tuning"])
+                                      "retry_with_other_tuning",
+                                      "no_room_beside_the_table", "budget_for_a_later_vector"])
 def test_batch_commit(program, scenario):
     n = 1 << 17
     q = workloads.ntt_primes(n, 1)[0]

@@ -48,8 +48,10 @@ struct vkhel_batch {
 	uint32_t nclasses;
 	void *dev;             /* poly jobs, then 3 ntt-job arrays per composed class */
 	uint64_t dev_bytes;
-	void *scratch;
+	void *scratch;         /* slices the products cannot do without */
 	uint64_t scratch_bytes;
+	void *extra;           /* slices of extra_scratch */
+	uint64_t extra_bytes;
 	vkcu_poly_job *dev_poly;
 	vkcu_ntt_job *dev_ntt; /* [3 * njobs]: b->scratch, a->c, c->c */
 	void *graph;
@@ -470,6 +472,43 @@ static int ragged_setup(struct vkhel_batch *b) {
 	return VKHEL_OK;
 }
 
+/* Classes that run faster composed than fused (vkcu_few_composed; not under
+ * tuning entry (3, 2), which asks for as few launches as possible): those with
+ * NTT(b) given or scratch of their own as they are, the others where n words a
+ * product can be had.  A batch keeps them for its life, so a context with a
+ * budget gives none: its later vectors must fit as they did without. */
+static void compose_few(struct vkhel_batch *b) {
+	struct vkhel_ctx *ctx = b->ctx;
+	if (vkh_variant(3, 2) == 1)
+		return;
+	uint64_t work = 0, words = 0, class_words[MAX_CLASSES];
+	int few[MAX_CLASSES];
+	for (uint32_t k = 0; k < b->nclasses; k++)
+		work += class_work(&b->classes[k]);
+	for (uint32_t k = 0; k < b->nclasses; k++) {
+		const struct vkh_job_class *cl = &b->classes[k];
+		const int avail = vkh_variant(3, 0) == 1 ? (int) (class_work(cl) * ctx->sms / work) : ctx->sms;
+		few[k] = cl->kind == VKH_JOB_POLYMUL && cl->fused &&
+				vkcu_few_composed(cl->count, cl->log_n, cl->qclass, avail);
+		class_words[k] = 0;
+		for (uint32_t i = cl->first; few[k] && !cl->b_ntt && i < cl->first + cl->count; i++)
+			if (!b->recs[i].needs_scratch)
+				class_words[k] += slice_words(cl->log_n);
+		words += class_words[k];
+	}
+	const int room = words && !ctx->budget && vkh_dev_try_alloc(ctx, words * sizeof(uint64_t), &b->extra);
+	if (room)
+		b->extra_bytes = words * sizeof(uint64_t);
+	for (uint32_t k = 0; k < b->nclasses; k++) {
+		struct vkh_job_class *cl = &b->classes[k];
+		if (!few[k] || (class_words[k] && !room))
+			continue;
+		cl->fused = 0;
+		for (uint32_t i = cl->first; class_words[k] && i < cl->first + cl->count; i++)
+			b->recs[i].extra_scratch = !b->recs[i].needs_scratch;
+	}
+}
+
 int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 	if (!b)
 		return vkh_fail(NULL, VKHEL_ERR_INVALID_ARGUMENT, "batch_commit: NULL batch");
@@ -490,8 +529,9 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 	b->fork = NULL;
 	vkh_dev_free(ctx, b->dev, b->dev_bytes);
 	vkh_dev_free(ctx, b->scratch, b->scratch_bytes);
-	b->dev = b->scratch = NULL;
-	b->dev_bytes = b->scratch_bytes = 0;
+	vkh_dev_free(ctx, b->extra, b->extra_bytes);
+	b->dev = b->scratch = b->extra = NULL;
+	b->dev_bytes = b->scratch_bytes = b->extra_bytes = 0;
 	qsort(b->recs, b->njobs, sizeof(*b->recs), cmp_rec);
 
 	/* classes and scratch slices; every slice starts on a 256-byte boundary:
@@ -532,49 +572,11 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 		if (r->needs_scratch)
 			scratch_words += slice_words(r->log_n);
 	}
-	/* classes that run faster composed, where their scratch can be had (not
-	 * under tuning entry (3, 2), which asks for as few launches as possible) */
-	uint64_t work = 0, extra_words = 0;
-	for (uint32_t k = 0; k < b->nclasses; k++)
-		work += class_work(&b->classes[k]);
-	for (int pass = vkh_variant(3, 2) == 1 ? 2 : 0; pass < 2; pass++) { /* 0: those with NTT(b) given and the words of the others, 1: the others */
-		for (uint32_t k = 0; k < b->nclasses; k++) {
-			struct vkh_job_class *cl = &b->classes[k];
-			const int avail = vkh_variant(3, 0) == 1 ? (int) (class_work(cl) * ctx->sms / work) : ctx->sms;
-			if (cl->kind != VKH_JOB_POLYMUL || !cl->fused ||
-					!vkcu_few_composed(cl->count, cl->log_n, cl->qclass, avail))
-				continue;
-			if (pass == 1 || cl->b_ntt)
-				cl->fused = 0;
-			for (uint32_t i = cl->first; !cl->b_ntt && i < cl->first + cl->count; i++) {
-				if (pass == 0 && !b->recs[i].needs_scratch)
-					extra_words += slice_words(cl->log_n);
-				b->recs[i].extra_scratch = pass == 1;
-			}
-		}
-		if (pass == 0 && extra_words) {
-			b->scratch_bytes = (scratch_words + extra_words) * sizeof(uint64_t);
-			if (!vkh_dev_try_alloc(ctx, b->scratch_bytes, &b->scratch)) {
-				b->scratch_bytes = 0;
-				break;
-			}
-		}
-	}
-	if (scratch_words && !b->scratch) {
+	if (scratch_words) {
 		b->scratch_bytes = scratch_words * sizeof(uint64_t);
-		int st = vkh_dev_alloc(ctx, b->scratch_bytes, &b->scratch);
-		if (st)
-			return st;
-	}
-	if (b->scratch) {
-		uint64_t off = 0;
-		for (uint32_t i = 0; i < b->njobs; i++) {
-			struct job_rec *r = &b->recs[i];
-			if (r->needs_scratch || r->extra_scratch) {
-				r->job.scratch = (uint64_t *) b->scratch + off;
-				off += slice_words(r->log_n);
-			}
-		}
+		const int sst = vkh_dev_alloc(ctx, b->scratch_bytes, &b->scratch);
+		if (sst)
+			return sst;
 	}
 
 	/* device job table: poly jobs, then per composed class 3 ntt-job arrays
@@ -582,6 +584,19 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 	const uint64_t poly_bytes = sizeof(vkcu_poly_job) * b->njobs;
 	const uint64_t ntt_off = (poly_bytes + 255) & ~(uint64_t) 255;
 	b->dev_bytes = ntt_off + sizeof(vkcu_ntt_job) * 3 * (uint64_t) b->njobs;
+	int st = vkh_dev_alloc(ctx, b->dev_bytes, &b->dev);
+	if (st)
+		return st;
+	compose_few(b); /* after the memory that the batch cannot do without */
+	uint64_t *needed = b->scratch, *extra = b->extra;
+	for (uint32_t i = 0; i < b->njobs; i++) {
+		struct job_rec *r = &b->recs[i];
+		uint64_t **from = r->needs_scratch ? &needed : r->extra_scratch ? &extra : NULL;
+		if (from) {
+			r->job.scratch = *from;
+			*from += slice_words(r->log_n);
+		}
+	}
 	void *host = calloc(1, b->dev_bytes);
 	if (!host)
 		return vkh_fail(ctx, VKHEL_ERR_OUT_OF_MEMORY, "batch_commit: host allocation failed");
@@ -590,11 +605,6 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 	for (uint32_t i = 0; i < b->njobs; i++)
 		hp[i] = b->recs[i].job;
 	vkh_fill_ntt_jobs(hp, hn, b->classes, b->nclasses);
-	int st = vkh_dev_alloc(ctx, b->dev_bytes, &b->dev);
-	if (st) {
-		free(host);
-		return st;
-	}
 	int e = vkcu_h2d(ctx->stream, b->dev, host, b->dev_bytes);
 	if (!e)
 		e = vkcu_sync(ctx->stream);
@@ -684,6 +694,7 @@ void vkhel_batch_destroy(struct vkhel_batch *b) {
 	vkcu_event_destroy(b->fork);
 	vkh_dev_free(ctx, b->dev, b->dev_bytes);
 	vkh_dev_free(ctx, b->scratch, b->scratch_bytes);
+	vkh_dev_free(ctx, b->extra, b->extra_bytes);
 	vkh_dev_free(ctx, b->ragged_dev, b->ragged_bytes);
 	free(b->recs);
 	free(b->lifts);
