@@ -383,34 +383,30 @@ def _op(name, *args):
     _check_ctx(ctx.ptr)
 
 
-# The transforms and element-wise calls take their arguments apart themselves
-# (the plain pattern of four calls at n = 4096 61 -> 55 us); what is no vector
-# or table goes through _op.
+# The transforms and element-wise calls take vectors and tables apart themselves
+# (the plain pattern of four calls at n = 4096 61 -> 55 us); a call with anything
+# else goes through _op, which unwraps those two types alone: the pointer of
+# another object (a batch, a server) must not reach a function that takes it for
+# a vector's.
 def _unary(name, a, res, *rest):
-    try:
-        ctx, pa, pr = a.ctx, a.ptr, res.ptr
-    except AttributeError:
+    if not (isinstance(a, Vector) and isinstance(res, Vector)):
         return _op(name, a, res, *rest)
-    getattr(lib(), name)(pa, pr, *rest)
-    _check_ctx(ctx.ptr)
+    getattr(lib(), name)(a.ptr, res.ptr, *rest)
+    _check_ctx(a.ctx.ptr)
 
 
 def _binary(name, a, b, res, *rest):
-    try:
-        ctx, pa, pb, pr = a.ctx, a.ptr, b.ptr, res.ptr
-    except AttributeError:
+    if not (isinstance(a, Vector) and isinstance(b, Vector) and isinstance(res, Vector)):
         return _op(name, a, b, res, *rest)
-    getattr(lib(), name)(pa, pb, pr, *rest)
-    _check_ctx(ctx.ptr)
+    getattr(lib(), name)(a.ptr, b.ptr, res.ptr, *rest)
+    _check_ctx(a.ctx.ptr)
 
 
 def _transform(name, a, res, tables):
-    try:
-        ctx, pa, pr, pt = a.ctx, a.ptr, res.ptr, tables.ptr
-    except AttributeError:
+    if not (isinstance(a, Vector) and isinstance(res, Vector) and isinstance(tables, NttTables)):
         return _op(name, a, res, tables)
-    getattr(lib(), name)(pa, pr, pt)
-    _check_ctx(ctx.ptr)
+    getattr(lib(), name)(a.ptr, res.ptr, tables.ptr)
+    _check_ctx(a.ctx.ptr)
 
 
 def elemfma(a, b, res, multiplier, mod): _binary("vkhel_vector_elemfma", a, b, res, int(multiplier), int(mod))
