@@ -694,21 +694,35 @@ static int polymul_impl(const struct vkhel_vector *a, const struct vkhel_vector 
 			return st;
 		scratch = tmp;
 	}
+	const int qclass = vkcu_qclass(t->q);
 	/* one product of the largest fused degree is faster in global passes and
 	 * sub-blocks over more SMs, which need a buffer for b's; without one (the
 	 * budget, a full device) the fused kernel does */
-	const int passes = vkcu_few_composed(1, t->log_n, vkcu_qclass(t->q), ctx->sms) &&
+	const int passes = vkcu_few_composed(1, t->log_n, qclass, ctx->sms) &&
 			(b_ntt || tmp || vkh_dev_try_alloc(ctx, bytes, &tmp));
 	if (tmp)
 		scratch = tmp;
 	int e;
 	if (fused && !passes) {
 		const vkcu_poly_job job = {a->dev, b->dev, res->dev, scratch, d->dev_set, b_ntt ? VKCU_JOB_B_NTT : 0};
-		e = vkcu_polymul_lift(ctx->stream, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms, ctx->sms, lp, b_ntt);
-	} else {
+		e = vkcu_polymul_lift(ctx->stream, NULL, 1, &job, t->log_n, qclass, ctx->sms, ctx->sms, lp, b_ntt);
+	} else if (t->log_n >= vkcu_max_fused_log_n() && qclass != VKCU_Q63) {
 		const vkcu_poly_job job = {a->dev, b->dev, res->dev, scratch, d->dev_set, b_ntt ? VKCU_JOB_B_NTT : 0};
-		e = vkcu_polymul_composed(ctx->stream, NULL, NULL, NULL, NULL, 1, &job, t->log_n, vkcu_qclass(t->q), ctx->sms,
-				lp, b_ntt);
+		e = vkcu_polymul_composed(ctx->stream, NULL, NULL, NULL, NULL, 1, &job, t->log_n, qclass, ctx->sms, lp, b_ntt);
+	} else {
+		/* n < 2^8, and q >= 2^62 past one cluster; elemmul takes its constants by
+		 * value, where the batch's pointwise kernel fetches each job's (a call at
+		 * n = 2^7 29.3 us against 30.5) */
+		const vkcu_ntt_job jb = {b->dev, scratch, d->dev_set};
+		const vkcu_ntt_job ja = {a->dev, res->dev, d->dev_set};
+		const vkcu_ntt_job jc = {res->dev, res->dev, d->dev_set};
+		e = b_ntt ? 0 : vkcu_ntt_forward(ctx->stream, NULL, 1, &jb, t->log_n, qclass, ctx->sms, ctx->sms);
+		if (!e)
+			e = vkcu_ntt_forward(ctx->stream, NULL, 1, &ja, t->log_n, qclass, ctx->sms, ctx->sms);
+		if (!e)
+			e = vkcu_elemmul(ctx->stream, res->dev, res->dev, scratch, t->n, t->q, t->mu, t->qbits);
+		if (!e)
+			e = vkcu_ntt_inverse_lift(ctx->stream, NULL, 1, &jc, t->log_n, qclass, ctx->sms, ctx->sms, lp);
 	}
 	st = finish(ctx, e, "polymul");
 	if (tmp)

@@ -230,13 +230,13 @@ int vkcu_lift_jobs(void *stream, const vkcu_ntt_job *jobs, int njobs, const vkcu
  * outputs; the word the reference's elemmul stores): the pointwise step of a
  * polymul that is not fused. */
 int vkcu_pointwise(void *stream, const vkcu_poly_job *jobs, int njobs,
-		const vkcu_poly_job *one, uint32_t log_n, int qclass, int sms);
+		uint32_t log_n, int qclass, int sms);
 /* 1 where a class of products of a single-launch degree is faster through
  * vkcu_polymul_composed (few of the largest one): needs scratch for b. */
 int vkcu_few_composed(long njobs, uint32_t log_n, int qclass, int avail);
 /* Products outside the single-launch degrees, and those.  b, a and c are the jobs'
- * transforms b -> scratch, a -> c and c -> c (device arrays, or NULL with a
- * single job `one`). */
+ * transforms b -> scratch, a -> c and c -> c (device arrays, or, for 2^17 and
+ * more with q < 2^62, NULL with a single job `one`). */
 int vkcu_polymul_composed(void *stream, const vkcu_poly_job *jobs, const vkcu_ntt_job *b,
 		const vkcu_ntt_job *a, const vkcu_ntt_job *c, int njobs, const vkcu_poly_job *one,
 		uint32_t log_n, int qclass, int sms, const vkcu_lift *lift, int b_ntt);

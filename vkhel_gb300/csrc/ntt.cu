@@ -546,11 +546,11 @@ extern "C" int vkcu_polymul_composed(void* stream, const vkcu_poly_job* jobs, co
     return polymul_large<Mod60>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
   if (log_n >= (uint32_t)kMaxCluster && qclass == VKCU_Q62)
     return polymul_large<Mod62>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
-  const vkcu_ntt_job ob{o.b, o.scratch, o.tw}, oa{o.a, o.c, o.tw}, oc{o.c, o.c, o.tw};
-  int e = b_ntt ? 0 : vkcu_ntt_forward(stream, b, njobs, &ob, log_n, qclass, sms, sms);
-  if (!e) e = vkcu_ntt_forward(stream, a, njobs, &oa, log_n, qclass, sms, sms);
-  if (!e) e = vkcu_pointwise(stream, jobs, njobs, one, log_n, qclass, sms);
-  if (!e) e = vkcu_ntt_inverse_lift(stream, c, njobs, &oc, log_n, qclass, sms, sms, lift);
+  if (!jobs) return (int)cudaErrorInvalidValue;  // single calls issue these four themselves
+  int e = b_ntt ? 0 : vkcu_ntt_forward(stream, b, njobs, nullptr, log_n, qclass, sms, sms);
+  if (!e) e = vkcu_ntt_forward(stream, a, njobs, nullptr, log_n, qclass, sms, sms);
+  if (!e) e = vkcu_pointwise(stream, jobs, njobs, log_n, qclass, sms);
+  if (!e) e = vkcu_ntt_inverse_lift(stream, c, njobs, nullptr, log_n, qclass, sms, sms, lift);
   return e;
 }
 
@@ -656,13 +656,13 @@ extern "C" int vkcu_lift_jobs(void* stream, const vkcu_ntt_job* jobs, int njobs,
 // thread two 16-byte pairs of c and of scratch per round, loads first.
 template <class M>
 __global__ void __launch_bounds__(256)
-    k_pointwise(const vkcu_poly_job* __restrict__ jobs, int njobs, vkcu_poly_job one, int log_n) {
+    k_pointwise(const vkcu_poly_job* __restrict__ jobs, int njobs, int log_n) {
   const int lw = log_n < 11 ? log_n : 11;  // log2 of the words of a chunk
   const long cpj = 1L << (log_n - lw);    // chunks per job
   const long total = (long)njobs * cpj;
   const int pairs = 1 << (lw - 1);         // n >= 2
   for (long ch = blockIdx.x; ch < total; ch += gridDim.x) {
-    const vkcu_poly_job job = fetch_job(jobs, one, (int)(ch >> (log_n - lw)));
+    const vkcu_poly_job job = jobs[ch >> (log_n - lw)];
     const Tw t = load_tw(job.tw);
     const long base = (ch & (cpj - 1)) << lw;
     u64* c = reinterpret_cast<u64*>(job.c) + base;
@@ -685,15 +685,13 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-extern "C" int vkcu_pointwise(void* stream, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job* one,
-                              uint32_t log_n, int qclass, int sms) {
-  if (njobs < 1 || (!jobs && !one) || log_n < 1) return (int)cudaErrorInvalidValue;
-  const vkcu_poly_job o = one ? *one : vkcu_poly_job{};
+extern "C" int vkcu_pointwise(void* stream, const vkcu_poly_job* jobs, int njobs, uint32_t log_n, int qclass, int sms) {
+  if (njobs < 1 || !jobs || log_n < 1) return (int)cudaErrorInvalidValue;
   const long chunks = (long)njobs << (log_n > 11 ? log_n - 11 : 0);
   long blocks = chunks;
   if (blocks > (long)sms * 8) blocks = (long)sms * 8;
   return by_class(qclass, [&](auto m) {
-    k_pointwise<decltype(m)><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(jobs, njobs, o, (int)log_n);
+    k_pointwise<decltype(m)><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(jobs, njobs, (int)log_n);
     vkcu_count_launches(1);
     return (int)cudaGetLastError();
   });
