@@ -20,7 +20,7 @@
 
 /* At most MAX_KINDS (kind, degree, q below 2^62 or not, epilogue, NTT(b)
  * given) combinations; each with q < 2^62 is one class or two (VKCU_Q60 and
- * VKCU_Q62). */
+ * VKCU_Q62, vkh_merge_classes). */
 #define MAX_KINDS 64
 #define MAX_CLASSES (2 * MAX_KINDS)
 
@@ -276,13 +276,48 @@ static int cmp_rec(const void *x, const void *y) {
 		return (a->kind > b->kind) - (a->kind < b->kind);
 	if (a->log_n != b->log_n)
 		return (a->log_n > b->log_n) - (a->log_n < b->log_n);
-	if (a->qclass != b->qclass)
+	if ((a->qclass == VKCU_Q63) != (b->qclass == VKCU_Q63))
 		return (a->qclass > b->qclass) - (a->qclass < b->qclass);
 	if (a->lift != b->lift)
 		return (a->lift > b->lift) - (a->lift < b->lift);
 	if (a->b_ntt != b->b_ntt)
 		return (a->b_ntt > b->b_ntt) - (a->b_ntt < b->b_ntt);
+	if (a->qclass != b->qclass) /* last, for vkh_merge_classes */
+		return (a->qclass > b->qclass) - (a->qclass < b->qclass);
 	return (a->order > b->order) - (a->order < b->order);
+}
+
+/* Classes on the two sides of 2^60 and alike otherwise. */
+static int same_but_prime(const struct vkh_job_class *a, const struct vkh_job_class *b) {
+	return a->kind == b->kind && a->log_n == b->log_n && a->lift == b->lift && a->b_ntt == b->b_ntt &&
+			a->qclass == VKCU_Q60 && b->qclass == VKCU_Q62;
+}
+
+/* The kernels of VKCU_Q62 take every modulus below 2^62.  Two launches, one per
+ * class, pay where the words with q < 2^60 are many enough for their faster
+ * butterflies to outweigh a launch and, at 2^13 .. 2^15, whose jobs take whole
+ * SMs, a partial round: from 3 2^18 such words on (2^18 below 2^8, 3 2^20 at
+ * 2^13 .. 2^15).  One launch / two, us, with half (an eighth) of the primes
+ * above 2^60: products of 2^10 x 300 16 / 24 (16 / 20), x 1000 35 / 34, x 4000
+ * 107 / 103 (108 / 94); 2^12 x 152 22 / 28 (22 / 25), x 500 72 / 62 (72 / 64);
+ * 2^14 x 12 25 / 30 (25 / 32), x 60 45 / 45 (45 / 104), x 200 122 / 138 (123 /
+ * 138), x 456 234 / 234 (232 / 247), x 1000 535 / 524 (533 / 462); 2^16 x 10
+ * 57 / 60, x 38 180 / 165; 2^17 x 9 68 / 76, x 18 190 / 166; 8000 of 2^5 31 /
+ * 31, 30000 86 / 70; transforms alike. */
+uint32_t vkh_merge_classes(struct vkh_job_class *classes, uint32_t nclasses, int always) {
+	uint32_t m = 0;
+	for (uint32_t k = 0; k < nclasses; k++) {
+		struct vkh_job_class *p = m ? &classes[m - 1] : NULL, *c = &classes[k];
+		const uint64_t words = p ? (uint64_t) p->count << p->log_n : 0;
+		const uint64_t many = (uint64_t) (c->log_n < 8 ? 1 : c->log_n >= 13 && c->log_n <= 15 ? 12 : 3) << 18;
+		if (p && same_but_prime(p, c) && (always || words < many)) {
+			p->qclass = c->qclass;
+			p->count += c->count;
+		} else {
+			classes[m++] = *c;
+		}
+	}
+	return m;
 }
 
 /* Launch the kernels of `nclasses` degree classes on `stream`: one fused
@@ -549,29 +584,18 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 		if (b->nclasses == 0 || b->classes[b->nclasses - 1].kind != r->kind ||
 				b->classes[b->nclasses - 1].log_n != r->log_n || b->classes[b->nclasses - 1].qclass != (int) r->qclass ||
 				b->classes[b->nclasses - 1].lift != r->lift || b->classes[b->nclasses - 1].b_ntt != r->b_ntt) {
-			int new_kind = 1;
-			for (uint32_t k = 0; r->qclass == VKCU_Q62 && k < b->nclasses; k++) {
-				const struct vkh_job_class *c = &b->classes[k];
-				if (c->kind == r->kind && c->log_n == r->log_n && c->qclass == VKCU_Q60 && c->lift == r->lift &&
-						c->b_ntt == r->b_ntt)
-					new_kind = 0;
-			}
-			if (new_kind && nkinds++ == MAX_KINDS)
+			const struct vkh_job_class c = {
+					.kind = r->kind, .log_n = r->log_n, .qclass = (int) r->qclass, .lift = r->lift, .b_ntt = r->b_ntt,
+					.first = i, .fused = r->log_n >= 8 && r->log_n <= vkcu_max_fused_log_n()};
+			if (!(b->nclasses && same_but_prime(&b->classes[b->nclasses - 1], &c)) && nkinds++ == MAX_KINDS)
 				return vkh_fail(ctx, VKHEL_ERR_UNSUPPORTED, "batch_commit: too many degree classes");
-			struct vkh_job_class *cl = &b->classes[b->nclasses++];
-			cl->kind = r->kind;
-			cl->log_n = r->log_n;
-			cl->qclass = (int) r->qclass;
-			cl->lift = r->lift;
-			cl->b_ntt = r->b_ntt;
-			cl->first = i;
-			cl->count = 0;
-			cl->fused = r->log_n >= 8 && r->log_n <= vkcu_max_fused_log_n();
+			b->classes[b->nclasses++] = c;
 		}
 		b->classes[b->nclasses - 1].count++;
 		if (r->needs_scratch)
 			scratch_words += slice_words(r->log_n);
 	}
+	b->nclasses = vkh_merge_classes(b->classes, b->nclasses, 0);
 	if (scratch_words) {
 		b->scratch_bytes = scratch_words * sizeof(uint64_t);
 		const int sst = vkh_dev_alloc(ctx, b->scratch_bytes, &b->scratch);

@@ -108,7 +108,7 @@ struct vkh_job_class {
 	uint32_t log_n;
 	uint32_t first, count;
 	int fused;
-	int qclass;            /* modulus class of every job, VKCU_Q60 .. VKCU_Q63 */
+	int qclass;            /* modulus class of its kernels (vkcu_qclass of the largest q) */
 	uint32_t lift;         /* index into the lift table, 0 = none */
 	uint32_t b_ntt;        /* polymul jobs whose b holds NTT(b) (VKCU_JOB_B_NTT) */
 };
@@ -119,6 +119,9 @@ int vkh_issue_classes(void *stream, int sms, int avail, const vkcu_poly_job *dev
 int vkh_issue_classes_forked(void *stream, void *const *aux, void *fork, void *const *join, int sms,
 		const vkcu_poly_job *dev_poly, const vkcu_ntt_job *dev_ntt, const struct vkh_job_class *classes,
 		uint32_t nclasses, const vkcu_lift *lifts);
+/* Joins classes that differ in VKCU_Q60 / VKCU_Q62 alone and follow one another,
+ * where one launch is faster than two (or always); returns how many are left. */
+uint32_t vkh_merge_classes(struct vkh_job_class *classes, uint32_t nclasses, int always);
 void vkh_fill_ntt_jobs(const vkcu_poly_job *poly, vkcu_ntt_job *ntt, const struct vkh_job_class *classes,
 		uint32_t nclasses);
 /* tuning.c -- variant of kernel family (VKHEL_TUNE_*) for degree 2^log_n */

@@ -149,6 +149,10 @@ static uint64_t req_bytes(const struct srv_req *r) {
 /* Host bytes a request uploads per limb word: a and b, or a alone. */
 static uint64_t up_per_word(const struct srv_req *r) { return r->op ? 8 : 16; }
 
+/* Sort keys of a chunk's jobs: degree, q >= 2^62, resident operand, q >= 2^60,
+ * job index (classes that vkh_merge_classes can join stand side by side). */
+#define KEY_Q63 ((uint64_t) 1 << 39)
+#define KEY_Q62 ((uint64_t) 1 << 37)
 static int cmp_job_log_n(const void *x, const void *y) {
 	const uint64_t a = *(const uint64_t *) x, b = *(const uint64_t *) y;
 	return (a > b) - (a < b);
@@ -203,8 +207,8 @@ static int issue_chunk(struct vkhel_server *s, struct srv_slot *sl, uint32_t c, 
 	qsort(keys + j0, j1 - j0, sizeof(uint64_t), cmp_job_log_n);
 	for (uint32_t i = j0; i < j1; i++) {
 		const uint32_t log_n = (uint32_t) (keys[i] >> 40);
-		const int qclass = (int) ((keys[i] >> 38) & 3);
-		const uint32_t b_ntt = (uint32_t) ((keys[i] >> 37) & 1);
+		const uint32_t b_ntt = (uint32_t) ((keys[i] >> 38) & 1);
+		const int qclass = keys[i] & KEY_Q63 ? VKCU_Q63 : keys[i] & KEY_Q62 ? VKCU_Q62 : VKCU_Q60;
 		sl->host_poly[i] = tmp[keys[i] & 0x1fffffffffull];
 		if (nclasses == 0 || classes[nclasses - 1].log_n != log_n || classes[nclasses - 1].qclass != qclass ||
 				classes[nclasses - 1].b_ntt != b_ntt) {
@@ -222,6 +226,7 @@ static int issue_chunk(struct vkhel_server *s, struct srv_slot *sl, uint32_t c, 
 		}
 		classes[nclasses - 1].count++;
 	}
+	nclasses = vkh_merge_classes(classes, nclasses, 0);
 	vkh_fill_ntt_jobs(sl->host_poly, sl->host_ntt, classes, nclasses);
 	vkcu_poly_job *dpoly = sl->dev_jobs;
 	vkcu_ntt_job *dntt = (vkcu_ntt_job *) ((char *) sl->dev_jobs + sizeof(vkcu_poly_job) * cap);
@@ -295,8 +300,9 @@ static void launch_slot(struct vkhel_server *s, struct srv_slot *sl) {
 				j.scratch = fused ? j.c : base + 3 * words + (uint64_t) k * r->n;
 			}
 			j.tw = d->dev_set;
-			keys[njobs] = ((uint64_t) r->log_n << 40) | ((uint64_t) vkcu_qclass(r->tables[k]->q) << 38) |
-					((uint64_t) (r->op != NULL) << 37) | njobs;
+			const int qclass = vkcu_qclass(r->tables[k]->q);
+			keys[njobs] = ((uint64_t) r->log_n << 40) | (qclass == VKCU_Q63 ? KEY_Q63 : 0) |
+					((uint64_t) (r->op != NULL) << 38) | (qclass == VKCU_Q62 ? KEY_Q62 : 0) | njobs;
 			tmp[njobs++] = j;
 			acc += up_per_word(r) * r->n;
 			const int last = i + 1 == sl->nreqs && k + 1 == r->limbs;
