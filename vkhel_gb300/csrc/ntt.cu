@@ -261,17 +261,44 @@ static int inverse_passes(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, 
   return 0;
 }
 
-// log2 of the sub-blocks per transform of 2^log_n > 2^17 words: 2^16-word
-// sub-blocks on clusters of 4 CTAs (one radix-16 global pass at 2^20, and four
-// radix-16 passes inside), or 2^14-word ones on clusters of 8 small CTAs where
-// the former would leave half of the SMs idle.  Products, 4-CTA / 8-CTA: 1 of
-// 2^18 (4 sub-blocks of 2^16) 86 / 37 us, 4 of 2^18 (16) 94 / 66 us, 9 of 2^18
-// (36) 108 / 128 us, 15 of 2^20 (240) 722 / 907 us; forward transforms and
-// products on CTA-resident 2^14-word sub-blocks and more global passes before:
-// 90, 99, 121 and 885 us.
-static int sub_log_of(int njobs, int log_n, int sms) {
-  return log_n > 17 && ((long)njobs << (log_n - 16)) * 8 > (long)sms ? log_n - 16 : log_n - 14;
-}
+// log2 of the sub-blocks per transform of 2^log_n >= 2^17 words, and whether each
+// is one CTA's:
+//   * few: 2^14 words on clusters of 8 small CTAs, where 2^16-word sub-blocks
+//     would leave half of the SMs idle.  Products, 4-CTA / 8-CTA: 1 of 2^18 (4
+//     sub-blocks of 2^16) 86 / 37 us, 4 of 2^18 (16) 94 / 66 us, 9 of 2^18 (36)
+//     108 / 128 us, 15 of 2^20 (240) 722 / 907 us;
+//   * 2^16 words on clusters of 4 CTAs: two stages less above them, one pass over
+//     HBM less for it at most degrees, and a product's sub-blocks in one launch;
+//   * 2^14 words on one CTA (products: both transforms, the pointwise kernel and
+//     the inverse): no room lost between clusters -- 36 of 4 CTAs fit 152 SMs --
+//     and rounds of 38 in their place.
+// Transforms take the last where it adds no pass over HBM or saves one round in
+// eight, products where it saves one in five, which outweighs three more
+// launches over HBM.  4-CTA clusters / CTAs, us,
+// q < 2^60: 19 x 2^18 (3 rounds / 2) forward 95 / 66, inverse 96 / 68, product
+// 272 / 212; 18 x 2^18 (2 / 2) 70 / 64, 70 / 66, 196 / 209; 7 x 2^20 (4 / 3) 135
+// / 105, 141 / 118, 394 / 345; 13 x 2^20 (6 / 6) 215 / 208, 225 / 227, 615 /
+// 685; 14 x 2^20 (7 / 6) 244 / 214, 253 / 234, 696 / 710; 4 x 2^21 (4 / 4) 156
+// / 144, 164 / 165, 442 / 473; 2 x 2^24 (15 / 14) 632 / 618, 684 / 711, 1800 /
+// 2062; q in [2^60, 2^62): 19 x 2^18 105 / 72, 109 / 76,
+// 310 / 232; 7 x 2^20 150 / 117, 161 / 129, 454 / 380.
+struct Subs {
+  int log = 0;
+  bool cta = false;
+  Subs(int njobs, int log_n, int sms, bool product) {
+    const long subs = log_n < 18 ? 0 : (long)njobs << (log_n - 16);  // of 2^16 words
+    if (subs * 8 <= sms) {
+      log = log_n - 14;
+      return;
+    }
+    const long clusters = sms * 9L / 38, ctas = sms / 4;
+    const long rounds = (subs + clusters - 1) / clusters, cta_rounds = (subs + ctas - 1) / ctas;
+    const bool no_more_passes = log_n == 18 || log_n == 21;  // 2 or 5 stages above 2^16 words, 4 or 7 above 2^14
+    const long saved = rounds - cta_rounds;
+    cta = product ? saved * 5 >= rounds : saved * 8 >= rounds || no_more_passes;
+    log = log_n - (cta ? 14 : 16);
+  }
+};
 
 }  // namespace vk
 
@@ -394,9 +421,10 @@ static int forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
     const int e = forward_passes<M>(st, jobs, njobs, o, (int)log_n, GlobalPlan{sub_log}, sms);
     return e ? e : fwd_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms);
   } else {
-    const int sub_log = sub_log_of(njobs, (int)log_n, sms);
-    const int e = forward_passes<M>(st, jobs, njobs, o, (int)log_n, GlobalPlan{sub_log}, sms);
-    return e ? e : fwd_cluster_sub<M>(st, jobs, njobs, o, (int)log_n, sub_log);
+    const Subs subs(njobs, (int)log_n, sms, false);
+    if (const int e = forward_passes<M>(st, jobs, njobs, o, (int)log_n, GlobalPlan{subs.log}, sms)) return e;
+    return subs.cta ? fwd_cta_sub<M>(st, jobs, njobs, o, subs.log, sms)
+                    : fwd_cluster_sub<M>(st, jobs, njobs, o, (int)log_n, subs.log);
   }
 }
 
@@ -449,8 +477,10 @@ static int inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
       sub_log = (int)log_n - kMaxCta;
       e = inv_cta_wide(st, jobs, njobs, o, kMaxCta, sub_log, sms, nullptr);
     } else {
-      sub_log = sub_log_of(njobs, (int)log_n, sms);
-      e = inv_cluster_sub<M>(st, jobs, njobs, o, (int)log_n, sub_log);
+      const Subs subs(njobs, (int)log_n, sms, false);
+      sub_log = subs.log;
+      e = subs.cta ? inv_cta_sub<M>(st, jobs, njobs, o, sub_log, sms)
+                   : inv_cluster_sub<M>(st, jobs, njobs, o, (int)log_n, sub_log);
     }
     return e ? e : inverse_passes<M>(st, jobs, njobs, o, (int)log_n, GlobalPlan{sub_log}, sms, 0, lp);
   }
@@ -465,7 +495,7 @@ extern "C" int vkcu_ntt_inverse_lift(void* stream, const vkcu_ntt_job* jobs, int
                   [&](auto m) { return inverse<decltype(m)>(stream, jobs, njobs, one, log_n, sms, avail, lift); });
 }
 
-// A product of 2^17 .. 2^26, q < 2^62: the global passes of b
+// A product of 2^17 .. 2^26 in clusters, q < 2^62: the global passes of b
 // (into scratch) and of a (into c), one launch for every sub-block's forward,
 // product and inverse, the inverse global passes of c.  b, a and c give these
 // the jobs of the passes.
@@ -474,7 +504,7 @@ static int polymul_large(cudaStream_t st, const vkcu_poly_job* jobs, const vkcu_
                          const vkcu_ntt_job* c, int njobs, const vkcu_poly_job& one, int log_n, int sms,
                          const vkcu_lift* lift, int b_ntt) {
   const vkcu_ntt_job ob{one.b, one.scratch, one.tw}, oa{one.a, one.c, one.tw}, oc{one.c, one.c, one.tw};
-  const int sub_log = sub_log_of(njobs, log_n, sms);
+  const int sub_log = Subs(njobs, log_n, sms, true).log;
   const GlobalPlan plan{sub_log};
   int e = b_ntt ? 0 : forward_passes<M>(st, b, njobs, ob, log_n, plan, sms);
   if (!e) e = forward_passes<M>(st, a, njobs, oa, log_n, plan, sms);
@@ -524,8 +554,8 @@ extern "C" int vkcu_polymul(void* stream, const vkcu_poly_job* jobs, int njobs, 
 }
 
 // A product outside the single-launch degrees (or few of 2^17): as above; for
-// n < 2^8, and q >= 2^62 past one cluster, forward(b), forward(a), pointwise,
-// inverse.
+// n < 2^8, and past one cluster where each sub-block is one CTA's (Subs above,
+// q >= 2^62), forward(b), forward(a), pointwise, inverse.
 extern "C" int vkcu_few_composed(long njobs, uint32_t log_n, int qclass, int avail) {
   return qclass != VKCU_Q63 && few_of_17(njobs, log_n, avail);
 }
@@ -542,9 +572,10 @@ extern "C" int vkcu_polymul_composed(void* stream, const vkcu_poly_job* jobs, co
   const bool aligned =
       jobs != nullptr || (aligned32(o.a) && aligned32(o.b) && aligned32(o.c) && aligned32(o.scratch));
   if (log_n >= (uint32_t)kMaxCluster && !aligned) return (int)cudaErrorMisalignedAddress;
-  if (log_n >= (uint32_t)kMaxCluster && qclass == VKCU_Q60)
+  const bool clusters = log_n >= (uint32_t)kMaxCluster && !(jobs && Subs(njobs, (int)log_n, sms, true).cta);
+  if (clusters && qclass == VKCU_Q60)
     return polymul_large<Mod60>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
-  if (log_n >= (uint32_t)kMaxCluster && qclass == VKCU_Q62)
+  if (clusters && qclass == VKCU_Q62)
     return polymul_large<Mod62>(st, jobs, b, a, c, njobs, o, (int)log_n, sms, lp, b_ntt);
   if (!jobs) return (int)cudaErrorInvalidValue;  // single calls issue these four themselves
   int e = b_ntt ? 0 : vkcu_ntt_forward(stream, b, njobs, nullptr, log_n, qclass, sms, sms);

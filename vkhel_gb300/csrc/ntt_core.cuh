@@ -1251,6 +1251,13 @@ template <class M>
 int poly_cluster(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int logc, int logs,
                  const vkcu_lift* lift = nullptr);
 
+// The 2^sub_log sub-blocks of 2^14 words of transforms past one cluster, each on
+// one CTA, between their global passes (in place in out).
+template <class M>
+int fwd_cta_sub(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int sub_log, int sms);
+template <class M>
+int inv_cta_sub(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int sub_log, int sms);
+
 // The sub-blocks of 2^(log_n - sub_log) words of transforms and products past
 // one cluster, between their global passes (in place in out, or from c and
 // scratch to c): 2^16 words on 4 CTAs, or 2^14 words on 8.

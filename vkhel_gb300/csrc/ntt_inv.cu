@@ -4,5 +4,6 @@
 namespace vk {
 
 template int inv_cta<Mod60>(cudaStream_t, const vkcu_ntt_job*, int, const vkcu_ntt_job&, int, int, int);
+template int inv_cta_sub<Mod60>(cudaStream_t, const vkcu_ntt_job*, int, const vkcu_ntt_job&, int, int);
 
 }  // namespace vk

@@ -36,6 +36,19 @@ int inv_cta_lift(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkc
 }
 
 template <class M>
+int fwd_cta_sub(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int sub_log, int sms) {
+  return launch_cta<Shape<14, 32, 1, M>, k_ntt_fwd<14, 32, 1, M, true>>(st, (long)njobs << sub_log, sms, jobs, njobs,
+                                                                        one, sub_log);
+}
+
+template <class M>
+int inv_cta_sub(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int sub_log, int sms) {
+  const vkcu_lift none{};
+  return launch_cta<Shape<14, 32, 1, M>, k_ntt_inv<14, 32, 1, false, M, true>>(st, (long)njobs << sub_log, sms, jobs,
+                                                                               njobs, one, sub_log, none);
+}
+
+template <class M>
 int poly_cta(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int log_n, int sms,
              int variant) {
   const vkcu_lift none{};

@@ -4,5 +4,6 @@
 namespace vk {
 
 template int fwd_cta<Mod62>(cudaStream_t, const vkcu_ntt_job*, int, const vkcu_ntt_job&, int, int, int);
+template int fwd_cta_sub<Mod62>(cudaStream_t, const vkcu_ntt_job*, int, const vkcu_ntt_job&, int, int);
 
 }  // namespace vk
