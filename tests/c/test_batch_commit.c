@@ -157,7 +157,7 @@ int vkcu_ntt_inverse_lift(void *stream, const vkcu_ntt_job *jobs, int njobs, con
 	return 0;
 }
 int vkcu_polymul_ragged(void *stream, const vkcu_ragged_item *items, int n_cluster_items, int n_items,
-		const vkcu_poly_job *jobs, unsigned *counters, int sms) {
+		const vkcu_poly_job *jobs, unsigned *counters, int qclass) {
 	return 0;
 }
 uint32_t vkcu_max_fused_log_n(void) { return 17; }

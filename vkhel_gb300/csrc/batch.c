@@ -59,7 +59,7 @@ struct vkhel_batch {
 	/* a ragged batch as one launch (tuning family 3, log_n 2): item table,
 	 * job copies (plus a dummy copy for an odd pair), two counters and the
 	 * dummy products' output, in one device allocation */
-	int ragged;
+	int ragged, ragged_qclass;
 	uint32_t n_cluster_items, n_items;
 	void *ragged_dev;
 	uint64_t ragged_bytes;
@@ -415,7 +415,7 @@ static int issue(struct vkhel_batch *b) {
 		const uint64_t jobs_bytes = (sizeof(vkcu_poly_job) * (b->njobs + 2) + 255) & ~(uint64_t) 255;
 		return vkcu_polymul_ragged(b->ctx->stream, (const vkcu_ragged_item *) base, (int) b->n_cluster_items,
 				(int) b->n_items, (const vkcu_poly_job *) (base + items_bytes),
-				(unsigned *) (base + items_bytes + jobs_bytes), b->ctx->sms);
+				(unsigned *) (base + items_bytes + jobs_bytes), b->ragged_qclass);
 	}
 	if (b->naux)
 		return vkh_issue_classes_forked(b->ctx->stream, b->aux, b->fork, b->join, b->ctx->sms, b->dev_poly,
@@ -426,11 +426,12 @@ static int issue(struct vkhel_batch *b) {
 
 /* The single-launch form of a ragged batch (ntt_ragged.cu) when the tuning
  * table asks for it and every class is a fused product of degree 2^12 ..
- * 2^16 with q < 2^60 and no epilogue: items in decreasing size, 2^15 and
+ * 2^16 with q < 2^62 and no epilogue: items in decreasing size, 2^15 and
  * 2^12 products in pairs, an odd pair completed by a copy of its product
  * that writes a dummy buffer. */
 static int ragged_setup(struct vkhel_batch *b) {
 	b->ragged = 0;
+	b->ragged_qclass = VKCU_Q60;
 	if (b->ragged_dev) { /* a commit that failed after this step is being retried */
 		vkh_dev_free(b->ctx, b->ragged_dev, b->ragged_bytes);
 		b->ragged_dev = NULL;
@@ -441,9 +442,11 @@ static int ragged_setup(struct vkhel_batch *b) {
 	uint32_t first[17] = {0}, count[17] = {0};
 	for (uint32_t k = 0; k < b->nclasses; k++) {
 		const struct vkh_job_class *cl = &b->classes[k];
-		if (cl->kind != VKH_JOB_POLYMUL || !cl->fused || cl->qclass != VKCU_Q60 || cl->lift || cl->b_ntt || cl->log_n < 12 ||
+		if (cl->kind != VKH_JOB_POLYMUL || !cl->fused || cl->qclass == VKCU_Q63 || cl->lift || cl->b_ntt || cl->log_n < 12 ||
 				cl->log_n > 16 || count[cl->log_n])
 			return VKHEL_OK;
+		if (cl->qclass > b->ragged_qclass)
+			b->ragged_qclass = cl->qclass;
 		first[cl->log_n] = cl->first;
 		count[cl->log_n] = cl->count;
 	}
@@ -595,7 +598,8 @@ int vkhel_batch_commit(struct vkhel_batch *b, uint32_t flags) {
 		if (r->needs_scratch)
 			scratch_words += slice_words(r->log_n);
 	}
-	b->nclasses = vkh_merge_classes(b->classes, b->nclasses, 0);
+	/* (one launch of a ragged batch takes one class per degree) */
+	b->nclasses = vkh_merge_classes(b->classes, b->nclasses, vkh_variant(3, 2) == 1);
 	if (scratch_words) {
 		b->scratch_bytes = scratch_words * sizeof(uint64_t);
 		const int sst = vkh_dev_alloc(ctx, b->scratch_bytes, &b->scratch);

@@ -245,13 +245,14 @@ int vkcu_polymul_composed(void *stream, const vkcu_poly_job *jobs, const vkcu_nt
  * n_cluster_items of kind 16 (one product of 2^16 on a cluster of four CTAs)
  * or 15 (two products of 2^15, one per CTA pair), then kinds 14 and 13 (one
  * product per CTA) and 12 (two products per CTA); job0 / job1 index `jobs`.
- * `counters` is two words of device memory the launch resets first. */
+ * `counters` is two words of device memory the launch resets first; `qclass`
+ * is VKCU_Q60 where every job is of it, VKCU_Q62 otherwise. */
 typedef struct vkcu_ragged_item {
 	uint32_t kind;
 	uint32_t job0, job1;
 } vkcu_ragged_item;
 int vkcu_polymul_ragged(void *stream, const vkcu_ragged_item *items, int n_cluster_items,
-		int n_items, const vkcu_poly_job *jobs, unsigned *counters, int sms);
+		int n_items, const vkcu_poly_job *jobs, unsigned *counters, int qclass);
 
 /* Kernel variant table (tuning.c): family 0 = fused polymul, 1 = forward,
  * 2 = inverse, 3 = batch options (log_n 0: concurrent degree classes, 1:
