@@ -13,9 +13,41 @@ namespace vk {
 // ---------------------------------------------------------------------------
 // Simple kernels: one CTA per job, whole vector in shared memory, one
 // radix-2 stage per __syncthreads.  Used for n < 256, for n <= 2^14 when a
-// pointer is not 32-byte aligned, and as an independent cross-check.
+// pointer is not 32-byte aligned, and as an independent cross-check.  Latency
+// bounds them: a few loads and log2 n dependent butterflies.  So the products
+// are plain C, whose four multiplies run side by side where the throughput
+// kernels' chain of fused multiply-adds waits on itself; Mod62 serves q < 2^60
+// too, as its outputs need no constants beyond q; and below 2^8 a root's place
+// is its index.  With the throughput kernels' forms 8000 forward transforms of
+// 2^7 took 16.4 us and 100 products 16.4, now 14.4 and 14.4.
+__device__ __forceinline__ u64 shoup_lazy_short(u64 x, u64 w, u64 wp, u64 q) { return x * w - mulhi(x, wp) * q; }
 
-template <class M>
+struct Simple62 : Mod62 {
+  template <bool REDUCE>
+  __device__ __forceinline__ static void ct(u64& x, u64& y, u64 w, u64 wp, const Tw& t) {
+    const u64 xr = csub(x, t.q2), wy = shoup_lazy_short(y, w, wp, t.q);
+    x = xr + wy;
+    y = xr - wy + t.q2;
+  }
+  __device__ __forceinline__ static u64 mul(u64 d, u64 w, u64 wp, const Tw& t) {
+    return shoup_lazy_short(d, w, wp, t.q);
+  }
+};
+
+struct Simple63 : Mod63 {
+  template <bool REDUCE>
+  __device__ __forceinline__ static void ct(u64& x, u64& y, u64 w, u64 wp, const Tw& t) {
+    const u64 xr = csub(x, t.q), wy = csub(shoup_lazy_short(y, w, wp, t.q), t.q);
+    x = xr + wy;
+    y = xr - wy + t.q;
+  }
+  __device__ __forceinline__ static u64 mul(u64 d, u64 w, u64 wp, const Tw& t) {
+    return shoup_lazy_short(d, w, wp, t.q);
+  }
+};
+
+// ROWS: n >= 2^8, whose last roots stand in rows (vkcu_tw_slot).
+template <class M, bool ROWS>
 __global__ void k_ntt_fwd_simple(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one,
                                  int log_n) {
   extern __shared__ u64 sm[];
@@ -23,6 +55,7 @@ __global__ void k_ntt_fwd_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
   for (int w = blockIdx.x; w < njobs; w += gridDim.x) {
     const vkcu_ntt_job job = fetch_job(jobs, one, w);
     const Tw t = load_tw(job.tw);
+    const typename M::Out to(t);
     const u64* in = reinterpret_cast<const u64*>(job.in);
     for (int i = threadIdx.x; i < n; i += blockDim.x) sm[i] = in[i];
     __syncthreads();
@@ -31,7 +64,8 @@ __global__ void k_ntt_fwd_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
       for (int p = threadIdx.x; p < n / 2; p += blockDim.x) {
         const int blk = p >> (log_n - 1 - s);
         const int x = blk * 2 * half + (p & (half - 1));
-        const ulonglong2 wt = ld_tw(t.fwd + vkcu_tw_slot(log_n, (1u << s) + blk));
+        const ulonglong2 wt =
+            ld_tw(ROWS ? t.fwd + vkcu_tw_slot(log_n, (1u << s) + blk) : t.fwd + (1 << s) + blk);
         if (s == 0)
           ct_first<M>(sm[x], sm[x + half], wt.x, wt.y, t);
         else
@@ -40,13 +74,12 @@ __global__ void k_ntt_fwd_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
       __syncthreads();
     }
     u64* out = reinterpret_cast<u64*>(job.out);
-    const typename M::Out to(t);
     for (int i = threadIdx.x; i < n; i += blockDim.x) out[i] = to.canon(sm[i]);
     __syncthreads();
   }
 }
 
-template <class M>
+template <class M, bool ROWS>
 __global__ void k_ntt_inv_simple(const vkcu_ntt_job* __restrict__ jobs, int njobs, vkcu_ntt_job one,
                                  int log_n) {
   extern __shared__ u64 sm[];
@@ -54,6 +87,7 @@ __global__ void k_ntt_inv_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
   for (int w = blockIdx.x; w < njobs; w += gridDim.x) {
     const vkcu_ntt_job job = fetch_job(jobs, one, w);
     const Tw t = load_tw(job.tw);
+    const ulonglong2 f0 = ld_late2(t.fold), f1 = ld_late2(t.fold + 1);
     const u64* in = reinterpret_cast<const u64*>(job.in);
     for (int i = threadIdx.x; i < n; i += blockDim.x) sm[i] = in[i];
     __syncthreads();
@@ -68,11 +102,11 @@ __global__ void k_ntt_inv_simple(const vkcu_ntt_job* __restrict__ jobs, int njob
         else
           M::template sd<1>(sm[x], sm[x + half], t, sum, dif);
         if (s == 0) {
-          const ulonglong2 f0 = t.fold[0], f1 = t.fold[1];
-          sm[x] = shoup(sum, f0.x, f0.y, t.q);
-          sm[x + half] = shoup(dif, f1.x, f1.y, t.q);
+          sm[x] = csub(shoup_lazy_short(sum, f0.x, f0.y, t.q), t.q);
+          sm[x + half] = csub(shoup_lazy_short(dif, f1.x, f1.y, t.q), t.q);
         } else {
-          const ulonglong2 wt = ld_tw(t.inv + vkcu_tw_slot(log_n, (1u << s) + blk));
+          const ulonglong2 wt =
+            ld_tw(ROWS ? t.inv + vkcu_tw_slot(log_n, (1u << s) + blk) : t.inv + (1 << s) + blk);
           sm[x] = M::template settle<M::sum_bound(1)>(M::sum(sum, t), t);
           sm[x + half] = M::mul(dif, wt.x, wt.y, t);
         }
@@ -166,13 +200,13 @@ static constexpr int kMaxLogN = 26;     // global passes + 2^14-word sub-blocks
 
 static bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
 
-template <class M>
-static int simple(cudaStream_t st, bool inverse, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one,
-                  int log_n, int sms) {
+template <class S, bool ROWS>
+static int simple_launch(cudaStream_t st, bool inverse, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one,
+                         int log_n, int sms) {
   const int n = 1 << log_n;
   const int threads = n / 2 < 32 ? 32 : (n / 2 > 512 ? 512 : n / 2);
   const int smem = n * 8;
-  auto kern = inverse ? k_ntt_inv_simple<M> : k_ntt_fwd_simple<M>;
+  auto kern = inverse ? k_ntt_inv_simple<S, ROWS> : k_ntt_fwd_simple<S, ROWS>;
   // threads and shared memory depend on n: one occupancy per direction and
   // degree; the kernel's shared-memory limit is the largest n (2^14) always
   static KernelSetup setups[2][kMaxCta + 1];
@@ -182,6 +216,14 @@ static int simple(cudaStream_t st, bool inverse, const vkcu_ntt_job* jobs, int n
   kern<<<grid, threads, smem, st>>>(jobs, njobs, one, log_n);
   vkcu_count_launches(1);
   return (int)cudaGetLastError();
+}
+
+template <class M>
+static int simple(cudaStream_t st, bool inverse, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one,
+                  int log_n, int sms) {
+  using S = std::conditional_t<std::is_same<M, Mod63>::value, Simple63, Simple62>;
+  return log_n < VKCU_TW_ROWS_LOG_N ? simple_launch<S, false>(st, inverse, jobs, njobs, one, log_n, sms)
+                                    : simple_launch<S, true>(st, inverse, jobs, njobs, one, log_n, sms);
 }
 
 // The stages above the sub-blocks: `g` of them in as few passes of <= 4 as
