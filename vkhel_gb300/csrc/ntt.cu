@@ -358,8 +358,9 @@ static bool jobs_aligned(const vkcu_ntt_job* jobs, const vkcu_ntt_job* one) {
 // log2 of the CTAs that share a job where a launch has fewer jobs than the SMs
 // it may count on (`avail`: all, or its share of a batch's concurrent classes),
 // 0 for the degree's own kernel (one CTA to 2^14, 2 / 4 CTAs at 2^15 / 2^16).
-// A single call (one job passed by value) of n >= 2^14 takes 16 CTAs; batches
-// and server micro-batches keep to 8, since their classes run beside other
+// A single call (one job passed by value) of 2^14 .. 2^16 takes 16 CTAs, and so
+// does a product of 2^17 without scratch (few_of_17 below has the others);
+// batches and server micro-batches keep to 8, since their classes run beside other
 // kernels and a 16-CTA cluster can only start once 16 SMs of one GPC are free
 // at the same time.  Tuning entry (3, 1) = 1 turns the split off, (3, 3) = 1
 // keeps single calls on 8.  The lines, from products timed per job count and
@@ -442,7 +443,7 @@ static int forward(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
     if (log_n <= (uint32_t)kMaxCta) return fwd_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms);
     if (log_n <= (uint32_t)kMaxCluster) return fwd_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta);
   } else {
-    if (const int lc = few_of_17(njobs, log_n, avail) ? 0 : split_log(njobs, log_n, avail, jobs == nullptr)) {
+    if (const int lc = log_n < (uint32_t)kMaxCluster ? split_log(njobs, log_n, avail, jobs == nullptr) : 0) {
       const int e = fwd_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc);
       // a GPU that cannot host 16-CTA clusters: the set-up refuses before any launch
       return e == (int)cudaErrorInvalidConfiguration && lc == 4
@@ -497,7 +498,7 @@ static int inverse(void* stream, const vkcu_ntt_job* jobs, int njobs, const vkcu
       if (log_n <= (uint32_t)kMaxCta) return inv_cta_wide(st, jobs, njobs, o, (int)log_n, 0, sms, lp);
       if (log_n <= (uint32_t)kMaxCluster) return inv_cluster_wide(st, jobs, njobs, o, (int)log_n - kMaxCta, lp);
     } else {
-      if (const int lc = few_of_17(njobs, log_n, avail) ? 0 : split_log(njobs, log_n, avail, jobs == nullptr)) {
+      if (const int lc = log_n < (uint32_t)kMaxCluster ? split_log(njobs, log_n, avail, jobs == nullptr) : 0) {
         const int r = inv_cluster<M>(st, jobs, njobs, o, lc, (int)log_n - lc, lp);
         return r == (int)cudaErrorInvalidConfiguration && lc == 4
                    ? inv_cluster<M>(st, jobs, njobs, o, 3, (int)log_n - 3, lp)

@@ -425,8 +425,9 @@ using Small13 = Shape<13, 32, 1, M>;
 
 // logc: cluster size 2^logc; logs: sub-block size 2^logs: 14, or, for fewer
 // jobs than SMs, 9 .. 13 with logc = 3, 12 / 13 with logc = 1 or 2 (n = 2^13,
-// 2^14), 10 .. 13 with logc = 4 (n = 2^14 .. 2^17 on 16 CTAs, a cluster size
-// the GPU allows on request).
+// 2^14), 10 .. 12 with logc = 4 (n = 2^14 .. 2^16 on 16 CTAs, a cluster size
+// the GPU allows on request).  Products have 13 with logc = 4 too, for one of
+// 2^17 without the scratch that the global passes want.
 #define VK_CLUSTER_SHAPES(X)                                 \
   switch (logc * 32 + logs) {                                \
     case 1 * 32 + 14: return X(1, SubShape<M>);              \
@@ -442,7 +443,6 @@ using Small13 = Shape<13, 32, 1, M>;
     case 3 * 32 + 13: return X(3, Small13<M>);               \
     case 4 * 32 + 10: return X(4, Small10<M>);               \
     case 4 * 32 + 11: return X(4, Small11<M>);               \
-    case 4 * 32 + 13: return X(4, Small13<M>);               \
     case 4 * 32 + 12: return X(4, Small12<M>);               \
     default: return (int)cudaErrorInvalidValue;              \
   }
@@ -480,6 +480,7 @@ int poly_cluster(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vk
   if (lift) return poly_cluster_lifted<M>(st, jobs, njobs, one, logc, logs, *lift);
   const vkcu_lift l{};
 #define X(L, S) launch_cluster<L, S, k_polymul_cluster<L, S, false>>(st, njobs, jobs, njobs, one, 0, l)
+  if (logc == 4 && logs == 13) return X(4, Small13<M>);
   VK_CLUSTER_SHAPES(X)
 #undef X
 }
