@@ -34,13 +34,27 @@ REPORT = os.path.join(HERE, "tuning", "gb300_report.json")
 POLYMUL, FORWARD, INVERSE, BATCH = 0, 1, 2, 3
 # a variant replaces the incumbent (variant 0 for the many-jobs bucket, the
 # many-jobs choice for the other buckets) only when it is this much faster:
-# smaller gaps are within run-to-run noise
-MARGIN = 0.015
+# smaller gaps are within run-to-run noise (three runs of this program on one
+# GPU: a variant's time over variant 0's differs by up to 0.7 % for batches of
+# 40 us and more, 2.5 % for shorter ones)
+MARGIN = 0.02
 # jobs per SM timed for each bucket of the table (<= 1, <= 2, <= 4, more)
 BUCKET_JOBS_PER_SM = (1.0, 1.5, 3.0, 8.0)
 VARIANTS = {8: [0, 1], 9: [0, 1], 10: [0, 1, 2], 11: [0, 1, 2], 12: [0, 1, 2], 13: [0, 1, 2], 14: [0, 1]}
 DESCRIBE = {0: "default shape", 1: "two radix-16 groups in flight per thread",
             2: "other words-per-thread shape"}
+
+
+def _time_variants(ctx, bt, family, log_n, variants, reps, blocks=7):
+    """Seconds per launch of `bt` (not a graph: the variant is read at every
+    launch) with each variant: the median of `blocks` blocks, the variants in
+    turn within each, so that a slow spell of the machine falls on all."""
+    times = {v: [] for v in variants}
+    for _ in range(blocks):
+        for v in variants:
+            vk.lib().vkhel_tune_set(family, log_n, v)
+            times[v].append(_time_batch(ctx, bt, reps))
+    return {v: sorted(t)[len(t) // 2] for v, t in times.items()}
 
 
 def _time_batch(ctx, bt, reps):
@@ -79,19 +93,15 @@ def _tune_family(ctx, sms, family, reps):
         incumbent = 0
         for bucket in reversed(range(len(counts))):
             count = counts[bucket]
-            times = {}
-            for v in variants:
-                L.vkhel_tune_set(family, log_n, v)
-                bt = vk.Batch(ctx)
-                if family == POLYMUL:
-                    for j in range(count):
-                        bt.add_polymul([t], a.device_ptr + 8 * j * n, b.device_ptr + 8 * j * n,
-                                       c.device_ptr + 8 * j * n)
-                else:
-                    bt.add_transform([t] * count, a, c, inverse=family == INVERSE)
-                bt.commit(graph=False)  # the variant is read at every launch
-                times[v] = _time_batch(ctx, bt, reps)
-                bt.close()
+            bt = vk.Batch(ctx)
+            if family == POLYMUL:
+                for j in range(count):
+                    bt.add_polymul([t], a.device_ptr + 8 * j * n, b.device_ptr + 8 * j * n, c.device_ptr + 8 * j * n)
+            else:
+                bt.add_transform([t] * count, a, c, inverse=family == INVERSE)
+            bt.commit(graph=False)
+            times = _time_variants(ctx, bt, family, log_n, variants, reps)
+            bt.close()
             v_best = choose(times, incumbent)
             if bucket == len(counts) - 1:
                 incumbent = v_best
