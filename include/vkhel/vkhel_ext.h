@@ -227,6 +227,10 @@ int vkhel_batch_add_polymul_lift(struct vkhel_batch *batch,
 		const struct vkhel_vector *a, const struct vkhel_vector *b,
 		struct vkhel_vector *c, const struct vkhel_lift_step *steps,
 		uint32_t nsteps);
+/* Takes the batch's device memory (job table, scratch) and makes it ready to
+ * launch; after a failure it may be called again.  Few products of n = 131072
+ * also take n words each, which make them faster, where those can be had and
+ * the context has no budget. */
 int vkhel_batch_commit(struct vkhel_batch *batch, uint32_t flags);
 /* Enqueue one run on the context stream and return (asynchronous). */
 int vkhel_batch_launch(struct vkhel_batch *batch);
@@ -281,10 +285,10 @@ void vkhel_elem_batch_destroy(struct vkhel_elem_batch *batch);
  * concurrent streams; log_n 1: 1 = never split few jobs of n = 2^12 .. 2^17
  * (fewer than the SMs, e.g. a single call, or those past a launch's whole
  * rounds) over more CTAs than their degree's own kernel (the default, 0,
- * splits them: single calls of n >= 2^14 over 16 CTAs, others over 2, 4 or 8
- * by degree and count); log_n 2: 1 = run a ragged batch of fused products of
- * 2^12 .. 2^16 as one persistent launch; log_n 3: 1 = single calls over 8
- * CTAs only. */
+ * splits them: single calls of n = 2^14 .. 2^16 over 16 CTAs, few of 2^17 over
+ * sub-blocks of 8, others over 2, 4 or 8 by degree and count); log_n 2: 1 = run
+ * a ragged batch of fused products of 2^12 .. 2^16 (q < 2^62) as one persistent
+ * launch; log_n 3: 1 = single calls over 8 CTAs only. */
 enum vkhel_tune_family {
 	VKHEL_TUNE_POLYMUL = 0,
 	VKHEL_TUNE_FORWARD = 1,

@@ -15,9 +15,9 @@ the device so that a profiler capture of one launch ends quickly.
   inv_cluster   64 inverse transforms of n = 2^16 (batch)       k_ntt_inv_cluster<2,..>
   twiddles      device twiddle tables for n = 2^20              k_twiddles
   global        16 forward + 16 inverse transforms of n = 2^20  k_fwd_global, k_inv_global,
-                k_ntt_{fwd,inv}_cluster<2,..> on the 2^16-word sub-blocks
-  pointwise     32 polymuls of n = 2^18                         k_fwd_global, k_polymul_cluster<2,..>
-                on the 2^16-word sub-blocks, k_inv_global
+                k_ntt_{fwd,inv}<14,..> on the 2^14-word sub-blocks
+  pointwise     32 polymuls of n = 2^18, 63-bit primes          k_fwd_global, k_ntt_fwd<14,..>,
+                k_pointwise, k_ntt_inv<14,..>, k_inv_global
   simple        4096 forward + inverse transforms of n = 2^7    k_ntt_fwd_simple, k_ntt_inv_simple
   wide_polymul  256 polymuls of n = 2^14, 63-bit primes         k_polymul<14,..,Mod63>
   cluster_polymul  64 polymuls of n = 2^16 (single-limb batch)  k_polymul_cluster<2,..>
@@ -113,7 +113,9 @@ def case_global(ctx):
 
 
 def case_pointwise(ctx):
-    return _polymul_batch(ctx, 1 << 18, 32, primes=4)
+    """Past one cluster products with q < 2^62 multiply inside their sub-blocks'
+    launch; k_pointwise serves those with q >= 2^62 (and n < 2^8)."""
+    return _polymul_batch(ctx, 1 << 18, 32, bits=63, primes=4)
 
 
 def case_simple(ctx):

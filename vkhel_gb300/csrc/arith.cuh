@@ -10,13 +10,13 @@
 //    here with the same constants so that every output, canonical or not,
 //    equals the reference's for every 64-bit input.
 //
-//  * Lazy (Harvey) butterflies for the transforms.  Values travel in [0, 4q)
-//    (forward) or [0, 2q) (inverse) and are made canonical once at the end, so
-//    a butterfly costs one Shoup product and no full reduction.  This needs
-//    4q <= 2^64, i.e. q < 2^62, which the table builder enforces.  Canonical
-//    outputs equal the reference's stage-by-stage canonical arithmetic
-//    (nttfwdbutterfly.comp:44-57, nttrevbutterfly.comp:44-57) because both are
-//    the same residues mod q.
+//  * What lazy (Harvey) butterflies are made of.  Values travel a few multiples
+//    of q above it, as far as 64 bits allow for the modulus class (ntt_core.cuh:
+//    12q for q < 2^60, 4q for q < 2^62, 2q for q < 2^63), and are made canonical
+//    once at the end, so a butterfly costs one Shoup product and no full
+//    reduction.  Canonical outputs equal the reference's stage-by-stage canonical
+//    arithmetic (nttfwdbutterfly.comp:44-57, nttrevbutterfly.comp:44-57) because
+//    both are the same residues mod q.
 #pragma once
 
 #include <cstdint>

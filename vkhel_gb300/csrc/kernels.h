@@ -265,7 +265,7 @@ int vkh_variant_jobs(int family, int log_n, long njobs, int sms);
 int vkcu_measure_int_peak(void *stream, int sms, double *bfly_per_s, double *imad_per_s);
 /* Largest log_n of the single-launch kernels (one CTA up to 2^14, one
  * cluster up to 2^17), and the largest log_n handled at all (2^26: passes
- * over HBM plus 2^14-word sub-blocks). */
+ * over HBM plus sub-blocks of 2^14 or 2^16 words). */
 uint32_t vkcu_max_fused_log_n(void);
 uint32_t vkcu_max_log_n(void);
 

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256)
 
 static constexpr int kMaxCta = 14;      // one CTA per transform
 static constexpr int kMaxCluster = 17;  // one cluster of up to 8 CTAs
-static constexpr int kMaxLogN = 26;     // global passes + 2^14-word sub-blocks
+static constexpr int kMaxLogN = 26;     // global passes + sub-blocks of 2^14 or 2^16 words
 
 static bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
 
@@ -371,6 +371,9 @@ static bool jobs_aligned(const vkcu_ntt_job* jobs, const vkcu_ntt_job* one) {
 //         100: 66 / 70 / 57 / 72
 //   2^15: (2 / 4 / 8) 19 jobs 70 / 47 / 41, 50: 72 / 75 / 62, 60: 72 / 76 / 88
 //   2^16: (4 / 8) 19 jobs 78 / 78, 24: 78 / 86
+// (2^14 stops at half the SMs although 100 products would still gain on 4 CTAs:
+// transforms and products with NTT(b) given lose there, see Tail, which tells
+// them apart.)
 static int split_log(long njobs, uint32_t log_n, long avail, bool single) {
   if (log_n < 12 || log_n > 17 || vkh_variant(3, 1) != 0) return 0;
   if (single && log_n >= 14 && njobs * 16 <= avail && vkh_variant(3, 3) == 0) return 4;
@@ -393,8 +396,10 @@ static bool few_of_17(long njobs, uint32_t log_n, long avail) {
 
 // The last jobs of a launch whose kernel runs `round` jobs at a time, one per
 // SM or SM pair: those past the whole rounds, where a split finishes them
-// sooner than a round of their own.  Only where the launch has the GPU to
-// itself -- concurrent classes fill a partial round anyway.  Products of 2^14
+// sooner than a round of their own.  Only where the launch may count on the
+// whole GPU -- concurrent classes of a batch fill a partial round anyway (the
+// server's chunks, whose classes run one after another on a stream each, count
+// on it too).  Products of 2^14
 // in us, without / with the split tail: 160 (8 past the round) 129 / 91, 200
 // (48) 131 / 108, 344 (40) 193 / 172; of 2^15, 80 (4) 139 / 103, 160 (8) 207 /
 // 172, 120 (44) 142 / 135.  A tail of 77 .. 106 products of 2^14 on 4 CTAs each

@@ -48,9 +48,9 @@ using SubShape = Shape<14, 32, 1, M>;  // the large-n sub-block
 
 // The column pass: the first LOGC stages, which mix the sub-blocks, and with
 // them the sub-block's own first pass (FIRSTK stages) where both fit one
-// radix-16 group -- 2^15 and 2^16 on 2^14-word sub-blocks, 2^12 and 2^16 on 8
-// CTAs -- which saves that pass over shared memory and its barrier (64 products of
-// 2^16 words 161.9 -> 153.7 us, 150 inverse transforms of 2^15 with a lift
+// radix-16 group -- 2^15 and 2^16 on 2^14-word sub-blocks, 2^16 on 8 CTAs --
+// which saves that pass over shared memory and its barrier (64 products of 2^16
+// words 161.9 -> 153.7 us, 150 inverse transforms of 2^15 with a lift
 // 75.9 -> 71.8 us, the ragged batch of 512 instances 3.22 -> 3.06 ms).
 // A group is W = 2^KK words TM apart; word j belongs to CTA j >> LJ.
 template <int LOGC, class S>

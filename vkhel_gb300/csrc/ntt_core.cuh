@@ -20,9 +20,10 @@
 //   * the first forward pass reads all of the thread's words from global
 //     memory up front (the loads are coalesced and all in flight at once);
 //   * the last forward pass works on groups of 16 consecutive words, whose
-//     results leave with 32-byte vector stores, or -- in the fused polymul --
-//     are multiplied pointwise by NTT(b) and run through the first inverse
-//     pass in the same registers;
+//     results leave through shared memory in whole lines (from 2^9 words; by
+//     32-byte vector stores below), or -- in the fused polymul -- are
+//     multiplied pointwise by NTT(b) and run through the first inverse pass in
+//     the same registers;
 //   * the last inverse pass folds n^-1 into its final stage and writes global
 //     memory coalesced.
 // Butterflies are lazy (Harvey): values stay in [0, kq) and are made canonical
@@ -35,7 +36,10 @@
 // (X + WY) mod 2^64 mod q and (X - WY) mod q (forward), or (X + Y) mod 2^64
 // mod q and W (X - Y mod q) (inverse).  All later stages see canonical values,
 // so only the first stage needs the reference's wrap-around behaviour; it is
-// taken on a rarely-used branch whenever an input is >= 2q.
+// taken on a rarely-used branch whenever an input is past the bound up to which
+// the class's lazy butterfly is congruent to it: forward, x >= 3q (Mod60), 2q
+// (Mod62) or q (Mod63); inverse, a word of the group >= 2^bits(q), or either
+// word >= q (Mod63).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -1241,7 +1245,8 @@ template <class M>
 int poly_cta_lift(cudaStream_t st, const vkcu_poly_job* jobs, int njobs, const vkcu_poly_job& one, int log_n, int sms,
                   int variant, const vkcu_lift& lift);
 // cluster of 2^logc CTAs with sub-blocks of 2^logs words, n = 2^(logc + logs):
-// logs = 14 for n = 2^15 .. 2^17; logc = 3 with logs = 10 / 11 for n = 2^13 / 2^14
+// logs = 14 for n = 2^15 .. 2^17, 9 .. 13 where few jobs are split further
+// (VK_CLUSTER_SHAPES in ntt_cluster.cuh)
 template <class M>
 int fwd_cluster(cudaStream_t st, const vkcu_ntt_job* jobs, int njobs, const vkcu_ntt_job& one, int logc, int logs);
 template <class M>
